@@ -8,7 +8,8 @@
 //     drain tile i with tcgen05.ld while the tensor cores already work on i+1;
 //   * one CTA per SM, static tile schedule banded over M for L2 reuse.
 //
-// Two kernels share this structure.  Products without a fused collective run on
+// Three kernels.  Plain products of at most 128 rows stream their weights through
+// gemm_small_sm100.cu.  Two kernels share the structure above: products without a fused collective run on
 // the pair kernel (mot_gemm_pair_kernel: clusters of two CTAs, tcgen05.mma
 // cta_group::2 on 256x256 tiles, six 32 KB stages per CTA); the single-CTA kernel
 // (mot_gemm_kernel, 128x256 tiles) carries the fused all-gather and reduce-scatter
@@ -989,6 +990,11 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 
 }  // namespace gemm
 
+// csrc/gemm_small_sm100.cu: products with a few rows of A (split <= 0: chosen by size)
+int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
+                      long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
+                      cudaStream_t st);
+
 struct CommArgs {
   int gather_b = 0, num_copy_ctas = 0, world = 1, my_rank = 0;
   const long long* shard_ptrs = nullptr;
@@ -1085,6 +1091,11 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
     return kHostBadArg;
   }
   const int G = group_mode == 0 ? 1 : num_groups;
+  // Up to 128 rows of A, plain y = x W^T: the weight-streaming kernel.  Its times against the pair kernel stand in
+  // gemm_small_sm100.cu; at 256 rows and 24576 x 4096 weights it loses (76.7 against 58.0 us).
+  if (M <= 128 && group_mode == 0 && !a_mn && !b_mn && (out_mode == 0 || out_mode == 2) && comm == nullptr &&
+      g_pair_mode != 0 && K > 0)
+    return launch_gemm_small(A, B, C, M, N, K, lda, ldb, ldc, out_mode == 2, residual, ldr, alpha, 0, stream);
 
   CUtensorMap tmA, tmB, tmBlocal;
   int rc;

@@ -1,0 +1,350 @@
+// gemm_small: y[M,N] = x[M,K] w[N,K]^T for a few rows of x (text decoding, short prompts, thumbnails), where the
+// product is a stream of weights.
+//
+// The roles of the operands are swapped: 128 rows of w are the M side of tcgen05.mma and the rows of x the N side
+// (16 .. 128), so no tensor-core row is spent on padding rows of x and the accumulator is [128 weight rows][rows
+// of x] in tensor memory.  What bounds it is the stream of w from HBM: the 128 x 64 weight tiles go through a ring of
+// TMA stages, and the reduction is split over the CTAs of a cluster so that (N / 128) x split CTAs, two per SM,
+// keep the whole chip loading.  The partial sums meet in shared memory: every CTA owns a part of the rows of x and
+// adds the cluster's partials for it in a fixed order (distributed shared memory, no atomics, deterministic).
+//
+// Programmatic dependent launch: the ring is filled with weights before griddepcontrol.wait, so the weights of a
+// product are on their way while the kernel in front of it (a norm, an attention) is still running.  Only operands
+// that an earlier kernel of the same chain writes (x, residual, y) are touched after the wait.  Kernels that write
+// weights do not trigger their dependents early, so weights are never read while they are being written.
+//
+// Measured (weights cold in L2, one launch in a chain, us; before = the 256 x 256 pair kernel, of whose 16 - 96 tiles
+// these shapes fill a fraction of the chip; floor = weight bytes at 6.65 TB/s):
+//   N x K            rows 1: before  now  floor    rows 24: before  now    rows 128: before  now
+//   6144 x 4096             27.8   11.5    7.6              27.6   12.9              29.0   20.0
+//   4096 x 4096             27.4    8.2    5.0              27.5   10.3              27.6   17.3
+//   24576 x 4096            63.4   35.2   30.3              54.1   36.3              56.1   43.5
+//   4096 x 12288            66.5   18.0   15.1              66.3   20.4              66.5   29.9
+//   151936 x 4096          335.5  188.2  187.2             263.5  228.4             280.8  263.8
+#include <string.h>
+
+#include <mutex>
+
+#include "host_common.h"
+#include "sm100_common.cuh"
+
+namespace snu1 {
+namespace gsmall {
+
+constexpr int BW = 128;                    // weight rows per tile (M of the instruction)
+constexpr int BK = 64;
+constexpr int W_STAGE = BW * BK * 2;       // 16 KB
+constexpr int NUM_THREADS = 192;           // warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
+
+template <int TN>
+struct Cfg {
+  static constexpr int X_STAGE = TN * BK * 2;
+  static constexpr int STAGE = W_STAGE + X_STAGE;
+  static constexpr int STAGES = TN <= 16 ? 6 : TN <= 32 ? 5 : TN <= 64 ? 4 : 3;   // two CTAs per SM
+  static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+  static constexpr int TMEM = TN < 32 ? 32 : TN;
+  static_assert(TN * BW * 4 <= STAGES * STAGE, "partial sums reuse the ring");
+};
+
+struct Args {
+  int M, N, K;
+  int split;          // CTAs of a cluster = parts of the reduction
+  void* C;
+  long long ldc;
+  int f32_out;
+  const __nv_bfloat16* residual;
+  long long ldr;
+  float alpha;
+  int* status;
+};
+
+__device__ __forceinline__ uint32_t cta_in_cluster() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
+  uint32_t ra;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(ra)
+               : "memory");
+  return v;
+}
+
+template <int TN>
+__global__ void __launch_bounds__(NUM_THREADS, 2)
+    gemm_small_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+                      const Args args) {
+  using C = Cfg<TN>;
+  extern __shared__ uint8_t smem_raw[];
+  // same window offset in every CTA of the cluster: the partial sums are read at this CTA's own offsets
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE);
+  uint64_t* full_bar = bars;
+  uint64_t* empty_bar = bars + C::STAGES;
+  uint64_t* acc_full = bars + 2 * C::STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::STAGES + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cta_in_cluster();
+  const int n0 = (blockIdx.x / args.split) * BW;
+  const int m0 = blockIdx.y * TN;
+  const int chunks = (args.K + BK - 1) / BK;
+  const int c_lo = (int)((long long)chunks * rank / args.split);
+  const int c_hi = (int)((long long)chunks * (rank + 1) / args.split);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < C::STAGES; ++i) {
+      mbar_init(&full_bar[i], 1);
+      mbar_init(&empty_bar[i], 1);
+    }
+    mbar_init(acc_full, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, C::TMEM);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const int n = c_hi - c_lo;
+      const int pre = n < C::STAGES ? n : C::STAGES;
+      for (int i = 0; i < pre; ++i) {
+        mbar_expect_tx(&full_bar[i], C::STAGE);
+        tma_load_2d(smem + i * C::STAGE, &tmW, &full_bar[i], (c_lo + i) * BK, n0);
+      }
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      for (int i = 0; i < pre; ++i)
+        tma_load_2d(smem + i * C::STAGE + W_STAGE, &tmX, &full_bar[i], (c_lo + i) * BK, m0);
+      for (int i = pre; i < n; ++i) {
+        const int s = i % C::STAGES;
+        if (!mbar_wait(&empty_bar[s], ((i / C::STAGES) & 1) ^ 1, abort_flag, args.status, 1)) break;
+        mbar_expect_tx(&full_bar[s], C::STAGE);
+        tma_load_2d(smem + s * C::STAGE, &tmW, &full_bar[s], (c_lo + i) * BK, n0);
+        tma_load_2d(smem + s * C::STAGE + W_STAGE, &tmX, &full_bar[s], (c_lo + i) * BK, m0);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(BW, TN, false, false);
+      bool ok = true;
+      for (int i = 0; i < c_hi - c_lo; ++i) {
+        const int s = i % C::STAGES;
+        if (!mbar_wait(&full_bar[s], (i / C::STAGES) & 1, abort_flag, args.status, 3)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t w_addr = smem_u32(smem + s * C::STAGE);
+        const uint32_t x_addr = w_addr + W_STAGE;
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k)
+          umma_bf16_ss(tmem_base, make_smem_desc(w_addr + k * 32, 0, 1024), make_smem_desc(x_addr + k * 32, 0, 1024),
+                       idesc, (i > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&empty_bar[s]);
+      }
+      if (ok) umma_commit(acc_full);
+    }
+    __syncwarp();
+  }
+  // partial sums: tensor memory -> [row of x][128 weight rows] in this CTA's ring (all of its products have retired)
+  const int rows = min(TN, args.M - m0);
+  float* part = reinterpret_cast<float*>(smem);
+  bool ok = true;
+  if (warp >= 2) {
+    const int quarter = warp & 3;
+    const int wr = quarter * 32 + lane;
+    ok = mbar_wait(acc_full, 0, abort_flag, args.status, 4);
+    if (ok) {
+      tc_fence_after();
+      const uint32_t ta = tmem_base + ((uint32_t)(quarter * 32) << 16);
+      if constexpr (TN == 16) {
+        uint32_t r[16];
+        tmem_ld_32x32b_x16(ta, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (j < rows) part[j * BW + wr] = __uint_as_float(r[j]);
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < TN; c += 32) {
+          if (c >= rows) break;
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(ta + c, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) part[(c + j) * BW + wr] = __uint_as_float(r[j]);
+        }
+      }
+      tc_fence_before();
+    }
+  }
+  cluster_sync();
+  if (warp >= 2) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // this CTA finishes rows [r_lo, r_hi) of the tile: 8 outputs per thread and step
+    const int r_lo = rows * rank / args.split, r_hi = rows * (rank + 1) / args.split;
+    const int tid = threadIdx.x - 64;
+    const uint32_t part_addr = smem_u32(part);
+    for (int v = r_lo * (BW / 8) + tid; v < r_hi * (BW / 8) && ok; v += 128) {
+      const int r = v / (BW / 8), c8 = (v % (BW / 8)) * 8;
+      const int n = n0 + c8;
+      if (n >= args.N) continue;
+      float o[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = 0.f;
+      for (int s = 0; s < args.split; ++s) {
+        const float4 a = ld_cluster_f4(part_addr + (r * BW + c8) * 4, s);
+        const float4 b = ld_cluster_f4(part_addr + (r * BW + c8) * 4 + 16, s);
+        o[0] += a.x; o[1] += a.y; o[2] += a.z; o[3] += a.w;
+        o[4] += b.x; o[5] += b.y; o[6] += b.z; o[7] += b.w;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] *= args.alpha;
+      const long long m = m0 + r;
+      if (args.f32_out) {
+        float4* cp = reinterpret_cast<float4*>(reinterpret_cast<float*>(args.C) + m * args.ldc + n);
+        cp[0] = make_float4(o[0], o[1], o[2], o[3]);
+        cp[1] = make_float4(o[4], o[5], o[6], o[7]);
+      } else {
+        if (args.residual != nullptr) {
+          const uint4 u = *reinterpret_cast<const uint4*>(args.residual + m * args.ldr + n);
+          const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = __bfloat1622float2(h[j]);
+            o[2 * j] += f.x;
+            o[2 * j + 1] += f.y;
+          }
+        }
+        uint4 u;
+        u.x = pack_bf16x2(o[0], o[1]);
+        u.y = pack_bf16x2(o[2], o[3]);
+        u.z = pack_bf16x2(o[4], o[5]);
+        u.w = pack_bf16x2(o[6], o[7]);
+        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(args.C) + m * args.ldc + n) = u;
+      }
+    }
+  }
+  // nobody leaves while another CTA of the cluster may still read its partial sums
+  if (*abort_flag && warp == 1) {
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2000000ull) {
+    }
+  }
+  tc_fence_before();
+  cluster_sync();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, C::TMEM);
+  }
+}
+
+template <int TN>
+static int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a, int tiles, int mt, cudaStream_t st) {
+  using C = Cfg<TN>;
+  int dev = 0;
+  SNU1_CUDA_CHECK(cudaGetDevice(&dev));
+  static std::once_flag once[64];
+  cudaError_t err = cudaSuccess;
+  std::call_once(once[dev & 63], [&]() {
+    err = cudaFuncSetAttribute(gemm_small_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+  });
+  SNU1_CUDA_CHECK(err);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = a.split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(tiles * a.split, mt, 1);
+  cfg.blockDim = dim3(NUM_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = C::SMEM;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  SNU1_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_small_kernel<TN>, tmW, tmX, a));
+  return kHostOk;
+}
+
+}  // namespace gsmall
+
+int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
+                      long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
+                      cudaStream_t st) {
+  using namespace gsmall;
+  const int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+  const int mt = (M + tn - 1) / tn;
+  const int tiles = (N + BW - 1) / BW;
+  const int chunks = (K + BK - 1) / BK;
+  if (split <= 0) {
+    // Split the reduction while the CTAs still fit the chip at two per SM.  Every part adds a pass over the partial
+    // sums, which grows with the rows of x: wide tiles keep at least 12 chunks (768 of the reduction) per part.
+    // 4096 x 4096 weights, 1 row, split 1 / 2 / 4 / 8: 20.9 / 11.9 / 9.1 / 8.2 us; 128 rows: 29.6 / 20.2 / 17.3 / 19.4.
+    split = 1;
+    while (split < 8 && tiles * mt * split * 2 <= 296 && chunks / (split * 2) >= (tn >= 64 ? 12 : 3)) split *= 2;
+  }
+  CUtensorMap tmW, tmX;
+  int rc;
+  {
+    uint64_t dims[2] = {(uint64_t)K, (uint64_t)N};
+    uint64_t strides[1] = {(uint64_t)ldw * 2};
+    uint32_t box[2] = {BK, BW};
+    if ((rc = encode_tmap_bf16(&tmW, w, 2, dims, strides, box)) != kHostOk) return rc;
+  }
+  {
+    uint64_t dims[2] = {(uint64_t)K, (uint64_t)M};
+    uint64_t strides[1] = {(uint64_t)ldx * 2};
+    uint32_t box[2] = {BK, (uint32_t)tn};
+    if ((rc = encode_tmap_bf16(&tmX, x, 2, dims, strides, box)) != kHostOk) return rc;
+  }
+  Args a;
+  memset(&a, 0, sizeof(a));
+  a.M = M;
+  a.N = N;
+  a.K = K;
+  a.split = split;
+  a.C = c;
+  a.ldc = ldc;
+  a.f32_out = f32_out;
+  a.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
+  a.ldr = ldr;
+  a.alpha = alpha;
+  a.status = device_status_word();
+  switch (tn) {
+    case 16: return launch<16>(tmW, tmX, a, tiles, mt, st);
+    case 32: return launch<32>(tmW, tmX, a, tiles, mt, st);
+    case 64: return launch<64>(tmW, tmX, a, tiles, mt, st);
+    default: return launch<128>(tmW, tmX, a, tiles, mt, st);
+  }
+}
+
+}  // namespace snu1
+
+// The same product with the reduction split given (0: chosen by size); snu1_gemm_bf16 comes here by itself.
+SNU1_API int snu1_gemm_small(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
+                             long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
+                             void* stream) {
+  return snu1::launch_gemm_small(x, w, c, M, N, K, ldx, ldw, ldc, f32_out, residual, ldr, alpha, split,
+                                 reinterpret_cast<cudaStream_t>(stream));
+}

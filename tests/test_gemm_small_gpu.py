@@ -1,0 +1,43 @@
+"""The weight-streaming product for a few rows (csrc/gemm_small_sm100.cu) against fp64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("split", [0, 1, 3, 8])
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 64, 65, 128, 129])      # edges of the row tiles 16 / 32 / 64 / 128
+@pytest.mark.parametrize("N,K", [(24, 520), (1000, 1096), (4096, 2048)])   # ragged weight rows and reduction
+def test_small_rows(M, N, K, split):
+    from sensenova_u1_b200.ops import _lib
+    from sensenova_u1_b200.ops._lib import c_float, c_int, c_ll, c_void_p
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    x, w, r = rnd(M, K), rnd(N, K), rnd(M, N)
+    ref = x.double() @ w.double().t()
+    P = lambda t: c_void_p(None if t is None else t.data_ptr())
+
+    def product(out, residual, f32):
+        _lib.call("gemm_small", P(x), P(w), P(out), c_int(M), c_int(N), c_int(K), c_ll(K), c_ll(K), c_ll(N), c_int(f32),
+                  P(residual), c_ll(0 if residual is None or residual.dim() == 1 else N), c_float(1.0), c_int(split),
+                  c_void_p(_lib.stream()))
+        return out.double()
+    f = product(torch.empty(M, N, device="cuda"), None, 1)
+    b = product(torch.empty(M, N, device="cuda", dtype=torch.bfloat16), r, 0)
+    bias = product(torch.empty(M, N, device="cuda", dtype=torch.bfloat16), r[0].contiguous(), 0)
+    _lib.check_status()
+    # fp32 sums of K / 16 tensor-core steps, each off by at most one unit in the last place of a partial sum
+    assert (f - ref).norm() / ref.norm() < K / 16 * 2.0 ** -23 + 1e-6
+    # one rounding to bf16: at most half a unit in the last place, 2^-8 of the value
+    for got, want in ((b, ref + r.double()), (bias, ref + r[0].double())):
+        assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + 1e-2).all()
+
+
+def test_few_rows_take_the_weight_streaming_kernel():
+    """``gemm_nt`` at 128 rows (this kernel) and at 129 (the pair kernel) on the same operands."""
+    from sensenova_u1_b200.ops import gemm
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x = torch.randn(129, 4096, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(4096, 4096, device="cuda", generator=g).to(torch.bfloat16)
+    a, b = gemm.gemm_nt(x[:128], w).double(), gemm.gemm_nt(x, w)[:128].double()
+    assert ((a - b).abs() <= b.abs() * 2.0 ** -7 + 1e-2).all()      # two roundings of nearly the same fp32 sum
