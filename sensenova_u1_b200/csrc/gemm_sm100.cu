@@ -993,7 +993,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 // csrc/gemm_small_sm100.cu: products with a few rows of A (split <= 0: chosen by size)
 int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
                       long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
-                      cudaStream_t st);
+                      int w_static, cudaStream_t st);
 
 struct CommArgs {
   int gather_b = 0, num_copy_ctas = 0, world = 1, my_rank = 0;
@@ -1052,7 +1052,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
                        int num_groups, const int* tile_group, const int* k_begin, const int* k_end,
                        long long b_group_stride, long long c_group_stride, int out_mode,
                        const void* residual, long long ldr, float alpha, long long a_rows,
-                       long long b_rows, cudaStream_t stream, const CommArgs* comm = nullptr) {
+                       long long b_rows, cudaStream_t stream, const CommArgs* comm = nullptr, int w_static = 0) {
   using namespace gemm;
   if (M <= 0 || N <= 0 || K < 0) {
     set_last_error("gemm: bad sizes M=%d N=%d K=%d", M, N, K);
@@ -1095,7 +1095,8 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   // gemm_small_sm100.cu; at 256 rows and 24576 x 4096 weights it loses (76.7 against 58.0 us).
   if (M <= 128 && group_mode == 0 && !a_mn && !b_mn && (out_mode == 0 || out_mode == 2) && comm == nullptr &&
       g_pair_mode != 0 && K > 0)
-    return launch_gemm_small(A, B, C, M, N, K, lda, ldb, ldc, out_mode == 2, residual, ldr, alpha, 0, stream);
+    return launch_gemm_small(A, B, C, M, N, K, lda, ldb, ldc, out_mode == 2, residual, ldr, alpha, 0, w_static,
+                             stream);
 
   CUtensorMap tmA, tmB, tmBlocal;
   int rc;
@@ -1263,6 +1264,19 @@ SNU1_API int snu1_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
                            reinterpret_cast<cudaStream_t>(stream));
 }
 
+
+// y = alpha * x w^T (+ residual) with w[N,K] that no kernel in flight on the stream writes: a short product may start
+// reading w while the kernel in front of it is still running.  out_mode 0 (bf16) or 2 (fp32).
+SNU1_API int snu1_linear_static(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw,
+                                long long ldy, int out_mode, const void* residual, long long ldr, float alpha,
+                                void* stream) {
+  if (out_mode != 0 && out_mode != 2) {
+    snu1::set_last_error("linear_static: out_mode must be 0 or 2");
+    return snu1::kHostBadArg;
+  }
+  return snu1::launch_gemm(x, w, y, M, N, K, ldx, ldw, ldy, 0, 0, 0, 1, nullptr, nullptr, nullptr, 0, 0, out_mode,
+                           residual, ldr, alpha, M, N, reinterpret_cast<cudaStream_t>(stream), nullptr, 1);
+}
 
 // Same product for an A / C of M rows of which only *m_rows_dev (a device scalar) are in use: row tiles past
 // that count are not visited.  For buffers sized for a worst case whose fill is only known on the device

@@ -8,10 +8,9 @@
 // keep the whole chip loading.  The partial sums meet in shared memory: every CTA owns a part of the rows of x and
 // adds the cluster's partials for it in a fixed order (distributed shared memory, no atomics, deterministic).
 //
-// Programmatic dependent launch: the ring is filled with weights before griddepcontrol.wait, so the weights of a
-// product are on their way while the kernel in front of it (a norm, an attention) is still running.  Only operands
-// that an earlier kernel of the same chain writes (x, residual, y) are touched after the wait.  Kernels that write
-// weights do not trigger their dependents early, so weights are never read while they are being written.
+// Programmatic dependent launch: the kernel is set up while the one in front of it (a norm, an attention) is still
+// running, and reads nothing before griddepcontrol.wait unless the caller says that no kernel of the running chain
+// writes w (``w_static``: the layers of an inference engine); then the ring is filled with weights before the wait.
 //
 // Measured (weights cold in L2, one launch in a chain, us; before = the 256 x 256 pair kernel, of whose 16 - 96 tiles
 // these shapes fill a fraction of the chip; floor = weight bytes at 6.65 TB/s):
@@ -55,6 +54,7 @@ struct Args {
   const __nv_bfloat16* residual;
   long long ldr;
   float alpha;
+  int w_static;       // w may be read before the preceding kernel has finished
   int* status;
 };
 
@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
     if (lane == 0) {
       const int n = c_hi - c_lo;
       const int pre = n < C::STAGES ? n : C::STAGES;
+      if (!args.w_static) asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(&full_bar[i], C::STAGE);
         tma_load_2d(smem + i * C::STAGE, &tmW, &full_bar[i], (c_lo + i) * BK, n0);
@@ -291,7 +292,7 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a,
 
 int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
                       long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
-                      cudaStream_t st) {
+                      int w_static, cudaStream_t st) {
   using namespace gsmall;
   const int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   const int mt = (M + tn - 1) / tn;
@@ -330,6 +331,7 @@ int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K
   a.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   a.ldr = ldr;
   a.alpha = alpha;
+  a.w_static = w_static;
   a.status = device_status_word();
   switch (tn) {
     case 16: return launch<16>(tmW, tmX, a, tiles, mt, st);
@@ -345,6 +347,6 @@ int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K
 SNU1_API int snu1_gemm_small(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
                              long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
                              void* stream) {
-  return snu1::launch_gemm_small(x, w, c, M, N, K, ldx, ldw, ldc, f32_out, residual, ldr, alpha, split,
+  return snu1::launch_gemm_small(x, w, c, M, N, K, ldx, ldw, ldc, f32_out, residual, ldr, alpha, split, 0,
                                  reinterpret_cast<cudaStream_t>(stream));
 }

@@ -42,6 +42,16 @@ class DocLayout:
     next_pos: int      # t index the next token / image takes
 
 
+@dataclass
+class DecodeRows:
+    """One query row per document, each reading its own document's cache rows up to its own: stands in for a
+    ``TilePlan`` in :meth:`InferenceEngine.layers`."""
+    meta_q: torch.Tensor
+    meta_k: torch.Tensor
+    first: torch.Tensor    # int32 [docs] first cache row of the document
+    max_keys: int          # longest range of the request
+
+
 class InferenceEngine:
     def __init__(self, cfg: ModelConfig, store: ParamStore, offload=None):
         """``offload``: a ``utils.offload.LayerOffloader``; the decoder-layer weights then come from it
@@ -150,9 +160,13 @@ class InferenceEngine:
                 # back to this layer (next step) after the barriers of all later layers, i.e. after I read
                 self.sp["bar"].barrier()
             q = qk[:, :qd].unflatten(1, (cfg.num_heads, 128))
-            o, _ = attn_ops.attention_fwd(q, self.kc[l][:kv_len], self.vc[l][:kv_len], plan, self.scale,
-                                          out=ws.get("i.o", (R, cfg.num_heads, 128)),
-                                          lse=ws.get("i.lse", (cfg.num_heads, R), torch.float32))
+            o = ws.get("i.o", (R, cfg.num_heads, 128))
+            if isinstance(plan, DecodeRows):
+                attn_ops.attention_decode(q, self.kc[l][:kv_len], self.vc[l][:kv_len], plan.meta_q, plan.meta_k,
+                                          plan.first, kv_rows, plan.max_keys, self.scale, o)
+            else:
+                attn_ops.attention_fwd(q, self.kc[l][:kv_len], self.vc[l][:kv_len], plan, self.scale, out=o,
+                                       lse=ws.get("i.lse", (cfg.num_heads, R), torch.float32))
             x1 = gemm.gemm_nt(o.view(R, qd), W("wo"), out=ws.get("i.x1", (R, H)), residual=x)
             h2 = fused.rmsnorm_fwd(x1, W("ffn_norm"), None, ws.get("i.h2", (R, H)), None, cfg.rms_eps)
             xo = ws.get(f"i.x{l & 1}", (R, H))
@@ -227,6 +241,7 @@ class InferenceEngine:
         x = self.layers(x.contiguous(), UND, pos3, plan, kv_rows, kv_pos)
         last = torch.tensor([sum(lens[:i + 1]) - 1 for i in range(n_docs)], device=self.dev)
         self._meta_k = mk
+        self._doc_starts = [lay.kv_start for lay in layouts]
         for lay, n in zip(layouts, lens):
             lay.next_pos = int(pos3[0][sum(lens[:layouts.index(lay)]) + n - 1]) + 1
         return layouts, x.index_select(0, last)
@@ -296,6 +311,13 @@ class InferenceEngine:
             "doc": torch.arange(n_docs, dtype=torch.int32, device=dev),
         }
         kv_len = self._meta_k.shape[0]
+        # Documents are numbered by their place in the last prefill: when the layouts are those documents in order, row
+        # d reads cache rows [kv_start, its own] and nothing else can be visible to it, so its keys are split over CTAs.
+        # Any other selection of layouts takes the tile plan, which looks at every cache row.
+        first = None
+        if [lay.kv_start for lay in layouts] == self._doc_starts[:n_docs]:
+            first = torch.tensor(self._doc_starts[:n_docs], dtype=torch.int32, device=dev)
+            max_keys = max(lay.img_start - lay.kv_start for lay in layouts) + max_new_tokens
         if sampling and float(sampling.get("repetition_penalty", 1.0) or 1.0) != 1.0:
             vocab = self.p["lm_head"].shape[0]
             st["seen"] = torch.zeros(n_docs, vocab, dtype=torch.bool, device=dev)      # advanced inside the graph
@@ -313,7 +335,8 @@ class InferenceEngine:
             pos3 = torch.stack([st["pos"], zero, zero]).contiguous()
             mq = attn_ops.make_meta(st["doc"], st["pos"])
             self._meta_k.index_copy_(0, st["kv_rows"], mq)
-            plan = attn_ops.build_plan(mq, self._meta_k)
+            plan = (DecodeRows(mq, self._meta_k, first, max_keys) if first is not None
+                    else attn_ops.build_plan(mq, self._meta_k))
             h = self.layers(x.contiguous(), UND, pos3, plan, st["kv_rows"], kv_len)
             st["h"].copy_(h)
             st["pos"].add_(1)

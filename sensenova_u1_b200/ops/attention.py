@@ -173,6 +173,25 @@ def attention_fwd(q, k, v, plan: TilePlan, scale: float, out=None, lse=None):
     return out, lse
 
 
+def attention_decode(q, k, v, meta_q, meta_k, first, last, max_keys: int, scale: float, out, split: int = 0):
+    """One query row per document: ``out[r] = attention(q[r])`` over the cache rows ``[first[r], last[r]]`` (int32 / int64
+    device tensors; ``last`` is the cache row of the query itself) that the mask rule lets it read.  ``q``/``out``
+    ``[rows,Hq,128]``, ``k``/``v`` ``[Sk,Hkv,128]``; ``max_keys``: longest range to expect (only chooses the split)."""
+    for t, nme in ((q, "q"), (k, "k"), (v, "v"), (out, "out")):
+        _check_heads(t, nme)
+    rows, Hq, _ = q.shape
+    Sk, Hkv, _ = k.shape
+    if first.dtype != torch.int32 or last.dtype != torch.int64 or first.numel() != rows or last.numel() != rows:
+        raise ValueError("first / last must be int32 / int64 tensors with one entry per query row")
+    assert meta_q.shape[0] == rows and meta_k.shape[0] == Sk and v.shape[0] == Sk
+    _lib.call("attn_decode", c_void_p(q.data_ptr()), c_ll(q.stride(0)), c_void_p(k.data_ptr()), c_ll(k.stride(0)),
+              c_void_p(v.data_ptr()), c_ll(v.stride(0)), c_void_p(out.data_ptr()), c_ll(out.stride(0)),
+              c_void_p(meta_q.data_ptr()), c_void_p(meta_k.data_ptr()), c_void_p(first.data_ptr()),
+              c_void_p(last.data_ptr()), c_int(rows), c_int(Sk), c_int(Hq), c_int(Hkv), c_float(scale),
+              c_int(max_keys), c_int(split), c_void_p(_lib.stream()))
+    return out
+
+
 def attention_bwd(q, k, v, o, dout, lse, plan: TilePlan, scale: float, dq=None, dk=None, dv=None,
                   delta=None):
     """Gradients of :func:`attention_fwd`.  ``dq``/``dk``/``dv`` may be column
