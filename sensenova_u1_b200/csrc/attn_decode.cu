@@ -118,8 +118,8 @@ __global__ void __launch_bounds__(THREADS, 2) attn_decode_kernel(const Args a) {
   const int rep = a.Hq / a.Hkv, per_kv = rep / HG;
   const int kvh = blockIdx.y / per_kv;
   const int h0 = kvh * rep + (blockIdx.y % per_kv) * HG;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
+  pdl_trigger();
 
   const int lo = max(0, a.first[row]);
   const int hi = (int)min((long long)a.Sk, a.last[row] + 1);

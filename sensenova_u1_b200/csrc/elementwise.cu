@@ -129,6 +129,57 @@ __global__ void __launch_bounds__(RN_THREADS, 2)
   }
 }
 
+// One CTA per row, VPT vectors per thread: for products of few rows, where the warp kernel would leave most SMs without
+// work and one warp with 16 loads of its own.  Part of the programmatic-launch chain of a decoder layer.
+template <int VPT>
+__global__ void __launch_bounds__(RN_THREADS)
+    rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gain,
+                           const int* __restrict__ tile_group, __nv_bfloat16* __restrict__ y,
+                           float* __restrict__ rstd_out, int H, float eps) {
+  __shared__ float scratch[RN_THREADS / 32];
+  const int row = blockIdx.x, nvec = H / 8;
+  pdl_wait();
+  pdl_trigger();
+  int g = tile_group ? tile_group[row >> 7] : 0;
+  if (g < 0) g = 0;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + (long long)row * H);
+  const uint4* gr = reinterpret_cast<const uint4*>(gain + (long long)g * H);
+  uint4* yr = reinterpret_cast<uint4*>(y + (long long)row * H);
+  uint4 v[VPT], w[VPT];
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    const int c = threadIdx.x + j * RN_THREADS;
+    v[j] = w[j] = make_uint4(0, 0, 0, 0);
+    if (c < nvec) {
+      v[j] = xr[c];
+      w[j] = __ldg(gr + c);
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    float f[8];
+    unpack8(v[j], f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss += f[i] * f[i];
+  }
+  ss = block_sum<RN_THREADS>(ss, scratch);
+  const float rstd = rsqrtf(ss / H + eps);
+  if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    const int c = threadIdx.x + j * RN_THREADS;
+    if (c < nvec) {
+      float f[8], gg[8];
+      unpack8(v[j], f);
+      unpack8(w[j], gg);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = f[i] * rstd * gg[i];
+      yr[c] = pack8(f);
+    }
+  }
+}
+
 // dx = rstd * (g*dy - xhat * mean(g*dy*xhat)) (+ dres);  dgain[g] += sum_rows dy * xhat.
 // Each CTA owns ROWS_PER_CTA consecutive rows of one tile and keeps its gain
 // gradient in registers until the end, then adds it to the fp32 accumulator.
@@ -305,6 +356,103 @@ __global__ void __launch_bounds__(QK_THREADS)
   }
 }
 
+// The same for a decoder layer of the inference engine, fused with the write into the K/V cache: q goes to ``q_out``,
+// k (normalised and rotated) and v to cache row kv_rows[row].  Sixteen lanes of 8 elements own a head.  A CTA
+// has one row, or 16 heads of it when rows are few; the heads are loaded before the sine table is ready.  Few rows are
+// bound by the launch, many by the chain position -> sine -> norm -> store of a CTA rather than by memory
+// ((n_q + 2 n_kv) heads read and written once: 30 us at 8192 rows; four rows per CTA with shared tables: 45 - 48 us).
+// 32 / 8 heads, us, against the kernel above and two index copies:
+//   rows       1     24    128    300   1024   8192
+//   before   9.1   11.0   11.4   11.8   16.5   93.9
+//   now      1.8    1.9    2.4    3.8    6.4   46.2
+constexpr int QC_THREADS = 256;
+constexpr int QC_GROUPS = QC_THREADS / 16;
+
+template <int PER>   // heads per group of lanes
+__global__ void __launch_bounds__(QC_THREADS)
+    qknorm_rope_cache_kernel(const __nv_bfloat16* __restrict__ qkv, long long ld_in, __nv_bfloat16* __restrict__ q_out,
+                             long long ld_q, __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc,
+                             long long cache_rows, const long long* __restrict__ kv_rows,
+                             const __nv_bfloat16* __restrict__ gains, const int* __restrict__ pos,
+                             const float* __restrict__ inv_t, const float* __restrict__ inv_hw, int rows, int n_q,
+                             int n_kv, int hpc, float eps, int* status) {
+  __shared__ float2 tab[64];      // cos, sin
+  const int row = blockIdx.x;
+  const int sub = threadIdx.x & 15;
+  const int grp = threadIdx.x >> 4;
+  const int n_heads = n_q + 2 * n_kv;
+  const int h_lo = blockIdx.y * hpc, h_hi = min(n_heads, h_lo + hpc);
+  pdl_wait();
+  pdl_trigger();
+  uint4 raw[PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int h = h_lo + grp + j * QC_GROUPS;
+    raw[j] = make_uint4(0, 0, 0, 0);
+    if (h < h_hi) raw[j] = *reinterpret_cast<const uint4*>(qkv + (long long)row * ld_in + h * 128 + sub * 8);
+  }
+  const long long dst = kv_rows[row];
+  const bool dst_ok = dst >= 0 && dst < cache_rows;
+  if (!dst_ok && threadIdx.x == 0) report_status(status, kBadShape, 5);
+  if (threadIdx.x < 64) {
+    const int i = threadIdx.x;
+    float ang;
+    if (i < 32) ang = (float)pos[row] * inv_t[i];
+    else if (i < 48) ang = (float)pos[rows + row] * inv_hw[i - 32];
+    else ang = (float)pos[2 * rows + row] * inv_hw[i - 48];
+    float sn, cs;
+    sincosf(ang, &sn, &cs);
+    tab[i] = make_float2(cs, sn);
+  }
+  // lane -> first entry of the table, partner, half of the rotation pair
+  int tab0, pxor;
+  bool first;
+  if (sub < 8) {           // t block, pairs (i, i + 32)
+    pxor = 4;
+    first = (sub & 4) == 0;
+    tab0 = (sub & 3) * 8;
+  } else {                 // h and w blocks, pairs (i, i + 16)
+    pxor = 2;
+    first = (sub & 2) == 0;
+    tab0 = (sub < 12 ? 32 : 48) + (sub & 1) * 8;
+  }
+  const uint4 gq = *reinterpret_cast<const uint4*>(gains + (sub >= 8 ? 64 : 0) + (sub & 7) * 8);
+  const uint4 gk = *reinterpret_cast<const uint4*>(gains + 128 + (sub >= 8 ? 64 : 0) + (sub & 7) * 8);
+  __syncthreads();
+  float2 t[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    t[i] = tab[tab0 + i];
+    if (first) t[i].y = -t[i].y;
+  }
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int h = h_lo + grp + j * QC_GROUPS;
+    if (h_lo + (threadIdx.x >> 5) * 2 + j * QC_GROUPS >= h_hi) break;          // both groups of the warp are done
+    const bool rot = h < n_q + n_kv;                                           // the heads of v are only copied
+    float v[8], g[8], o[8];
+    unpack8(raw[j], v);
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss += v[i] * v[i];
+#pragma unroll
+    for (int x = 4; x > 0; x >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, x);   // halves of 64 elements
+    const float rstd = rsqrtf(ss / 64.f + eps);
+    unpack8(h >= n_q ? gk : gq, g);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = v[i] * rstd * g[i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] = v[i] * t[i].x + __shfl_xor_sync(0xffffffffu, v[i], pxor) * t[i].y;
+    if (h >= h_hi) continue;
+    const uint4 u = rot ? pack8(o) : raw[j];
+    if (h < n_q) *reinterpret_cast<uint4*>(q_out + (long long)row * ld_q + h * 128 + sub * 8) = u;
+    else if (dst_ok) {
+      __nv_bfloat16* c = rot ? kc + (h - n_q) * 128 : vc + (h - n_q - n_kv) * 128;
+      *reinterpret_cast<uint4*>(c + dst * n_kv * 128 + sub * 8) = u;
+    }
+  }
+}
+
 // Backward: d_in = d(norm)(R^T d_out); dgains[g][which][64] += sum d_n * xhat.
 // `d` is updated in place (ld_d), qkv holds the saved pre-norm projections.
 __global__ void __launch_bounds__(QK_THREADS)
@@ -467,11 +615,26 @@ __global__ void __launch_bounds__(256)
 
 using namespace snu1;
 
+// Rows up to which the forward norm gives a CTA to every row.  H = 4096, us per launch, warp kernel / row kernel:
+//   rows       1     24    128    512   1184   2048
+//            2.8    4.1    4.2    4.6    5.2    6.4     (H = 2048: 1.9 .. 2.9)
+//            1.4    1.7    1.7    2.6    3.9      -     (H = 2048: 1.3 .. 2.7)
+// Beyond, both are bound by memory and the warp kernel needs no barrier.
+static constexpr int kRowKernelRows = 148 * 8;
+
 SNU1_API int snu1_rmsnorm_fwd(const void* x, const void* gain, const int* tile_group, void* y,
                               float* rstd, int rows, int H, float eps, void* stream) {
   if (H % 8 != 0 || rows <= 0) {
     set_last_error("rmsnorm_fwd: H must be a multiple of 8 (H=%d rows=%d)", H, rows);
     return kHostBadArg;
+  }
+  if (rows <= kRowKernelRows && H <= 8 * RN_THREADS * 4) {
+    const __nv_bfloat16 *xp = (const __nv_bfloat16*)x, *gp = (const __nv_bfloat16*)gain;
+    const int vpt = (H / 8 + RN_THREADS - 1) / RN_THREADS;
+    auto k = vpt <= 1 ? rmsnorm_fwd_row_kernel<1> : vpt == 2 ? rmsnorm_fwd_row_kernel<2> : rmsnorm_fwd_row_kernel<4>;
+    SNU1_CUDA_CHECK(launch_pdl(k, dim3(rows), dim3(RN_THREADS), 0, (cudaStream_t)stream, xp, gp, tile_group,
+                               (__nv_bfloat16*)y, rstd, H, eps));
+    return kHostOk;
   }
   {
     const int wgrid = (rows + 7) / 8 < 148 * 8 ? (rows + 7) / 8 : 148 * 8;
@@ -528,6 +691,30 @@ SNU1_API int snu1_qknorm_rope_fwd(const void* qkv, long long ld_in, void* out, l
       (const __nv_bfloat16*)qkv, ld_in, (__nv_bfloat16*)out, ld_out, (const __nv_bfloat16*)gains,
       tile_group, pos, inv_t, inv_hw, rows, n_q_heads, n_kv_heads, eps);
   SNU1_CUDA_CHECK(cudaGetLastError());
+  return kHostOk;
+}
+
+// q heads of ``qkv`` -> q_out, k and v heads -> rows kv_rows[] of the caches ([cache_rows][n_kv][128], contiguous).  A row
+// index outside the cache is skipped and reported through the status word.
+SNU1_API int snu1_qknorm_rope_cache(const void* qkv, long long ld_in, void* q_out, long long ld_q, void* kc, void* vc,
+                                    long long cache_rows, const long long* kv_rows, const void* gains, const int* pos,
+                                    const float* inv_t, const float* inv_hw, int rows, int n_q, int n_kv, float eps,
+                                    void* stream) {
+  const int heads = n_q + 2 * n_kv;
+  if (rows <= 0 || n_q <= 0 || n_kv <= 0 || ld_in % 8 || ld_q % 8 ||
+      ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(kc) |
+        reinterpret_cast<uintptr_t>(vc) | reinterpret_cast<uintptr_t>(gains)) & 15) != 0) {
+    set_last_error("qknorm_rope_cache: rows=%d, %d + %d heads; rows must be 16-byte aligned", rows, n_q, n_kv);
+    return kHostBadArg;
+  }
+  // few rows: a CTA per 16 heads, so that every group of lanes has one; otherwise a CTA per row (of up to 128 heads)
+  const int hpc = rows <= 148 ? QC_GROUPS : heads < 8 * QC_GROUPS ? heads : 8 * QC_GROUPS;
+  const int per = (hpc + QC_GROUPS - 1) / QC_GROUPS;
+  auto k = per <= 1 ? qknorm_rope_cache_kernel<1> : per <= 3 ? qknorm_rope_cache_kernel<3> : qknorm_rope_cache_kernel<8>;
+  SNU1_CUDA_CHECK(launch_pdl(k, dim3(rows, (heads + hpc - 1) / hpc), dim3(QC_THREADS), 0, (cudaStream_t)stream,
+                             (const __nv_bfloat16*)qkv, ld_in, (__nv_bfloat16*)q_out, ld_q, (__nv_bfloat16*)kc,
+                             (__nv_bfloat16*)vc, cache_rows, kv_rows, (const __nv_bfloat16*)gains, pos, inv_t, inv_hw,
+                             rows, n_q, n_kv, hpc, eps, device_status_word()));
   return kHostOk;
 }
 

@@ -118,19 +118,19 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
     if (lane == 0) {
       const int n = c_hi - c_lo;
       const int pre = n < C::STAGES ? n : C::STAGES;
-      if (!args.w_static) asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (!args.w_static) pdl_wait();
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(&full_bar[i], C::STAGE);
         tma_load_2d(smem + i * C::STAGE, &tmW, &full_bar[i], (c_lo + i) * BK, n0);
       }
-      asm volatile("griddepcontrol.wait;" ::: "memory");
+      pdl_wait();
+      pdl_trigger();
       for (int i = 0; i < pre; ++i)
         tma_load_2d(smem + i * C::STAGE + W_STAGE, &tmX, &full_bar[i], (c_lo + i) * BK, m0);
       for (int i = pre; i < n; ++i) {
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
   }
   cluster_sync();
   if (warp >= 2) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
     // this CTA finishes rows [r_lo, r_hi) of the tile: 8 outputs per thread and step
     const int r_lo = rows * rank / args.split, r_hi = rows * (rank + 1) / args.split;
     const int tid = threadIdx.x - 64;

@@ -38,6 +38,22 @@ int num_sms();
     }                                                                                  \
   } while (0)
 
+// Launch with programmatic stream serialization: the kernel must call pdl_wait() (sm100_common.cuh).
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Encode a tiled bf16 tensor map with 128-byte swizzle.
 //   rank      : 2..4
 //   dims      : extents, innermost first (elements)

@@ -46,6 +46,13 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Programmatic dependent launch.  A kernel launched with launch_pdl() may start while the kernel in front of it still
+// runs; it calls pdl_wait() before it touches anything that an earlier kernel writes or reads, and only then
+// pdl_trigger(), which lets the next kernel start its own prologue.  So at most two kernels of a stream overlap, and a
+// kernel ahead of its wait can only race with the one directly in front of it.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(

@@ -139,16 +139,18 @@ class InferenceEngine:
             else:
                 W = lambda n: p[s + n][branch]
                 WE = lambda n: p[s + n]                     # expert mixtures are whole tensors of one branch
+            # offloaded weights arrive from a copy stream: products wait for it like for any other kernel
+            static = self.offload is None
             h1 = fused.rmsnorm_fwd(x, W("attn_norm"), None, ws.get("i.h1", (R, H)), None, cfg.rms_eps)
-            qkv = gemm.gemm_nt(h1, W("wqkv"), out=ws.get("i.qkv", (R, qd + 2 * kd)))
+            qkv = gemm.gemm_nt(h1, W("wqkv"), out=ws.get("i.qkv", (R, qd + 2 * kd)), w_static=static)
             qk = ws.get("i.qk", (R, qd + kd))
-            fused.qknorm_rope_fwd(qkv, qk, W("qk_norm"), None, pos3, self.inv_t, self.inv_hw,
-                                  cfg.num_heads, cfg.num_kv_heads, cfg.rms_eps)
             if publish is None:
-                self.kc[l].view(-1, kd).index_copy_(0, kv_rows, qk[:, qd:])
-                self.vc[l].view(-1, kd).index_copy_(0, kv_rows, qkv[:, qd + kd:])
+                fused.qknorm_rope_cache(qkv, qk[:, :qd], self.kc[l], self.vc[l], kv_rows, W("qk_norm"), pos3, self.inv_t,
+                                        self.inv_hw, cfg.num_heads, cfg.num_kv_heads, cfg.rms_eps)
             else:
                 from ..parallel.symm import peer_put
+                fused.qknorm_rope_fwd(qkv, qk, W("qk_norm"), None, pos3, self.inv_t, self.inv_hw,
+                                      cfg.num_heads, cfg.num_kv_heads, cfg.rms_eps)
                 kt, vt = ws.get("i.kt", (R, kd)), ws.get("i.vt", (R, kd))
                 kt.copy_(qk[:, qd:])
                 vt.copy_(qkv[:, qd + kd:])
@@ -167,13 +169,13 @@ class InferenceEngine:
             else:
                 attn_ops.attention_fwd(q, self.kc[l][:kv_len], self.vc[l][:kv_len], plan, self.scale, out=o,
                                        lse=ws.get("i.lse", (cfg.num_heads, R), torch.float32))
-            x1 = gemm.gemm_nt(o.view(R, qd), W("wo"), out=ws.get("i.x1", (R, H)), residual=x)
+            x1 = gemm.gemm_nt(o.view(R, qd), W("wo"), out=ws.get("i.x1", (R, H)), residual=x, w_static=static)
             h2 = fused.rmsnorm_fwd(x1, W("ffn_norm"), None, ws.get("i.h2", (R, H)), None, cfg.rms_eps)
             xo = ws.get(f"i.x{l & 1}", (R, H))
             if not cfg.is_moe:
-                gu = gemm.gemm_nt(h2, W("w13"), out=ws.get("i.gu", (R, 2 * cfg.ffn_size)))
+                gu = gemm.gemm_nt(h2, W("w13"), out=ws.get("i.gu", (R, 2 * cfg.ffn_size)), w_static=static)
                 act = fused.swiglu_fwd(gu, ws.get("i.act", (R, cfg.ffn_size)))
-                x = gemm.gemm_nt(act, W("w2"), out=xo, residual=x1)
+                x = gemm.gemm_nt(act, W("w2"), out=xo, residual=x1, w_static=static)
             else:
                 x = self._moe_ffn(WE, h2, x1, branch, xo)
         return x

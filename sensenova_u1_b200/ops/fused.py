@@ -34,6 +34,19 @@ def qknorm_rope_fwd(qkv, out, gains, tile_group, pos3, inv_t, inv_hw, n_q, n_kv,
     return out
 
 
+def qknorm_rope_cache(qkv, q_out, k_cache, v_cache, kv_rows, gains, pos3, inv_t, inv_hw, n_q, n_kv, eps):
+    """:func:`qknorm_rope_fwd` of a decoder layer with a cache: q heads to ``q_out`` [rows, n_q * 128], normalised and
+    rotated k and plain v to rows ``kv_rows`` (int64) of the caches ``[cache_rows, n_kv, 128]``."""
+    rows = qkv.shape[0]
+    if kv_rows.dtype != torch.int64 or kv_rows.numel() != rows or not (k_cache.is_contiguous() and v_cache.is_contiguous()):
+        raise ValueError("kv_rows must be int64 with one entry per row, the caches contiguous")
+    assert k_cache.shape == v_cache.shape and k_cache.shape[1] == n_kv
+    _lib.call("qknorm_rope_cache", P(qkv), c_ll(qkv.stride(0)), P(q_out), c_ll(q_out.stride(0)), P(k_cache), P(v_cache),
+              c_ll(k_cache.shape[0]), P(kv_rows), P(gains), P(pos3), P(inv_t), P(inv_hw), c_int(rows), c_int(n_q),
+              c_int(n_kv), c_float(eps), ST())
+    return q_out
+
+
 def qknorm_rope_bwd(qkv, d, gains, dgains, tile_group, pos3, inv_t, inv_hw, n_q, n_kv, eps):
     rows = qkv.shape[0]
     _lib.call("qknorm_rope_bwd", P(qkv), c_ll(qkv.stride(0)), P(d), c_ll(d.stride(0)), P(gains),

@@ -257,3 +257,56 @@ def test_peer_flag_wait_runs_out_and_the_device_keeps_answering():
     flags.fill_(1)                            # and the same wait returns at once when the flag is there
     _lib.call("wait_flags_limit", c_void_p(flags.data_ptr()), c_int(2), c_int(0), c_int(1), c_ll(50_000_000), st)
     _lib.check_status()
+
+
+@pytest.mark.parametrize("n_q,n_kv", [(2, 1), (32, 8), (32, 4), (96, 24)])    # 1 .. 9 heads per group of lanes
+@pytest.mark.parametrize("rows", [1, 148, 149, 300])                         # CTA per 16 heads up to 148 rows, per row beyond
+def test_qknorm_rope_cache(rows, n_q, n_kv):
+    from sensenova_u1_b200.config import tiny_mot
+    from sensenova_u1_b200.models import oracle
+    from sensenova_u1_b200.ops import _lib, fused
+    cfg = tiny_mot(head_dim=128, patch_size=16)
+    inv_t, inv_hw = (t.contiguous() for t in oracle.rope_inv_freq(cfg, DEV))
+    qkv = _bf(rows, (n_q + 2 * n_kv) * 128, seed=rows)
+    gains = (1 + 0.1 * torch.randn(4, 64, device=DEV)).to(torch.bfloat16)
+    pos3 = torch.randint(0, 3000, (3, rows), device=DEV, dtype=torch.int32)
+    ref = torch.empty(rows, (n_q + n_kv) * 128, device=DEV, dtype=torch.bfloat16)
+    fused.qknorm_rope_fwd(qkv, ref, gains, None, pos3, inv_t, inv_hw, n_q, n_kv, 1e-6)
+    to = torch.randperm(rows + 7, device=DEV)[:rows]
+    kc, vc = (torch.full((rows + 7, n_kv, 128), 3.0, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    q = torch.full((rows, n_q * 128), float("nan"), device=DEV, dtype=torch.bfloat16)
+    fused.qknorm_rope_cache(qkv, q, kc, vc, to, gains, pos3, inv_t, inv_hw, n_q, n_kv, 1e-6)
+    _lib.check_status()
+    k_ref, v_ref = torch.full_like(kc, 3.0), torch.full_like(vc, 3.0)
+    k_ref[to] = ref[:, n_q * 128:].view(rows, n_kv, 128)
+    v_ref[to] = qkv[:, (n_q + n_kv) * 128:].view(rows, n_kv, 128)
+    assert torch.equal(vc, v_ref)
+    # the sums of squares are added in another order: at most one rounding to bf16 apart, 2^-7 of the value
+    for got, want in ((q, ref[:, :n_q * 128]), (kc, k_ref)):
+        assert ((got.float() - want.float()).abs() <= want.float().abs() * 2.0 ** -7 + 1e-6).all()
+
+
+def test_qknorm_rope_cache_reports_a_row_outside_the_cache():
+    from sensenova_u1_b200.ops import _lib, fused
+    z = lambda *s, dt=torch.bfloat16: torch.ones(*s, device=DEV, dtype=dt)
+    kc, vc = z(4, 1, 128) * 5, z(4, 1, 128) * 5
+    rows = torch.tensor([2, 4], device=DEV)
+    fused.qknorm_rope_cache(z(2, 384), z(2, 128), kc, vc, rows, z(4, 64), z(3, 2, dt=torch.int32), z(32, dt=torch.float32),
+                            z(16, dt=torch.float32), 1, 1, 1e-6)
+    with pytest.raises(_lib.NativeLibraryError):
+        _lib.check_status()
+    assert (vc[2] == 1).all() and (vc[[0, 1, 3]] == 5).all()
+
+
+@pytest.mark.parametrize("rows", [1, 1184, 1185])      # CTA per row up to 1184 rows, warp per row beyond
+@pytest.mark.parametrize("H", [256, 384, 2048, 4096, 6144, 8192])
+def test_rmsnorm_fwd_row_kernel(rows, H):
+    from sensenova_u1_b200.models import oracle
+    from sensenova_u1_b200.ops import fused
+    x, gain = _bf(rows, H, seed=rows), _bf(2, H, seed=H)
+    tg = (torch.arange((rows + 127) // 128, device=DEV) % 3 - 1).int()           # -1: a padding tile takes set 0
+    y, rstd = torch.empty_like(x), torch.empty(rows, device=DEV)
+    fused.rmsnorm_fwd(x, gain, tg, y, rstd, 1e-6)
+    ref = oracle.rmsnorm(x.float(), gain.float()[tg.clamp(min=0).repeat_interleave(128)[:rows].long()], 1e-6)
+    assert ((y.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all()
+    torch.testing.assert_close(rstd, torch.rsqrt(x.float().pow(2).mean(1) + 1e-6), rtol=1e-5, atol=0)
