@@ -541,14 +541,6 @@ __global__ void __launch_bounds__(QK_THREADS)
 // SwiGLU on the fused projection [rows][gate(F) | up(F)].
 // ---------------------------------------------------------------------------
 // rows_dev (optional): the number of rows in use, read on the device, for buffers sized for a worst case
-// sigmoid(x) = 0.5 tanh(x / 2) + 0.5 with the hardware tanh: one special-function operation per element (the
-// exp + divide form costs two plus a Newton step, which made these kernels instruction-bound, not memory-bound).
-__device__ __forceinline__ float fast_tanh(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // One row per CTA step, columns strided over the threads: no 64-bit division per element vector.
 __global__ void __launch_bounds__(256)
     swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ act, long long rows, int F,
@@ -570,8 +562,7 @@ __global__ void __launch_bounds__(256)
       unpack8(base[fv + c], up);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float h = 0.5f * gt[j];
-        o[j] = fmaf(h, fast_tanh(h), h) * up[j];   // silu(g) = g sigmoid(g) = h tanh(h) + h
+        o[j] = silu_mul(gt[j], up[j]);
       }
       out[c] = pack8(o);
     }

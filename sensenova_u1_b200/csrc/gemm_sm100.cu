@@ -721,7 +721,15 @@ __device__ __forceinline__ PairUnit decode_pair(const Args& a, int u, int num_m,
   return c;
 }
 
-template <bool A_MN, bool B_MN>
+// SWIGLU: w holds F gate rows and then F up rows, C[M, F] = silu(x w_gate^T) * (x w_up^T).  The even CTA's half of a
+// column tile is 128 gate rows and the odd CTA's the matching up rows, so a row of the accumulator holds 128 gate and
+// 128 up columns and the epilogue writes 128 products: the [M, 2F] projection, written and read back by a kernel of its
+// own before, never reaches memory.  Gate and up are rounded to bf16 first, as when they were stored.
+// 24576 x 4096 weights, us, product + element-wise kernel / fused (up to 128 rows: gemm_small_sm100.cu):
+//   rows       1     64    128    256    512   1024   2048   4096    8192   16384
+//   two     40.6   45.1   49.3   64.1   90.9    169    309    658    1211    2585
+//   fused   35.5   39.7   44.1   56.5   82.4    153    287    533    1075    2305
+template <bool A_MN, bool B_MN, bool SWIGLU = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     mot_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const Args args) {
@@ -750,7 +758,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   if (args.m_rows_dev != nullptr) m_eff = min(m_eff, max(*args.m_rows_dev, 0));
   const int num_m = (m_eff + BM - 1) / BM;
   const int num_mp = (num_m + 1) / 2;
-  const int num_n = (args.N + BN - 1) / BN;
+  constexpr int CN = SWIGLU ? BN / 2 : BN;        // columns of C per tile
+  const int num_n = (args.N + CN - 1) / CN;
   const int num_units = num_mp * num_n * (args.group_mode == 2 ? args.num_groups : 1);
 
   if (threadIdx.x == 0) {
@@ -787,7 +796,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       for (int u = pair; u < num_units && ok; u += npairs) {
         const PairUnit pu = decode_pair(args, u, num_m, num_mp, num_n);
         const int m0 = pu.mp * (2 * BM) + (int)rank * BM;
-        const int n0 = pu.n_tile * BN + (int)rank * P_BN_HALF;
+        const int n0 = SWIGLU ? pu.n_tile * P_BN_HALF + (int)rank * args.N : pu.n_tile * BN + (int)rank * P_BN_HALF;
         for (int ps = 0; ps < pu.npass && ok; ++ps) {
           const int grp = args.group_mode == 1 ? (ps == 0 ? pu.group[0] : pu.group[1]) : 0;
           for (int k0 = pu.k_lo; k0 < pu.k_hi; k0 += BK, ++it) {
@@ -887,10 +896,38 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         const bool mine = ((ps == 0 ? pu.mask[0] : pu.mask[1]) >> rank) & 1;
         const int row = pu.mp * (2 * BM) + (int)rank * BM + quarter * 32 + lane;
         const bool row_ok = mine && row < args.M;
-        const int n0 = pu.n_tile * BN;
+        const int n0 = pu.n_tile * CN;
         const long long c_off =
             (args.group_mode == 2 ? pu.g * args.c_group_stride : 0) + (long long)row * args.ldc;
-        if (mine) {
+        if (SWIGLU && mine) {
+#pragma unroll 1
+          for (int ch = 0; ch < CN / 32; ++ch) {
+            const int col0 = n0 + ch * 32;
+            if (col0 >= args.N) break;  // warp-uniform
+            uint32_t g[32], up[32];
+            const uint32_t ta = tmem_base + acc * BN + ch * 32 + ((uint32_t)(quarter * 32) << 16);
+            tmem_ld_32x32b_x32(ta, g);
+            tmem_ld_32x32b_x32(ta + CN, up);
+            tmem_ld_wait();
+            __syncwarp();
+            if (row_ok) {
+              __nv_bfloat16* cp = reinterpret_cast<__nv_bfloat16*>(args.C) + c_off + col0;
+              const int ncols = min(32, args.N - col0);  // multiple of 8
+#pragma unroll
+              for (int j8 = 0; j8 < 4; ++j8) {
+                if (j8 * 8 >= ncols) break;
+                float o[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                  o[j] = silu_mul(round_bf16(__uint_as_float(g[j8 * 8 + j])), round_bf16(__uint_as_float(up[j8 * 8 + j])));
+                *reinterpret_cast<uint4*>(cp + j8 * 8) = make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]),
+                                                                    pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
+              }
+            }
+            __syncwarp();
+          }
+        }
+        if (!SWIGLU && mine) {
 #pragma unroll 1
         for (int ch = 0; ch < BN / 32; ++ch) {
           const int col0 = n0 + ch * 32;
@@ -993,7 +1030,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 // csrc/gemm_small_sm100.cu: products with a few rows of A (split <= 0: chosen by size)
 int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
                       long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
-                      int w_static, cudaStream_t st);
+                      int w_static, int swiglu, cudaStream_t st);
 
 struct CommArgs {
   int gather_b = 0, num_copy_ctas = 0, world = 1, my_rank = 0;
@@ -1012,7 +1049,7 @@ struct CommArgs {
 static int g_pair_mode = 1;
 static int g_pair_band = gemm::P_BAND;
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool SWIGLU = false>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const gemm::Args& args, long long units,
                        cudaStream_t stream) {
   using namespace gemm;
@@ -1030,11 +1067,11 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const gem
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (max_pairs < 0) {
-    SNU1_CUDA_CHECK(cudaFuncSetAttribute(mot_gemm_pair_kernel<A_MN, B_MN>,
+    SNU1_CUDA_CHECK(cudaFuncSetAttribute(mot_gemm_pair_kernel<A_MN, B_MN, SWIGLU>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES));
     cfg.gridDim = dim3(2 * (num_sms() / 2), 1, 1);
     int n = 0;
-    SNU1_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&n, mot_gemm_pair_kernel<A_MN, B_MN>, &cfg));
+    SNU1_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&n, mot_gemm_pair_kernel<A_MN, B_MN, SWIGLU>, &cfg));
     if (n < 1) {
       set_last_error("gemm: no 2-CTA cluster of the pair kernel fits on this device");
       return kHostBadArg;
@@ -1043,7 +1080,7 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const gem
   }
   const int pairs = (int)(units < max_pairs ? units : max_pairs);
   cfg.gridDim = dim3(2 * pairs, 1, 1);
-  SNU1_CUDA_CHECK(cudaLaunchKernelEx(&cfg, mot_gemm_pair_kernel<A_MN, B_MN>, tmA, tmB, args));
+  SNU1_CUDA_CHECK(cudaLaunchKernelEx(&cfg, mot_gemm_pair_kernel<A_MN, B_MN, SWIGLU>, tmA, tmB, args));
   return kHostOk;
 }
 
@@ -1052,7 +1089,8 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
                        int num_groups, const int* tile_group, const int* k_begin, const int* k_end,
                        long long b_group_stride, long long c_group_stride, int out_mode,
                        const void* residual, long long ldr, float alpha, long long a_rows,
-                       long long b_rows, cudaStream_t stream, const CommArgs* comm = nullptr, int w_static = 0) {
+                       long long b_rows, cudaStream_t stream, const CommArgs* comm = nullptr, int w_static = 0,
+                       int swiglu = 0) {
   using namespace gemm;
   if (M <= 0 || N <= 0 || K < 0) {
     set_last_error("gemm: bad sizes M=%d N=%d K=%d", M, N, K);
@@ -1094,8 +1132,8 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   // Up to 128 rows of A, plain y = x W^T: the weight-streaming kernel.  Its times against the pair kernel stand in
   // gemm_small_sm100.cu; at 256 rows and 24576 x 4096 weights it loses (76.7 against 58.0 us).
   if (M <= 128 && group_mode == 0 && !a_mn && !b_mn && (out_mode == 0 || out_mode == 2) && comm == nullptr &&
-      g_pair_mode != 0 && K > 0)
-    return launch_gemm_small(A, B, C, M, N, K, lda, ldb, ldc, out_mode == 2, residual, ldr, alpha, 0, w_static,
+      (g_pair_mode != 0 || swiglu) && K > 0)
+    return launch_gemm_small(A, B, C, M, N, K, lda, ldb, ldc, out_mode == 2, residual, ldr, alpha, 0, w_static, swiglu,
                              stream);
 
   CUtensorMap tmA, tmB, tmBlocal;
@@ -1115,7 +1153,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   }
   if (rc != kHostOk) return rc;
   const bool fused_comm = comm != nullptr && (comm->gather_b || comm->rs_ptrs != nullptr);
-  const bool use_pair = g_pair_mode != 0 && !fused_comm && out_mode <= 3;
+  const bool use_pair = (g_pair_mode != 0 || swiglu) && !fused_comm && out_mode <= 3;
   const int gB = group_mode == 1 ? G : 1;
   const uint64_t gstride_bytes = (uint64_t)(gB > 1 ? b_group_stride : (long long)b_rows * ldb) * 2;
   if (b_mn) {
@@ -1197,8 +1235,10 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   }
 
   if (use_pair) {
-    const long long units = (long long)((num_m + 1) / 2) * num_n * (group_mode == 2 ? G : 1);
-    if (!a_mn && !b_mn) rc = launch_pair<false, false>(tmA, tmB, args, units, stream);
+    const int cn = swiglu ? BN / 2 : BN;
+    const long long units = (long long)((num_m + 1) / 2) * ((N + cn - 1) / cn) * (group_mode == 2 ? G : 1);
+    if (swiglu) rc = launch_pair<false, false, true>(tmA, tmB, args, units, stream);
+    else if (!a_mn && !b_mn) rc = launch_pair<false, false>(tmA, tmB, args, units, stream);
     else if (!a_mn && b_mn) rc = launch_pair<false, true>(tmA, tmB, args, units, stream);
     else if (a_mn && !b_mn) rc = launch_pair<true, false>(tmA, tmB, args, units, stream);
     else rc = launch_pair<true, true>(tmA, tmB, args, units, stream);
@@ -1276,6 +1316,20 @@ SNU1_API int snu1_linear_static(const void* x, const void* w, void* y, int M, in
   }
   return snu1::launch_gemm(x, w, y, M, N, K, ldx, ldw, ldy, 0, 0, 0, 1, nullptr, nullptr, nullptr, 0, 0, out_mode,
                            residual, ldr, alpha, M, N, reinterpret_cast<cudaStream_t>(stream), nullptr, 1);
+}
+
+// y[M,F] = silu(x w_gate^T) * (x w_up^T) with w[2F,K] = F gate rows, then F up rows; gate and up are rounded to bf16
+// before the activation.  tile_group as in snu1_gemm_bf16 (null: one weight set).  w_static as in snu1_linear_static.
+SNU1_API int snu1_linear_swiglu(const void* x, const void* w, void* y, int M, int F, int K, long long ldx, long long ldw,
+                                long long ldy, const int* tile_group, int num_groups, long long w_group_stride,
+                                int w_static, void* stream) {
+  if (K <= 0) {
+    snu1::set_last_error("linear_swiglu: empty reduction");
+    return snu1::kHostBadArg;
+  }
+  return snu1::launch_gemm(x, w, y, M, F, K, ldx, ldw, ldy, 0, 0, tile_group != nullptr ? 1 : 0, num_groups, tile_group,
+                           nullptr, nullptr, w_group_stride, 0, 0, nullptr, 0, 1.0f, M, 2ll * F,
+                           reinterpret_cast<cudaStream_t>(stream), nullptr, w_static, 1);
 }
 
 // Same product for an A / C of M rows of which only *m_rows_dev (a device scalar) are in use: row tiles past

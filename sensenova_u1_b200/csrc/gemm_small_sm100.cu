@@ -78,7 +78,9 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
   return v;
 }
 
-template <int TN>
+// SWIGLU: w holds args.N gate rows and then as many up rows; a tile is 64 of each and gives 64 columns of
+// silu(gate) * up (both rounded to bf16 first, as when the projection was stored).
+template <int TN, bool SWIGLU>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
     gemm_small_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                       const Args args) {
@@ -96,7 +98,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cta_in_cluster();
-  const int n0 = (blockIdx.x / args.split) * BW;
+  constexpr int CN = SWIGLU ? BW / 2 : BW;      // columns of y per tile
+  const int n0 = (blockIdx.x / args.split) * CN;
   const int m0 = blockIdx.y * TN;
   const int chunks = (args.K + BK - 1) / BK;
   const int c_lo = (int)((long long)chunks * rank / args.split);
@@ -120,6 +123,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  auto load_w = [&](int s, int chunk) {
+    tma_load_2d(smem + s * C::STAGE, &tmW, &full_bar[s], chunk * BK, n0);
+    if (SWIGLU) tma_load_2d(smem + s * C::STAGE + W_STAGE / 2, &tmW, &full_bar[s], chunk * BK, args.N + n0);
+  };
   if (warp == 0) {
     if (lane == 0) {
       const int n = c_hi - c_lo;
@@ -127,7 +134,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
       if (!args.w_static) pdl_wait();
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(&full_bar[i], C::STAGE);
-        tma_load_2d(smem + i * C::STAGE, &tmW, &full_bar[i], (c_lo + i) * BK, n0);
+        load_w(i, c_lo + i);
       }
       pdl_wait();
       pdl_trigger();
@@ -137,7 +144,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
         const int s = i % C::STAGES;
         if (!mbar_wait(&empty_bar[s], ((i / C::STAGES) & 1) ^ 1, abort_flag, args.status, 1)) break;
         mbar_expect_tx(&full_bar[s], C::STAGE);
-        tma_load_2d(smem + s * C::STAGE, &tmW, &full_bar[s], (c_lo + i) * BK, n0);
+        load_w(s, c_lo + i);
         tma_load_2d(smem + s * C::STAGE + W_STAGE, &tmX, &full_bar[s], (c_lo + i) * BK, m0);
       }
     }
@@ -204,21 +211,31 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
     const int r_lo = rows * rank / args.split, r_hi = rows * (rank + 1) / args.split;
     const int tid = threadIdx.x - 64;
     const uint32_t part_addr = smem_u32(part);
-    for (int v = r_lo * (BW / 8) + tid; v < r_hi * (BW / 8) && ok; v += 128) {
-      const int r = v / (BW / 8), c8 = (v % (BW / 8)) * 8;
-      const int n = n0 + c8;
-      if (n >= args.N) continue;
-      float o[8];
+    auto sum8 = [&](int r, int c, float (&o)[8]) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) o[j] = 0.f;
       for (int s = 0; s < args.split; ++s) {
-        const float4 a = ld_cluster_f4(part_addr + (r * BW + c8) * 4, s);
-        const float4 b = ld_cluster_f4(part_addr + (r * BW + c8) * 4 + 16, s);
+        const float4 a = ld_cluster_f4(part_addr + (r * BW + c) * 4, s);
+        const float4 b = ld_cluster_f4(part_addr + (r * BW + c) * 4 + 16, s);
         o[0] += a.x; o[1] += a.y; o[2] += a.z; o[3] += a.w;
         o[4] += b.x; o[5] += b.y; o[6] += b.z; o[7] += b.w;
       }
+    };
+    for (int v = r_lo * (CN / 8) + tid; v < r_hi * (CN / 8) && ok; v += 128) {
+      const int r = v / (CN / 8), c8 = (v % (CN / 8)) * 8;
+      const int n = n0 + c8;
+      if (n >= args.N) continue;
+      float o[8];
+      sum8(r, c8, o);
+      if (SWIGLU) {
+        float up[8];
+        sum8(r, CN + c8, up);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] *= args.alpha;
+        for (int j = 0; j < 8; ++j) o[j] = silu_mul(round_bf16(o[j]), round_bf16(up[j]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] *= args.alpha;
+      }
       const long long m = m0 + r;
       if (args.f32_out) {
         float4* cp = reinterpret_cast<float4*>(reinterpret_cast<float*>(args.C) + m * args.ldc + n);
@@ -258,7 +275,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
   }
 }
 
-template <int TN>
+template <int TN, bool SWIGLU>
 static int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a, int tiles, int mt, cudaStream_t st) {
   using C = Cfg<TN>;
   int dev = 0;
@@ -266,7 +283,7 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a,
   static std::once_flag once[64];
   cudaError_t err = cudaSuccess;
   std::call_once(once[dev & 63], [&]() {
-    err = cudaFuncSetAttribute(gemm_small_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    err = cudaFuncSetAttribute(gemm_small_kernel<TN, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
   });
   SNU1_CUDA_CHECK(err);
   cudaLaunchConfig_t cfg;
@@ -284,7 +301,7 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a,
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  SNU1_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_small_kernel<TN>, tmW, tmX, a));
+  SNU1_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_small_kernel<TN, SWIGLU>, tmW, tmX, a));
   return kHostOk;
 }
 
@@ -292,11 +309,12 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a,
 
 int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
                       long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
-                      int w_static, cudaStream_t st) {
+                      int w_static, int swiglu, cudaStream_t st) {
   using namespace gsmall;
   const int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   const int mt = (M + tn - 1) / tn;
-  const int tiles = (N + BW - 1) / BW;
+  const int cn = swiglu ? BW / 2 : BW;
+  const int tiles = (N + cn - 1) / cn;
   const int chunks = (K + BK - 1) / BK;
   if (split <= 0) {
     // Split the reduction while the CTAs still fit the chip at two per SM.  Every part adds a pass over the partial
@@ -308,9 +326,9 @@ int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K
   CUtensorMap tmW, tmX;
   int rc;
   {
-    uint64_t dims[2] = {(uint64_t)K, (uint64_t)N};
+    uint64_t dims[2] = {(uint64_t)K, (uint64_t)N * (swiglu ? 2 : 1)};
     uint64_t strides[1] = {(uint64_t)ldw * 2};
-    uint32_t box[2] = {BK, BW};
+    uint32_t box[2] = {BK, (uint32_t)cn};
     if ((rc = encode_tmap_bf16(&tmW, w, 2, dims, strides, box)) != kHostOk) return rc;
   }
   {
@@ -333,12 +351,15 @@ int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K
   a.alpha = alpha;
   a.w_static = w_static;
   a.status = device_status_word();
+#define SNU1_SMALL(TN) \
+  return swiglu ? launch<TN, true>(tmW, tmX, a, tiles, mt, st) : launch<TN, false>(tmW, tmX, a, tiles, mt, st)
   switch (tn) {
-    case 16: return launch<16>(tmW, tmX, a, tiles, mt, st);
-    case 32: return launch<32>(tmW, tmX, a, tiles, mt, st);
-    case 64: return launch<64>(tmW, tmX, a, tiles, mt, st);
-    default: return launch<128>(tmW, tmX, a, tiles, mt, st);
+    case 16: SNU1_SMALL(16);
+    case 32: SNU1_SMALL(32);
+    case 64: SNU1_SMALL(64);
+    default: SNU1_SMALL(128);
   }
+#undef SNU1_SMALL
 }
 
 }  // namespace snu1
@@ -347,6 +368,6 @@ int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K
 SNU1_API int snu1_gemm_small(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
                              long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
                              void* stream) {
-  return snu1::launch_gemm_small(x, w, c, M, N, K, ldx, ldw, ldc, f32_out, residual, ldr, alpha, split, 0,
+  return snu1::launch_gemm_small(x, w, c, M, N, K, ldx, ldw, ldc, f32_out, residual, ldr, alpha, split, 0, 0,
                                  reinterpret_cast<cudaStream_t>(stream));
 }

@@ -298,4 +298,18 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// sigmoid(x) = 0.5 tanh(x / 2) + 0.5 with the hardware tanh: one special-function operation per element (the
+// exp + divide form costs two plus a Newton step, which made the SwiGLU kernels instruction-bound, not memory-bound).
+__device__ __forceinline__ float fast_tanh(float x) {
+  float y;
+  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// silu(g) * u, with silu(g) = g sigmoid(g) = h tanh(h) + h, h = g / 2
+__device__ __forceinline__ float silu_mul(float g, float u) {
+  const float h = 0.5f * g;
+  return fmaf(h, fast_tanh(h), h) * u;
+}
+__device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+
 }  // namespace snu1

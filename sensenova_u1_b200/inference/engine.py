@@ -173,8 +173,7 @@ class InferenceEngine:
             h2 = fused.rmsnorm_fwd(x1, W("ffn_norm"), None, ws.get("i.h2", (R, H)), None, cfg.rms_eps)
             xo = ws.get(f"i.x{l & 1}", (R, H))
             if not cfg.is_moe:
-                gu = gemm.gemm_nt(h2, W("w13"), out=ws.get("i.gu", (R, 2 * cfg.ffn_size)), w_static=static)
-                act = fused.swiglu_fwd(gu, ws.get("i.act", (R, cfg.ffn_size)))
+                act = gemm.linear_swiglu(h2, W("w13"), out=ws.get("i.act", (R, cfg.ffn_size)), w_static=static)
                 x = gemm.gemm_nt(act, W("w2"), out=xo, residual=x1, w_static=static)
             else:
                 x = self._moe_ffn(WE, h2, x1, branch, xo)
@@ -196,8 +195,8 @@ class InferenceEngine:
         r = moe.route(logits, K, cfg.norm_topk_prob)
         xp = ws.get("i.moe.xp", (r.max_rows, H), zero=True)
         moe.gather(h2, r, xp)
-        gu = gemm.gemm_nt(xp, W(f"moe_{br}.w13"), out=ws.get("i.moe.gu", (r.max_rows, 2 * Fe)), tile_group=r.tile_group)
-        act = fused.swiglu_fwd(gu, ws.get("i.moe.act", (r.max_rows, Fe)))
+        act = gemm.linear_swiglu(xp, W(f"moe_{br}.w13"), out=ws.get("i.moe.act", (r.max_rows, Fe)),
+                                 tile_group=r.tile_group)
         yp = gemm.gemm_nt(act, W(f"moe_{br}.w2"), out=ws.get("i.moe.yp", (r.max_rows, H)), tile_group=r.tile_group)
         return moe.combine(yp, r, x1, out)
 

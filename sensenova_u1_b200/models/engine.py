@@ -279,8 +279,12 @@ class MoTEngine:
         s = self._pfx(l)
         S = h2.shape[0]
         tg = b.tile_group
-        gu = gemm.gemm_nt(h2, p[s + "w13"], out=ws.get(pn + "gu", (S, 2 * cfg.ffn_size)), tile_group=tg)
-        act = fused.swiglu_fwd(gu, ws.get("act", (S, cfg.ffn_size)))
+        if out is not None and not pn:
+            # forward pass of a layer that backward evaluates again: the projection itself is not needed
+            gu, act = None, gemm.linear_swiglu(h2, p[s + "w13"], out=ws.get("act", (S, cfg.ffn_size)), tile_group=tg)
+        else:
+            gu = gemm.gemm_nt(h2, p[s + "w13"], out=ws.get(pn + "gu", (S, 2 * cfg.ffn_size)), tile_group=tg)
+            act = fused.swiglu_fwd(gu, ws.get("act", (S, cfg.ffn_size)))
         if out is not None:
             self._tp_sum(gemm.gemm_nt(act, p[s + "w2"], out=out, tile_group=tg, residual=self._res(x1)))
         return dict(gu=gu, act=act)

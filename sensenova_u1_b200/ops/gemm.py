@@ -112,6 +112,24 @@ def gemm_nt(x, w, out=None, *, tile_group=None, residual=None, out_mode=OUT_BF16
     return out
 
 
+def linear_swiglu(x, w13, out=None, *, tile_group=None, w_static=False):
+    """``out[M,F] = silu(x @ gate^T) * (x @ up^T)`` with ``w13[(G,)2F,K]`` = gate rows, then up rows: the product of
+    :func:`gemm_nt` and ``fused.swiglu_fwd`` in one kernel."""
+    _check(x, "x"); _check(w13, "w13")
+    M, K = x.shape
+    grouped = w13.dim() == 3
+    F = w13.shape[-2] // 2
+    assert w13.shape[-1] == K and w13.shape[-2] == 2 * F
+    if grouped and tile_group is None:
+        raise ValueError("grouped weights need tile_group")
+    out = _out(out, M, F, OUT_BF16_STORE, x.device)
+    _lib.call("linear_swiglu", c_void_p(x.data_ptr()), c_void_p(w13.data_ptr()), c_void_p(out.data_ptr()), c_int(M),
+              c_int(F), c_int(K), c_ll(x.stride(0)), c_ll(w13.stride(-2)), c_ll(out.stride(0)),
+              c_void_p(_lib.ptr(tile_group) if grouped else None), c_int(w13.shape[0] if grouped else 1),
+              c_ll(w13.stride(0) if grouped else 0), c_int(1 if w_static else 0), c_void_p(_lib.stream()))
+    return out
+
+
 def gemm_nn(dy, w, out=None, *, tile_group=None, residual=None, out_mode=OUT_BF16_STORE, alpha=1.0, rows_dev=None):
     """``out[M,Kin] = dy[M,Nout] @ w[(G,)Nout,Kin]``  (w is read MN-major)."""
     _check(dy, "dy"); _check(w, "w")

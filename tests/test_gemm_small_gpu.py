@@ -41,3 +41,35 @@ def test_few_rows_take_the_weight_streaming_kernel():
     w = torch.randn(4096, 4096, device="cuda", generator=g).to(torch.bfloat16)
     a, b = gemm.gemm_nt(x[:128], w).double(), gemm.gemm_nt(x, w)[:128].double()
     assert ((a - b).abs() <= b.abs() * 2.0 ** -7 + 1e-2).all()      # two roundings of nearly the same fp32 sum
+
+
+@pytest.mark.parametrize("M", [1, 17, 64, 128, 129, 300, 1000])        # weight-streaming kernel up to 128 rows, pair kernel beyond
+@pytest.mark.parametrize("F,K", [(24, 72), (64, 512), (200, 1096), (768, 2048), (3072, 1024)])   # ragged and whole column tiles
+@pytest.mark.parametrize("static", [False, True])
+def test_linear_swiglu_equals_product_and_activation(M, F, K, static):
+    from sensenova_u1_b200.ops import fused, gemm
+    g = torch.Generator(device="cuda").manual_seed(M + F)
+    x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(2 * F, K, device="cuda", generator=g) * K ** -0.5).to(torch.bfloat16)
+    guard = torch.full((M + 1, F), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm.linear_swiglu(x, w, out=guard[:M], w_static=static)
+    gu = gemm.gemm_nt(x, w)
+    ref = fused.swiglu_fwd(gu, torch.empty(M, F, device="cuda", dtype=torch.bfloat16))
+    # the same sums in the same order, the same roundings
+    assert torch.equal(guard[:M], ref) and (guard[M] == 7).all()
+    want = torch.nn.functional.silu(gu[:, :F].double()) * gu[:, F:].double()
+    # hardware tanh: absolute error 2^-11 of sigmoid, then one rounding
+    assert ((ref.double() - want).abs() <= want.abs() * 2.0 ** -8 + (gu[:, :F] * gu[:, F:]).double().abs() * 2.0 ** -11 + 1e-6).all()
+
+
+def test_linear_swiglu_grouped():
+    from sensenova_u1_b200.ops import fused, gemm
+    g = torch.Generator(device="cuda").manual_seed(5)
+    F, K, tg = 384, 256, torch.tensor([1, 1, 0, -1, 2, 0, 2], dtype=torch.int32, device="cuda")
+    x = torch.randn(7 * 128, K, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(3, 2 * F, K, device="cuda", generator=g) * K ** -0.5).to(torch.bfloat16)
+    out = gemm.linear_swiglu(x, w, out=torch.full((7 * 128, F), 7.0, device="cuda", dtype=torch.bfloat16), tile_group=tg)
+    gu = gemm.gemm_nt(x, w, out=torch.zeros(7 * 128, 2 * F, device="cuda", dtype=torch.bfloat16), tile_group=tg)
+    ref = fused.swiglu_fwd(gu, torch.empty(7 * 128, F, device="cuda", dtype=torch.bfloat16))
+    keep = (tg >= 0).repeat_interleave(128)
+    assert torch.equal(out[keep], ref[keep]) and (out[~keep] == 7).all()
