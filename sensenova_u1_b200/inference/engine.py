@@ -71,6 +71,7 @@ class InferenceEngine:
         self.kc: List[torch.Tensor] = []
         self.vc: List[torch.Tensor] = []
         self.stats = torch.zeros(4 + 4 * 592, dtype=torch.float32, device=self.dev)   # sums + per-block partials
+        self._graph = self._capture_stream = None     # last captured decode step, for its memory (see _capture)
         self.sp = None      # sequence-parallel sampling state (enable_sequence_parallel)
 
     def enable_sequence_parallel(self, group) -> None:
@@ -131,6 +132,19 @@ class InferenceEngine:
         qd, kd = cfg.q_dim, cfg.kv_dim
         if self.offload is not None:
             self.offload.set_phase("prefix" if branch == UND else "denoise")
+        static = self.offload is None           # offloaded weights arrive from a copy stream between the kernels
+        h1, h2, x1 = (ws.get(n, (R, H)) for n in ("i.h1", "i.h2", "i.x1"))
+        xo = [ws.get(f"i.x{i}", (R, H)) for i in range(2)]
+        qkv, qk = ws.get("i.qkv", (R, qd + 2 * kd)), ws.get("i.qk", (R, qd + kd))
+        qf = qk[:, :qd]
+        q = qf.unflatten(1, (cfg.num_heads, 128))
+        o = ws.get("i.o", (R, cfg.num_heads, 128))
+        of = o.view(R, qd)
+        lse = act = None
+        if not isinstance(plan, DecodeRows):
+            lse = ws.get("i.lse", (cfg.num_heads, R), torch.float32)
+        if not cfg.is_moe:
+            act = ws.get("i.act", (R, cfg.ffn_size))
         for l in range(cfg.num_layers):
             s = f"layers.{l}."
             if self.offload is not None:
@@ -139,13 +153,10 @@ class InferenceEngine:
             else:
                 W = lambda n: p[s + n][branch]
                 WE = lambda n: p[s + n]                     # expert mixtures are whole tensors of one branch
-            # offloaded weights arrive from a copy stream: products wait for it like for any other kernel
-            static = self.offload is None
-            h1 = fused.rmsnorm_fwd(x, W("attn_norm"), None, ws.get("i.h1", (R, H)), None, cfg.rms_eps)
-            qkv = gemm.gemm_nt(h1, W("wqkv"), out=ws.get("i.qkv", (R, qd + 2 * kd)), w_static=static)
-            qk = ws.get("i.qk", (R, qd + kd))
+            fused.rmsnorm_fwd(x, W("attn_norm"), None, h1, None, cfg.rms_eps)
+            gemm.gemm_nt(h1, W("wqkv"), out=qkv, w_static=static)
             if publish is None:
-                fused.qknorm_rope_cache(qkv, qk[:, :qd], self.kc[l], self.vc[l], kv_rows, W("qk_norm"), pos3, self.inv_t,
+                fused.qknorm_rope_cache(qkv, qf, self.kc[l], self.vc[l], kv_rows, W("qk_norm"), pos3, self.inv_t,
                                         self.inv_hw, cfg.num_heads, cfg.num_kv_heads, cfg.rms_eps)
             else:
                 from ..parallel.symm import peer_put
@@ -161,22 +172,19 @@ class InferenceEngine:
                 # every peer's slice of this layer is in my cache after the barrier; a peer can only come
                 # back to this layer (next step) after the barriers of all later layers, i.e. after I read
                 self.sp["bar"].barrier()
-            q = qk[:, :qd].unflatten(1, (cfg.num_heads, 128))
-            o = ws.get("i.o", (R, cfg.num_heads, 128))
-            if isinstance(plan, DecodeRows):
-                attn_ops.attention_decode(q, self.kc[l][:kv_len], self.vc[l][:kv_len], plan.meta_q, plan.meta_k,
-                                          plan.first, kv_rows, plan.max_keys, self.scale, o)
+            k, v = self.kc[l][:kv_len], self.vc[l][:kv_len]
+            if lse is None:
+                attn_ops.attention_decode(q, k, v, plan.meta_q, plan.meta_k, plan.first, kv_rows, plan.max_keys,
+                                          self.scale, o)
             else:
-                attn_ops.attention_fwd(q, self.kc[l][:kv_len], self.vc[l][:kv_len], plan, self.scale, out=o,
-                                       lse=ws.get("i.lse", (cfg.num_heads, R), torch.float32))
-            x1 = gemm.gemm_nt(o.view(R, qd), W("wo"), out=ws.get("i.x1", (R, H)), residual=x, w_static=static)
-            h2 = fused.rmsnorm_fwd(x1, W("ffn_norm"), None, ws.get("i.h2", (R, H)), None, cfg.rms_eps)
-            xo = ws.get(f"i.x{l & 1}", (R, H))
+                attn_ops.attention_fwd(q, k, v, plan, self.scale, out=o, lse=lse)
+            gemm.gemm_nt(of, W("wo"), out=x1, residual=x, w_static=static)
+            fused.rmsnorm_fwd(x1, W("ffn_norm"), None, h2, None, cfg.rms_eps)
             if not cfg.is_moe:
-                act = gemm.linear_swiglu(h2, W("w13"), out=ws.get("i.act", (R, cfg.ffn_size)), w_static=static)
-                x = gemm.gemm_nt(act, W("w2"), out=xo, residual=x1, w_static=static)
+                gemm.linear_swiglu(h2, W("w13"), out=act, w_static=static)
+                x = gemm.gemm_nt(act, W("w2"), out=xo[l & 1], residual=x1, w_static=static)
             else:
-                x = self._moe_ffn(WE, h2, x1, branch, xo)
+                x = self._moe_ffn(WE, h2, x1, branch, xo[l & 1])
         return x
 
     def _moe_ffn(self, W, h2, x1, branch, out):
@@ -357,10 +365,7 @@ class InferenceEngine:
         step_fn()                                   # eager: also warms every lazy initialisation
         done = 1
         if use_graph and max_new_tokens > 2:
-            torch.cuda.synchronize()
-            graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph):
-                step_fn()
+            graph = self._capture(step_fn)
         while done < max_new_tokens:
             if done % check_every == 0 and finished():
                 break
@@ -384,6 +389,33 @@ class InferenceEngine:
             lay.next_pos += done
         self.last_decode_steps, self.last_decode_graph = done, graph is not None
         return out
+
+    def _capture(self, fn):
+        """CUDA graph of ``fn()``.  Its temporaries come from the memory pool of the graph before it, which is kept (and
+        never replayed again) for that purpose: ``torch.cuda.graph`` collects garbage and empties the allocator's cache
+        first, and every request then paid for returning that memory to the driver and asking for it again (5 - 400 ms
+        on a shared host)."""
+        cur, old = torch.cuda.current_stream(), self._graph
+        if self._capture_stream is None:             # always the same one: the pool's free blocks belong to a stream
+            self._capture_stream = torch.cuda.Stream()
+        self._capture_stream.wait_stream(cur)
+        graph = torch.cuda.CUDAGraph()
+        try:
+            with torch.cuda.stream(self._capture_stream):
+                graph.capture_begin(pool=None if old is None else old.pool())
+                try:
+                    fn()
+                finally:
+                    graph.capture_end()
+        except torch.cuda.OutOfMemoryError:          # the cache holds what the pool needs: let torch empty it first
+            self._graph = old = None
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                fn()
+        cur.wait_stream(self._capture_stream)
+        self._graph = graph
+        return graph
 
     # --------------------------------------------------------------- generation
     @torch.no_grad()

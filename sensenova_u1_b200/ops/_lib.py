@@ -56,7 +56,9 @@ def ptr(t) -> int | None:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device (without building a Stream object: 0.2 us instead of 4, once
+    per launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 # kernels launched per entry point (for launch accounting)
