@@ -182,28 +182,30 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc_kk = make_idesc_bf16(128, 128, false, false);
       constexpr uint32_t idesc_kmn = make_idesc_bf16(128, 128, false, true);
-      const uint32_t q_addr = smem_u32(sQ), do_addr = smem_u32(sdO), ds_addr = smem_u32(sdS);
-      bool ok = mbar_wait(q_full, 0, abort_flag, args.status, 3);
+      const uint64_t q_desc = make_smem_desc(smem_u32(sQ), 0, 1024), do_desc = make_smem_desc(smem_u32(sdO), 0, 1024);
+      const uint64_t ds_desc = make_smem_desc(smem_u32(sdS), 0, 1024);
+      const uint64_t k_desc = make_smem_desc(smem_u32(sK), 0, 1024), v_desc = make_smem_desc(smem_u32(sV), 0, 1024);
+      const uint64_t kt_desc = make_smem_desc(smem_u32(sK), HALF_BYTES, 1024);
+      constexpr uint32_t tile = TILE_BYTES >> 4, half_tile = HALF_BYTES >> 4;
+      bool ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0, abort_flag, args.status, 3));
       auto issue_s = [&](int j) {
-        const uint32_t k_addr = smem_u32(sK + (j & 1) * TILE_BYTES);
+        const uint64_t kd = k_desc + (j & 1) * tile;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const uint32_t off = (k >> 2) * HALF_BYTES + (k & 3) * 32;
-          umma_bf16_ss(tmem_S, make_smem_desc(q_addr + off, 0, 1024),
-                       make_smem_desc(k_addr + off, 0, 1024), idesc_kk, k > 0 ? 1u : 0u);
+          const uint32_t off = (k >> 2) * half_tile + (k & 3) * 2;
+          umma_bf16_ss(tmem_S, q_desc + off, kd + off, idesc_kk, k > 0 ? 1u : 0u);
         }
         umma_commit(s_full);
       };
       auto issue_dp = [&](int j) {
-        const uint32_t v_addr = smem_u32(sV + (j & 1) * TILE_BYTES);
+        const uint64_t vd = v_desc + (j & 1) * tile;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const uint32_t off = (k >> 2) * HALF_BYTES + (k & 3) * 32;
-          umma_bf16_ss(tmem_dP, make_smem_desc(do_addr + off, 0, 1024),
-                       make_smem_desc(v_addr + off, 0, 1024), idesc_kk, k > 0 ? 1u : 0u);
+          const uint32_t off = (k >> 2) * half_tile + (k & 3) * 2;
+          umma_bf16_ss(tmem_dP, do_desc + off, vd + off, idesc_kk, k > 0 ? 1u : 0u);
         }
         umma_commit(dp_full);
       };
@@ -219,29 +221,33 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
         bool progressed = false;
         if (next_s < n && next_s <= next_dq + 1) {
           const int j = next_s;
-          const bool s_free = j == 0 || mbar_try_wait(s_empty, (j - 1) & 1);
-          const bool dp_free = j == 0 || mbar_try_wait(dp_empty, (j - 1) & 1);
-          if (s_free && dp_free && mbar_try_wait(&kv_full[j & 1], (j >> 1) & 1)) {
+          const bool s_free = j == 0 || mbar_ready(s_empty, (j - 1) & 1);
+          const bool dp_free = j == 0 || mbar_ready(dp_empty, (j - 1) & 1);
+          if (s_free && dp_free && mbar_ready(&kv_full[j & 1], (j >> 1) & 1)) {
             tc_fence_after();
-            issue_s(j);
-            issue_dp(j);
+            if (elect_one()) {
+              issue_s(j);
+              issue_dp(j);
+            }
+            __syncwarp();
             ++next_s;
             progressed = true;
           }
         }
-        if (next_dq < next_s && mbar_try_wait(ds_full, next_dq & 1)) {
+        if (next_dq < next_s && mbar_ready(ds_full, next_dq & 1)) {
           const int j = next_dq;
           tc_fence_after();
-          const uint32_t k_addr = smem_u32(sK + (j & 1) * TILE_BYTES);
+          const uint64_t kd = kt_desc + (j & 1) * tile;
+          const uint32_t acc0 = j > 0 ? 1u : 0u;
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const uint32_t a_off = (k >> 2) * HALF_BYTES + (k & 3) * 32;
-            umma_bf16_ss(tmem_dQ, make_smem_desc(ds_addr + a_off, 0, 1024),
-                         make_smem_desc(k_addr + k * 2048, HALF_BYTES, 1024), idesc_kmn,
-                         (j > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < 8; ++k)
+              umma_bf16_ss(tmem_dQ, ds_desc + (k >> 2) * half_tile + (k & 3) * 2, kd + k * (2048 >> 4), idesc_kmn,
+                           k > 0 ? 1u : acc0);
+            umma_commit(&kv_empty[j & 1]);
+            umma_commit(ds_done);
           }
-          umma_commit(&kv_empty[j & 1]);
-          umma_commit(ds_done);
+          __syncwarp();
           ++next_dq;
           progressed = true;
         }
@@ -250,13 +256,13 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
           spins = 0;
         } else if ((++spins & 0x3ff) == 0) {
           // bounded: nothing became ready for kLocalWaitNs -> report and let every role drain
-          if (*abort_flag) {
+          const uint64_t now = globaltimer_ns();
+          if (t_idle == 0) t_idle = now;
+          if (__any_sync(0xffffffffu, *abort_flag != 0)) {
             ok = false;
-          } else if (t_idle == 0) {
-            t_idle = globaltimer_ns();
-          } else if (globaltimer_ns() - t_idle > kLocalWaitNs) {
+          } else if (__any_sync(0xffffffffu, now - t_idle > kLocalWaitNs)) {
             *abort_flag = 1;
-            report_status(args.status, kWaitTimeout, 2);
+            if (lane == 0) report_status(args.status, kWaitTimeout, 2);
             ok = false;
           }
         }
@@ -551,29 +557,26 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
       if (i + 1 < n) fetch(i + 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc_st = make_idesc_bf16(128, 64, false, false);
       constexpr uint32_t idesc_acc = make_idesc_bf16(128, 128, false, true);
-      const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV);
-      const uint32_t pt_addr = smem_u32(sPT), dst_addr = smem_u32(sdST);
-      bool ok = mbar_wait(kv_full, 0, abort_flag, args.status, 3);
+      const uint64_t k_desc = make_smem_desc(smem_u32(sK), 0, 1024), v_desc = make_smem_desc(smem_u32(sV), 0, 1024);
+      const uint64_t q_desc = make_smem_desc(smem_u32(sQ), 0, 1024), do_desc = make_smem_desc(smem_u32(sdO), 0, 1024);
+      const uint64_t qt_desc = make_smem_desc(smem_u32(sQ), SUB_HALF, 1024), dot_desc = make_smem_desc(smem_u32(sdO), SUB_HALF, 1024);
+      const uint64_t pt_desc = make_smem_desc(smem_u32(sPT), 0, 1024), dst_desc = make_smem_desc(smem_u32(sdST), 0, 1024);
+      constexpr uint32_t sub = SUB_TILE >> 4;
+      bool ok = __all_sync(0xffffffffu, mbar_wait(kv_full, 0, abort_flag, args.status, 3));
       auto issue_sdp = [&](int i) {
         const int s = i & 1, qs = i % DKV_STAGES;
-        const uint32_t q_addr = smem_u32(sQ + qs * SUB_TILE), do_addr = smem_u32(sdO + qs * SUB_TILE);
+        const uint64_t qd = q_desc + qs * sub, dod = do_desc + qs * sub;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint32_t a_off = (k >> 2) * HALF_BYTES + (k & 3) * 32;
-          const uint32_t b_off = (k >> 2) * SUB_HALF + (k & 3) * 32;
-          umma_bf16_ss(tmem_ST + s * 64, make_smem_desc(k_addr + a_off, 0, 1024),
-                       make_smem_desc(q_addr + b_off, 0, 1024), idesc_st, k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < 8; ++k)
+          umma_bf16_ss(tmem_ST + s * 64, k_desc + (k >> 2) * (HALF_BYTES >> 4) + (k & 3) * 2,
+                       qd + (k >> 2) * (SUB_HALF >> 4) + (k & 3) * 2, idesc_st, k > 0 ? 1u : 0u);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint32_t a_off = (k >> 2) * HALF_BYTES + (k & 3) * 32;
-          const uint32_t b_off = (k >> 2) * SUB_HALF + (k & 3) * 32;
-          umma_bf16_ss(tmem_dPT + s * 64, make_smem_desc(v_addr + a_off, 0, 1024),
-                       make_smem_desc(do_addr + b_off, 0, 1024), idesc_st, k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < 8; ++k)
+          umma_bf16_ss(tmem_dPT + s * 64, v_desc + (k >> 2) * (HALF_BYTES >> 4) + (k & 3) * 2,
+                       dod + (k >> 2) * (SUB_HALF >> 4) + (k & 3) * 2, idesc_st, k > 0 ? 1u : 0u);
         umma_commit(&sdp_full[s]);
       };
       // Two queues, issued in whichever order their inputs become ready: S^T / dP^T of sub-tile `next_s`
@@ -588,33 +591,32 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
         bool progressed = false;
         if (next_s < n && next_s <= next_acc + 1) {
           const int i = next_s;
-          if (mbar_try_wait(&sdp_empty[i & 1], ((i >> 1) & 1) ^ 1) &&
-              mbar_try_wait(&qdo_full[i % DKV_STAGES], (i / DKV_STAGES) & 1)) {
+          if (mbar_ready(&sdp_empty[i & 1], ((i >> 1) & 1) ^ 1) &&
+              mbar_ready(&qdo_full[i % DKV_STAGES], (i / DKV_STAGES) & 1)) {
             tc_fence_after();
-            issue_sdp(i);
+            if (elect_one()) issue_sdp(i);
+            __syncwarp();
             ++next_s;
             progressed = true;
           }
         }
-        if (next_acc < next_s && mbar_try_wait(pds_full, next_acc & 1)) {
+        if (next_acc < next_s && mbar_ready(pds_full, next_acc & 1)) {
           const int i = next_acc;
           tc_fence_after();
           const int qs = i % DKV_STAGES;
-          const uint32_t q_addr = smem_u32(sQ + qs * SUB_TILE), do_addr = smem_u32(sdO + qs * SUB_TILE);
+          const uint64_t qd = qt_desc + qs * sub, dod = dot_desc + qs * sub;
+          const uint32_t acc0 = i > 0 ? 1u : 0u;
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {  // reduction over the 64 query rows
-            umma_bf16_ss(tmem_dV, make_smem_desc(pt_addr + k * 32, 0, 1024),
-                         make_smem_desc(do_addr + k * 2048, SUB_HALF, 1024), idesc_acc,
-                         (i > 0 || k > 0) ? 1u : 0u);
-          }
+            for (int k = 0; k < 4; ++k)   // reduction over the 64 query rows
+              umma_bf16_ss(tmem_dV, pt_desc + k * 2, dod + k * (2048 >> 4), idesc_acc, k > 0 ? 1u : acc0);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            umma_bf16_ss(tmem_dK, make_smem_desc(dst_addr + k * 32, 0, 1024),
-                         make_smem_desc(q_addr + k * 2048, SUB_HALF, 1024), idesc_acc,
-                         (i > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < 4; ++k)
+              umma_bf16_ss(tmem_dK, dst_desc + k * 2, qd + k * (2048 >> 4), idesc_acc, k > 0 ? 1u : acc0);
+            umma_commit(&qdo_empty[qs]);
+            umma_commit(pds_done);
           }
-          umma_commit(&qdo_empty[qs]);
-          umma_commit(pds_done);
+          __syncwarp();
           ++next_acc;
           progressed = true;
         }
@@ -623,13 +625,13 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
           spins = 0;
         } else if ((++spins & 0x3ff) == 0) {
           // bounded: nothing became ready for kLocalWaitNs -> report and let every role drain
-          if (*abort_flag) {
+          const uint64_t now = globaltimer_ns();
+          if (t_idle == 0) t_idle = now;
+          if (__any_sync(0xffffffffu, *abort_flag != 0)) {
             ok = false;
-          } else if (t_idle == 0) {
-            t_idle = globaltimer_ns();
-          } else if (globaltimer_ns() - t_idle > kLocalWaitNs) {
+          } else if (__any_sync(0xffffffffu, now - t_idle > kLocalWaitNs)) {
             *abort_flag = 1;
-            report_status(args.status, kWaitTimeout, 2);
+            if (lane == 0) report_status(args.status, kWaitTimeout, 2);
             ok = false;
           }
         }
