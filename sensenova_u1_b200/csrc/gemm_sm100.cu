@@ -830,8 +830,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (even CTA only) ----------------------------
-    if (lane == 0 && rank == 0) {
+    // The warp stays converged and one elected lane issues (see mbar_ready in attn_common.cuh).  From a lane == 0 branch:
+    // 4096 x 24576 x 4096 561 -> 536 us, 4096 x 4096 x 12288 299 -> 289, 16384 x 6144 x 4096 565 -> 542.
+    if (rank == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
+      const uint64_t a_desc = make_smem_desc(smem_u32(sA), A_MN ? MN_CHUNK_BYTES : 0, 1024);
+      const uint64_t b_desc = make_smem_desc(smem_u32(sB), B_MN ? MN_CHUNK_BYTES : 0, 1024);
       uint32_t it = 0;
       uint32_t tile_it = 0;
       bool ok = true;
@@ -840,7 +844,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         for (int ps = 0; ps < pu.npass && ok; ++ps) {
           const int acc = tile_it & 1;
           const uint32_t acc_ph = (tile_it >> 1) & 1;
-          if (!mbar_wait_cl(&acc_empty[acc], acc_ph ^ 1, abort_flag, args.status, 2)) {
+          if (!__all_sync(0xffffffffu, mbar_wait_cl(&acc_empty[acc], acc_ph ^ 1, abort_flag, args.status, 2))) {
             ok = false;
             break;
           }
@@ -850,29 +854,31 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
           for (int k0 = pu.k_lo; k0 < pu.k_hi; k0 += BK, ++it) {
             const int s = it % P_STAGES;
             const uint32_t ph = (it / P_STAGES) & 1;
-            if (!mbar_wait_cl(&full_bar[s], ph, abort_flag, args.status, 3)) {
+            if (!__all_sync(0xffffffffu, mbar_wait_cl(&full_bar[s], ph, abort_flag, args.status, 3))) {
               ok = false;
               break;
             }
             tc_fence_after();
-            const uint32_t a_addr = smem_u32(sA + s * P_A_BYTES);
-            const uint32_t b_addr = smem_u32(sB + s * P_B_BYTES);
+            const uint64_t da = a_desc + s * (P_A_BYTES >> 4), db = b_desc + s * (P_B_BYTES >> 4);
+            const uint32_t acc0 = first ? 0u : 1u;
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k) {
-              const uint64_t da = A_MN ? make_smem_desc(a_addr + k * (UMMA_K * 128), MN_CHUNK_BYTES, 1024)
-                                       : make_smem_desc(a_addr + k * (UMMA_K * 2), 0, 1024);
-              const uint64_t db = B_MN ? make_smem_desc(b_addr + k * (UMMA_K * 128), MN_CHUNK_BYTES, 1024)
-                                       : make_smem_desc(b_addr + k * (UMMA_K * 2), 0, 1024);
-              umma_pair_bf16_ss(d_tmem, da, db, idesc, first ? 0u : 1u);
-              first = false;
+              for (int k = 0; k < BK / UMMA_K; ++k)
+                umma_pair_bf16_ss(d_tmem, da + k * (UMMA_K * (A_MN ? 128 : 2) >> 4), db + k * (UMMA_K * (B_MN ? 128 : 2) >> 4),
+                                  idesc, k > 0 ? 1u : acc0);
+              // the stage is reusable in both CTAs once these products retire
+              umma_pair_commit(smem_u32(&empty_bar[s]));
+              umma_pair_commit(mapa_shared(smem_u32(&empty_bar[s]), 1));
             }
-            // the stage is reusable in both CTAs once these products retire
-            umma_pair_commit(smem_u32(&empty_bar[s]));
-            umma_pair_commit(mapa_shared(smem_u32(&empty_bar[s]), 1));
+            __syncwarp();
+            first = false;
           }
           if (!ok) break;
-          umma_pair_commit(smem_u32(&acc_full[acc]));
-          umma_pair_commit(mapa_shared(smem_u32(&acc_full[acc]), 1));
+          if (elect_one()) {
+            umma_pair_commit(smem_u32(&acc_full[acc]));
+            umma_pair_commit(mapa_shared(smem_u32(&acc_full[acc]), 1));
+          }
+          __syncwarp();
           ++tile_it;
         }
       }
