@@ -19,23 +19,22 @@ constexpr int kMaxTopK = 16;
 // One warp per token.  logits [R,E] fp32 -> probs (optional, fp32 [R,E]), top-k ids / weights.
 // Ties are broken towards the lower expert index (as torch.topk on a sorted scan would for
 // equal values is unspecified; the oracle test uses distinct values).
-__global__ void __launch_bounds__(256)
-    moe_router_kernel(const float* __restrict__ logits, int R, int E, int K, int norm_topk,
-                      float* __restrict__ probs_out, int* __restrict__ top_idx, float* __restrict__ top_w,
-                      int* __restrict__ counts, const int* __restrict__ row_valid,
-                      const float* __restrict__ sel_bias, float* __restrict__ lse_out,
-                      const int* __restrict__ row_class, int* __restrict__ class_counts) {
-  const int row = (blockIdx.x * 256 + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (row >= R) return;
-  const bool valid = row_valid == nullptr || row_valid[row] != 0;
+struct RoutedSlot {   // lane k of the warp: k-th choice of the row
+  int expert;
+  float weight;
+  float lse;
+};
+__device__ __forceinline__ RoutedSlot route_row(const float* __restrict__ logits, int E, int K, int norm_topk,
+                                                float* __restrict__ probs_out, const float* __restrict__ sel_bias, int lane) {
+  float my_w, lse;
+  int my_e;
   constexpr int PER = kMaxExperts / 32;
   float v[PER];
   float mx = -INFINITY;
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
     const int e = lane + 32 * i;
-    v[i] = e < E ? logits[(long long)row * E + e] : -INFINITY;
+    v[i] = e < E ? logits[e] : -INFINITY;
     mx = fmaxf(mx, v[i]);
   }
 #pragma unroll
@@ -49,7 +48,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   const float inv = 1.f / sum;
-  if (lse_out && lane == 0) lse_out[row] = valid ? mx + __logf(sum) : 0.f;     // log-sum-exp of the row (z-loss)
+  lse = mx + __logf(sum);     // log-sum-exp of the row (z-loss)
   // selection score: the probability, plus the per-expert correction bias of bias-based ("aux-free") load
   // balancing when given; the bias steers which experts are picked, the mixing weights stay the probabilities
   float sc[PER];
@@ -57,12 +56,12 @@ __global__ void __launch_bounds__(256)
   for (int i = 0; i < PER; ++i) {
     v[i] *= inv;
     const int e = lane + 32 * i;
-    if (probs_out && e < E) probs_out[(long long)row * E + e] = v[i];
+    if (probs_out && e < E) probs_out[e] = v[i];
     sc[i] = e < E ? v[i] + (sel_bias ? sel_bias[e] : 0.f) : -INFINITY;
   }
   float wsum = 0.f;
-  float my_w = 0.f;
-  int my_e = -1;
+  my_w = 0.f;
+  my_e = -1;
   for (int k = 0; k < K; ++k) {
     float best = -INFINITY;
     int be = 0x7fffffff;
@@ -83,6 +82,7 @@ __global__ void __launch_bounds__(256)
         be = oe;
       }
     }
+    be = min(be, E - 1);                              // no finite score left (NaN logits)
     const float pw = __shfl_sync(0xffffffffu, v[be >> 5], be & 31);     // the chosen expert's probability
     if ((be & 31) == lane) sc[be >> 5] = -INFINITY;  // remove from further rounds
     if (lane == k) {
@@ -91,14 +91,75 @@ __global__ void __launch_bounds__(256)
     }
     wsum += pw;
   }
+  return {my_e, norm_topk ? my_w / wsum : my_w, lse};
+}
+
+__global__ void __launch_bounds__(256)
+    moe_router_kernel(const float* __restrict__ logits, int R, int E, int K, int norm_topk,
+                      float* __restrict__ probs_out, int* __restrict__ top_idx, float* __restrict__ top_w,
+                      int* __restrict__ counts, const int* __restrict__ row_valid,
+                      const float* __restrict__ sel_bias, float* __restrict__ lse_out,
+                      const int* __restrict__ row_class, int* __restrict__ class_counts) {
+  const int row = (blockIdx.x * 256 + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (row >= R) return;
+  const bool valid = row_valid == nullptr || row_valid[row] != 0;
+  const RoutedSlot r = route_row(logits + (long long)row * E, E, K, norm_topk,
+                                 probs_out ? probs_out + (long long)row * E : nullptr, sel_bias, lane);
+  if (lse_out && lane == 0) lse_out[row] = valid ? r.lse : 0.f;
   if (lane < K) {
-    const float w = norm_topk ? my_w / wsum : my_w;
-    top_idx[(long long)row * K + lane] = valid ? my_e : -1;
-    top_w[(long long)row * K + lane] = valid ? w : 0.f;
+    top_idx[(long long)row * K + lane] = valid ? r.expert : -1;
+    top_w[(long long)row * K + lane] = valid ? r.weight : 0.f;
     if (valid) {
-      atomicAdd(counts + my_e, 1);
-      if (class_counts && row_class) atomicAdd(class_counts + row_class[row] * E + my_e, 1);
+      atomicAdd(counts + r.expert, 1);
+      if (class_counts && row_class) atomicAdd(class_counts + row_class[row] * E + r.expert, 1);
     }
+  }
+}
+
+// Router, segments and slots of a few rows (at most 32) in one CTA: decoding routes one row per document, where clearing
+// the counts and the three kernels of the general path took 12 us.  Same layout and the same order of slots.
+__global__ void __launch_bounds__(1024)
+    moe_route_few_kernel(const float* __restrict__ logits, int R, int E, int K, int norm_topk, int* __restrict__ top_idx,
+                         float* __restrict__ top_w, int max_tiles, int* __restrict__ tile_group, int* __restrict__ dest) {
+  __shared__ int s_idx[32 * kMaxTopK];
+  __shared__ int s_count[kMaxExperts], s_start[kMaxExperts];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_trigger();
+  for (int e = threadIdx.x; e < E; e += 1024) s_count[e] = 0;
+  __syncthreads();
+  if (warp < R) {
+    const RoutedSlot r = route_row(logits + (long long)warp * E, E, K, norm_topk, nullptr, nullptr, lane);
+    if (lane < K) {
+      const int i = warp * K + lane;
+      s_idx[i] = r.expert;
+      top_idx[i] = r.expert;
+      top_w[i] = r.weight;
+      atomicAdd(&s_count[r.expert], 1);
+    }
+  }
+  for (int t = threadIdx.x; t < max_tiles; t += 1024) tile_group[t] = -1;
+  __syncthreads();
+  // at most 32 rows: an expert with any row has one tile of 128
+  if (warp == 0) {
+    int acc = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane;
+      const bool used = e < E && s_count[e] > 0;
+      const uint32_t b = __ballot_sync(0xffffffffu, used);
+      const int t = acc + __popc(b & ((1u << lane) - 1));
+      if (e < E) s_start[e] = t * 128;
+      if (used) tile_group[t] = e;
+      acc += __popc(b);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < R * K; i += 1024) {
+    const int e = s_idx[i];
+    int n = 0;
+    for (int j = 0; j < i; ++j) n += s_idx[j] == e;
+    dest[i] = s_start[e] + n;
   }
 }
 
@@ -193,6 +254,8 @@ __global__ void __launch_bounds__(256)
 __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ dest,
                                   const int* __restrict__ top_idx, __nv_bfloat16* __restrict__ xp, int R, int K,
                                   int H) {
+  pdl_wait();
+  pdl_trigger();
   const int hv = H / 8;
   const long long total = (long long)R * K * hv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -210,6 +273,8 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ yp, const i
                                    const int* __restrict__ top_idx, const float* __restrict__ top_w,
                                    const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ y,
                                    int R, int K, int H) {
+  pdl_wait();
+  pdl_trigger();
   const int hv = H / 8;
   const long long total = (long long)R * hv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -229,17 +294,27 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ yp, const i
         acc[2 * e + 1] = f.y;
       }
     }
-    for (int k = 0; k < K; ++k) {
-      const long long rk = row * K + k;
-      if (top_idx[rk] < 0) continue;
-      const float w = top_w[rk];
-      const uint4 u = reinterpret_cast<const uint4*>(yp + (long long)dest[rk] * H)[c];
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+    for (int k0 = 0; k0 < K; k0 += 4) {       // four rows of the experts' outputs on their way at a time
+      uint4 u[4];
+      float w[4];
+      bool ok[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = __bfloat1622float2(h[e]);
-        acc[2 * e] += w * f.x;
-        acc[2 * e + 1] += w * f.y;
+      for (int j = 0; j < 4; ++j) {
+        const long long rk = row * K + min(k0 + j, K - 1);
+        ok[j] = k0 + j < K && top_idx[rk] >= 0;
+        w[j] = top_w[rk];
+        if (ok[j]) u[j] = reinterpret_cast<const uint4*>(yp + (long long)dest[rk] * H)[c];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (!ok[j]) continue;
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u[j]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __bfloat1622float2(h[e]);
+          acc[2 * e] += w[j] * f.x;
+          acc[2 * e + 1] += w[j] * f.y;
+        }
       }
     }
     uint4 o;
@@ -405,6 +480,19 @@ static int grid_1d(long long total, int block) {
 using namespace snu1;
 
 // counts [E] must be zero on entry.  max_tiles = number of 128-row tiles of the permuted buffer.
+// The same for at most 32 rows without the training outputs (no probabilities, no counts): top_idx, top_w [R,K],
+// tile_group [max_tiles] (expert of every 128-row tile, -1 beyond the last), dest [R,K].
+SNU1_API int snu1_moe_route_few(const float* logits, int R, int E, int K, int norm_topk, int* top_idx, float* top_w,
+                                int max_tiles, int* tile_group, int* dest, void* stream) {
+  if (R < 1 || R > 32 || E > kMaxExperts || K > kMaxTopK || K > E || K < 1 || max_tiles < (R * K < E ? R * K : E)) {
+    set_last_error("moe_route_few: R=%d (1..32) E=%d K=%d tiles=%d", R, E, K, max_tiles);
+    return kHostBadArg;
+  }
+  SNU1_CUDA_CHECK(launch_pdl(moe_route_few_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, logits, R, E, K, norm_topk,
+                             top_idx, top_w, max_tiles, tile_group, dest));
+  return kHostOk;
+}
+
 static int moe_route_impl(const float* logits, int R, int E, int K, int norm_topk, float* probs,
                           int* top_idx, float* top_w, int* counts, const int* row_valid, int max_tiles,
                           int* seg_start, int* seg_end, int* tile_group, int* total_rows, int* dest,
@@ -458,9 +546,8 @@ SNU1_API int snu1_moe_gather(const void* x, const int* dest, const int* top_idx,
     set_last_error("moe_gather: H must be a multiple of 8");
     return kHostBadArg;
   }
-  moe_gather_kernel<<<grid_1d((long long)R * K * (H / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)x, dest, top_idx, (__nv_bfloat16*)xp, R, K, H);
-  SNU1_CUDA_CHECK(cudaGetLastError());
+  SNU1_CUDA_CHECK(launch_pdl(moe_gather_kernel, dim3(grid_1d((long long)R * K * (H / 8), 256)), dim3(256), 0,
+                             (cudaStream_t)stream, (const __nv_bfloat16*)x, dest, top_idx, (__nv_bfloat16*)xp, R, K, H));
   return kHostOk;
 }
 
@@ -470,9 +557,11 @@ SNU1_API int snu1_moe_combine(const void* yp, const int* dest, const int* top_id
     set_last_error("moe_combine: H must be a multiple of 8");
     return kHostBadArg;
   }
-  moe_combine_kernel<<<grid_1d((long long)R * (H / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)yp, dest, top_idx, top_w, (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, R, K, H);
-  SNU1_CUDA_CHECK(cudaGetLastError());
+  // few rows: 64 threads per CTA, so that the columns of a row spread over the chip
+  const int threads = R <= 32 ? 64 : 256;
+  SNU1_CUDA_CHECK(launch_pdl(moe_combine_kernel, dim3(grid_1d((long long)R * (H / 8), threads)), dim3(threads), 0,
+                             (cudaStream_t)stream, (const __nv_bfloat16*)yp, dest, top_idx, top_w,
+                             (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, R, K, H));
   return kHostOk;
 }
 

@@ -199,9 +199,18 @@ class InferenceEngine:
         Fe = cfg.moe_intermediate_size
         gate = W(f"moe_{br}.gate")
         logits = gemm.gemm_nt(h2, gate, out=ws.get("i.moe.logits", (R, gate.shape[0]), torch.float32),
-                              out_mode=gemm.OUT_F32_STORE)
+                              out_mode=gemm.OUT_F32_STORE, w_static=self.offload is None)
+        if R <= moe.FEW_ROWS:
+            # Decoding: the experts' weights are streamed like those of any short product, only the experts in use.
+            # One token (8 of 128 experts, 768 x 2048), whole block: 99 -> 45 us.
+            r = moe.route_few(logits, K, cfg.norm_topk_prob, ws)
+            xp = moe.gather(h2, r, ws.get("i.moe.xp", (r.max_rows, H)))
+            act = gemm.gemm_experts(xp, W(f"moe_{br}.w13"), ws.get("i.moe.act", (r.max_rows, Fe)), r.tile_group, R, swiglu=True)
+            yp = gemm.gemm_experts(act, W(f"moe_{br}.w2"), ws.get("i.moe.yp", (r.max_rows, H)), r.tile_group, R)
+            return moe.combine(yp, r, x1, out)
         r = moe.route(logits, K, cfg.norm_topk_prob)
-        xp = ws.get("i.moe.xp", (r.max_rows, H), zero=True)
+        # rows between the experts' segments are never read: nothing is cleared
+        xp = ws.get("i.moe.xp", (r.max_rows, H))
         moe.gather(h2, r, xp)
         act = gemm.linear_swiglu(xp, W(f"moe_{br}.w13"), out=ws.get("i.moe.act", (r.max_rows, Fe)),
                                  tile_group=r.tile_group)

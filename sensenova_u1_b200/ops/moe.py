@@ -76,6 +76,21 @@ def route(logits: torch.Tensor, K: int, norm_topk: bool = True, row_valid=None, 
                    lse, row_class, cc)
 
 
+FEW_ROWS = 32     # rows that one CTA routes, see route_few
+
+
+def route_few(logits: torch.Tensor, K: int, norm_topk: bool, ws) -> Routing:
+    """:func:`route` for at most ``FEW_ROWS`` rows, inference only (no probabilities, counts or segment ends): one launch,
+    buffers from the workspace ``ws``.  ``max_rows`` covers one 128-row tile per expert in use."""
+    R, E = logits.shape
+    mt = min(R * K, E)
+    top_idx, top_w = ws.get("moe.few.idx", (R, K), torch.int32), ws.get("moe.few.w", (R, K), torch.float32)
+    tg, dest = ws.get("moe.few.tg", (mt,), torch.int32), ws.get("moe.few.dest", (R, K), torch.int32)
+    _lib.call("moe_route_few", P(logits), c_int(R), c_int(E), c_int(K), c_int(1 if norm_topk else 0), P(top_idx), P(top_w),
+              c_int(mt), P(tg), P(dest), ST())
+    return Routing(R, E, K, None, top_idx, top_w, None, None, None, tg, None, dest, mt * 128)
+
+
 def gather(x, r: Routing, xp):
     _lib.call("moe_gather", P(x), P(r.dest), P(r.top_idx), P(xp), c_int(r.R), c_int(r.K), c_int(x.shape[1]), ST())
     return xp

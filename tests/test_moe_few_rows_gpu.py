@@ -1,0 +1,73 @@
+"""Expert FFN of a few rows (decoding): one-CTA routing and expert products against the general path and fp64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+class _Bufs:
+    def get(self, name, shape, dtype=torch.bfloat16):
+        return torch.empty(shape, dtype=dtype, device="cuda")
+
+
+@pytest.mark.parametrize("R", [1, 2, 31, 32])
+@pytest.mark.parametrize("E,K", [(3, 2), (32, 1), (33, 5), (128, 8), (256, 16)])
+@pytest.mark.parametrize("norm", [True, False])
+def test_route_few_lays_out_like_route(R, E, K, norm):
+    from sensenova_u1_b200.ops import moe
+    g = torch.Generator(device="cuda").manual_seed(R * E)
+    logits = torch.randn(R, E, device="cuda", generator=g) * 2
+    a, b = moe.route_few(logits, K, norm, _Bufs()), moe.route(logits, K, norm)
+    assert torch.equal(a.top_idx, b.top_idx) and torch.equal(a.top_w, b.top_w) and torch.equal(a.dest, b.dest)
+    n = a.tile_group.numel()
+    assert n == min(R * K, E)
+    want = torch.full_like(a.tile_group, -1)
+    m = min(n, b.tile_group.numel())
+    want[:m] = b.tile_group[:m]
+    assert torch.equal(a.tile_group, want)
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17, 32])                       # row tiles of 16 and 32
+@pytest.mark.parametrize("N,K", [(24, 72), (200, 520), (768, 2048)])    # ragged and whole weight tiles
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_expert_products(rows, N, K, swiglu):
+    from sensenova_u1_b200.ops import _lib, gemm
+    g = torch.Generator(device="cuda").manual_seed(rows + N)
+    E, tg = 5, torch.tensor([4, 0, 2, -1], dtype=torch.int32, device="cuda")
+    x = torch.randn(4 * 128, K, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(E, N * (2 if swiglu else 1), K, device="cuda", generator=g) * K ** -0.5).to(torch.bfloat16)
+    out = gemm.gemm_experts(x, w, torch.full((4 * 128, N), 7.0, device="cuda", dtype=torch.bfloat16), tg, rows, swiglu=swiglu)
+    _lib.check_status()
+    for t, e in enumerate(tg.tolist()):
+        got = out[t * 128:t * 128 + rows].double()
+        if e < 0:
+            assert (out[t * 128:(t + 1) * 128] == 7).all()
+            continue
+        ref = x[t * 128:t * 128 + rows].double() @ w[e].double().t()
+        # fp32 sums, one rounding (2^-8 of the value); silu: both factors rounded first and the hardware tanh (2^-11)
+        if swiglu:
+            gate, up = ref[:, :N].to(torch.bfloat16).double(), ref[:, N:].to(torch.bfloat16).double()
+            ref = torch.nn.functional.silu(gate) * up
+            tol = ref.abs() * 2.0 ** -6 + (gate * up).abs() * 2.0 ** -10 + 1e-2
+        else:
+            tol = ref.abs() * 2.0 ** -8 + 1e-4
+        assert ((got - ref).abs() <= tol).all()
+
+
+def test_one_cta_path_equals_the_general_path(monkeypatch):
+    from sensenova_u1_b200.config import get_config
+    from sensenova_u1_b200.inference.engine import InferenceEngine
+    from sensenova_u1_b200.models.params import UND, ParamStore
+    from sensenova_u1_b200.ops import moe
+    cfg = get_config("a3b-mot", num_layers=1, num_experts=16, gen_num_experts=16)
+    store = ParamStore(cfg, device="cuda:0", with_grads=False)
+    store.init_weights(1)
+    eng = InferenceEngine(cfg, store)
+    x = torch.randn(32, cfg.hidden_size, device="cuda").to(torch.bfloat16)
+    W = lambda n: store.p["layers.0." + n]
+    outs = []
+    for few in (32, 0):
+        monkeypatch.setattr(moe, "FEW_ROWS", few)
+        outs.append(eng._moe_ffn(W, x, x, UND, torch.empty_like(x)).float())
+    # two bf16 roundings of the experts' outputs may differ by an ulp each
+    assert ((outs[0] - outs[1]).abs() <= outs[1].abs() * 2.0 ** -7 + 2e-2).all()
