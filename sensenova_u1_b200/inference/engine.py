@@ -286,13 +286,17 @@ class InferenceEngine:
         if not sampling.get("do_sample", False):
             return lg.argmax(-1)
         t = float(sampling.get("temperature", 1.0) or 1.0)
+        k = int(sampling.get("top_k", 0) or 0)
+        p_ = float(sampling.get("top_p", 1.0) or 1.0)
+        if (lg.is_cuda and lg.dim() == 2 and 0 < lg.shape[0] < 65536 and 0 < k < lg.shape[-1] and k <= fused.SAMPLER_MAX_K
+                and lg.shape[-1] <= fused.SAMPLER_MAX_VOCAB):
+            # the same draw in one launch: top-k first bounds what has to be sorted
+            return fused.sample_top_k_top_p(lg, torch.empty_like(lg).exponential_(1.0), t, k, p_)
         if t != 1.0:
             lg = lg / t
-        k = int(sampling.get("top_k", 0) or 0)
         if 0 < k < lg.shape[-1]:
             kth = torch.topk(lg, k, dim=-1).values[..., -1:]
             lg = lg.masked_fill(lg < kth, float("-inf"))
-        p_ = float(sampling.get("top_p", 1.0) or 1.0)
         if p_ < 1.0:
             srt, idx = torch.sort(lg, dim=-1, descending=True)
             cum = torch.softmax(srt, dim=-1).cumsum(-1)

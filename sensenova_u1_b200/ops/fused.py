@@ -132,6 +132,25 @@ def join_master(hi, lo, w32):
     _lib.call("join_master", P(hi), P(lo), P(w32), c_ll(w32.numel()), ST())
 
 
+# ---- token sampling (csrc/token_sampler.cu) ----------------------------------------------------------------
+SAMPLER_MAX_K, SAMPLER_MAX_VOCAB = 1024, 360_000      # sorted in one CTA; a row in the shared memory of eight
+
+
+def sample_top_k_top_p(logits, noise, temperature: float, k: int, top_p: float):
+    """Index per row of ``argmax(p / noise)``, with p the softmax of ``logits / temperature`` [rows, V] fp32 restricted to
+    the ``k`` largest (and their ties) and of those to the nucleus ``top_p``; ``noise`` ~ Exp(1), same shape."""
+    rows, V = logits.shape
+    if logits.stride(1) != 1:
+        logits = logits.contiguous()
+    if not (logits.dtype == noise.dtype == torch.float32 and noise.is_contiguous()
+            and noise.shape == logits.shape):
+        raise ValueError("logits and noise must be fp32 [rows, V]")
+    out = torch.empty(rows, dtype=torch.long, device=logits.device)
+    _lib.call("sample_top_k_top_p", P(logits), c_ll(logits.stride(0)), P(noise), P(out), c_int(rows), c_int(V), c_int(k),
+              c_float(1.0 / temperature), c_float(top_p), ST())
+    return out
+
+
 # ---- convolutional pixel head (csrc/pixel_head.cu) ---------------------------------------------------------
 def ps_im2col(x, A, h: int, w: int, C: int):
     """Pixel-shuffle(2) + 3x3 patch gather: x [h*w, 4C] -> A [(2h)(2w), 9C] (tap-major, channel-minor columns)."""
