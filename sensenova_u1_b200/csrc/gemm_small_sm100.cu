@@ -15,10 +15,10 @@
 // Measured (weights cold in L2, one launch in a chain, us; before = the 256 x 256 pair kernel, of whose 16 - 96 tiles
 // these shapes fill a fraction of the chip; floor = weight bytes at 6.65 TB/s):
 //   N x K            rows 1: before  now  floor    rows 24: before  now    rows 128: before  now
-//   6144 x 4096             27.8   11.5    7.6              27.6   12.9              29.0   20.0
-//   4096 x 4096             27.4    8.2    5.0              27.5   10.3              27.6   17.3
+//   6144 x 4096             27.8   11.5    7.6              27.6   12.9              29.0   16.7
+//   4096 x 4096             27.4    8.2    5.0              27.5   10.3              27.6   13.7
 //   24576 x 4096            63.4   35.2   30.3              54.1   36.3              56.1   43.5
-//   4096 x 12288            66.5   18.0   15.1              66.3   20.4              66.5   29.9
+//   4096 x 12288            66.5   18.0   15.1              66.3   20.4              66.5   25.3
 //   151936 x 4096          335.5  188.2  187.2             263.5  228.4             280.8  263.8
 #include <string.h>
 
@@ -35,11 +35,12 @@ constexpr int BK = 64;
 constexpr int W_STAGE = BW * BK * 2;       // 16 KB
 constexpr int NUM_THREADS = 192;           // warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
 
-template <int TN>
+// DEEP: one CTA per SM with the whole shared memory as its ring, for grids that do not fill the chip twice anyway.
+template <int TN, bool DEEP>
 struct Cfg {
   static constexpr int X_STAGE = TN * BK * 2;
   static constexpr int STAGE = W_STAGE + X_STAGE;
-  static constexpr int STAGES = TN <= 16 ? 6 : TN <= 32 ? 5 : TN <= 64 ? 4 : 3;   // two CTAs per SM
+  static constexpr int STAGES = (TN <= 16 ? 6 : TN <= 32 ? 5 : TN <= 64 ? 4 : 3) * (DEEP ? 2 : 1);
   static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
   static constexpr int TMEM = TN < 32 ? 32 : TN;
   static_assert(TN * BW * 4 <= STAGES * STAGE, "partial sums reuse the ring");
@@ -82,11 +83,11 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
 
 // SWIGLU: w holds args.N gate rows and then as many up rows; a tile is 64 of each and gives 64 columns of
 // silu(gate) * up (both rounded to bf16 first, as when the projection was stored).
-template <int TN, bool SWIGLU>
+template <int TN, bool SWIGLU, bool DEEP>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
     gemm_small_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                       const Args args) {
-  using C = Cfg<TN>;
+  using C = Cfg<TN, DEEP>;
   extern __shared__ uint8_t smem_raw[];
   // same window offset in every CTA of the cluster: the partial sums are read at this CTA's own offsets
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -288,15 +289,15 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
   }
 }
 
-template <int TN, bool SWIGLU>
+template <int TN, bool SWIGLU, bool DEEP>
 static int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a, int tiles, int mt, cudaStream_t st) {
-  using C = Cfg<TN>;
+  using C = Cfg<TN, DEEP>;
   int dev = 0;
   SNU1_CUDA_CHECK(cudaGetDevice(&dev));
   static std::once_flag once[64];
   cudaError_t err = cudaSuccess;
   std::call_once(once[dev & 63], [&]() {
-    err = cudaFuncSetAttribute(gemm_small_kernel<TN, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    err = cudaFuncSetAttribute(gemm_small_kernel<TN, SWIGLU, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
   });
   SNU1_CUDA_CHECK(err);
   cudaLaunchConfig_t cfg;
@@ -314,7 +315,7 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a,
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  SNU1_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_small_kernel<TN, SWIGLU>, tmW, tmX, a));
+  SNU1_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_small_kernel<TN, SWIGLU, DEEP>, tmW, tmX, a));
   return kHostOk;
 }
 
@@ -333,11 +334,15 @@ static int launch_gemm_small_any(const void* x, const void* w, void* c, int M, i
   const int tiles = (N + cn - 1) / cn;
   const int chunks = (K + BK - 1) / BK;
   if (split <= 0) {
-    // Split the reduction while the CTAs still fit the chip at two per SM.  Every part adds a pass over the partial
-    // sums, which grows with the rows of x: wide tiles keep at least 12 chunks (768 of the reduction) per part.
-    // 4096 x 4096 weights, 1 row, split 1 / 2 / 4 / 8: 20.9 / 11.9 / 9.1 / 8.2 us; 128 rows: 29.6 / 20.2 / 17.3 / 19.4.
+    // Split the reduction while the CTAs still fit the chip: at two per SM, or at one (with a ring of twice the depth)
+    // for wide row tiles, where a part also has a larger pass over the partial sums and keeps at least 12 chunks (768 of
+    // the reduction).  Powers of two: clusters of three were slower than two or four.
+    // 4096 x 4096 weights, 1 row, split 1 / 2 / 4 / 8: 20.9 / 11.9 / 9.1 / 8.2 us.
+    // 128 rows, us, two per SM (shallow) / one per SM (deep): 6144 x 4096 split 4 / 2: 21.0 / 16.7; 4096 x 4096 split 4:
+    // 14.5 / 13.7; 4096 x 12288 split 8 / 4: 31.1 / 25.3; 64 rows: 16.6 / 14.3, 12.1 / 11.7, 25.5 / 22.2.
+    const long long fit = tn >= 64 ? num_sms() : 2 * num_sms();
     split = 1;
-    while (split < 8 && tiles * mt * split * 2 <= 296 && chunks / (split * 2) >= (tn >= 64 ? 12 : 3)) split *= 2;
+    while (split < 8 && (long long)tiles * mt * split * 2 <= fit && chunks / (split * 2) >= (tn >= 64 ? 12 : 3)) split *= 2;
   }
   CUtensorMap tmW, tmX;
   int rc;
@@ -369,13 +374,14 @@ static int launch_gemm_small_any(const void* x, const void* w, void* c, int M, i
   a.alpha = alpha;
   a.w_static = w_static;
   a.status = device_status_word();
-#define SNU1_SMALL(TN) \
-  return swiglu ? launch<TN, true>(tmW, tmX, a, tiles, mt, st) : launch<TN, false>(tmW, tmX, a, tiles, mt, st)
+#define SNU1_SMALL(TN, DEEP)                                                   \
+  return swiglu ? launch<TN, true, DEEP>(tmW, tmX, a, tiles, mt, st) : launch<TN, false, DEEP>(tmW, tmX, a, tiles, mt, st)
+  const bool deep = tn >= 64 && (long long)tiles * mt * split <= num_sms();
   switch (tn) {
-    case 16: SNU1_SMALL(16);
-    case 32: SNU1_SMALL(32);
-    case 64: SNU1_SMALL(64);
-    default: SNU1_SMALL(128);
+    case 16: SNU1_SMALL(16, false);
+    case 32: SNU1_SMALL(32, false);
+    case 64: if (deep) SNU1_SMALL(64, true); SNU1_SMALL(64, false);
+    default: if (deep) SNU1_SMALL(128, true); SNU1_SMALL(128, false);
   }
 #undef SNU1_SMALL
 }
