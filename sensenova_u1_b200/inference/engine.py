@@ -140,9 +140,8 @@ class InferenceEngine:
         q = qf.unflatten(1, (cfg.num_heads, 128))
         o = ws.get("i.o", (R, cfg.num_heads, 128))
         of = o.view(R, qd)
-        lse = act = None
-        if not isinstance(plan, DecodeRows):
-            lse = ws.get("i.lse", (cfg.num_heads, R), torch.float32)
+        decode = isinstance(plan, DecodeRows)
+        act = None
         if not cfg.is_moe:
             act = ws.get("i.act", (R, cfg.ffn_size))
         for l in range(cfg.num_layers):
@@ -173,11 +172,11 @@ class InferenceEngine:
                 # back to this layer (next step) after the barriers of all later layers, i.e. after I read
                 self.sp["bar"].barrier()
             k, v = self.kc[l][:kv_len], self.vc[l][:kv_len]
-            if lse is None:
+            if decode:
                 attn_ops.attention_decode(q, k, v, plan.meta_q, plan.meta_k, plan.first, kv_rows, plan.max_keys,
                                           self.scale, o)
             else:
-                attn_ops.attention_fwd(q, k, v, plan, self.scale, out=o, lse=lse)
+                attn_ops.attention_fwd(q, k, v, plan, self.scale, out=o, want_lse=False)
             gemm.gemm_nt(of, W("wo"), out=x1, residual=x, w_static=static)
             fused.rmsnorm_fwd(x1, W("ffn_norm"), None, h2, None, cfg.rms_eps)
             if not cfg.is_moe:

@@ -151,9 +151,10 @@ def _check_heads(t, name):
         raise ValueError(f"{name} must be CUDA bf16 [S, H, 128] with contiguous heads")
 
 
-def attention_fwd(q, k, v, plan: TilePlan, scale: float, out=None, lse=None):
+def attention_fwd(q, k, v, plan: TilePlan, scale: float, out=None, lse=None, want_lse: bool = True):
     """Returns ``(out [Sq,Hq,128] bf16, lse [Hq,Sq] fp32 in log2 units)``.
-    ``q``/``k``/``v`` may be column slices of wider row-major buffers."""
+    ``q``/``k``/``v`` may be column slices of wider row-major buffers.  ``want_lse=False``: no backward pass will follow;
+    ``lse`` is None and a faster kernel runs, whose roundings differ."""
     for t, nme in ((q, "q"), (k, "k"), (v, "v")):
         _check_heads(t, nme)
     Sq, Hq, _ = q.shape
@@ -161,11 +162,13 @@ def attention_fwd(q, k, v, plan: TilePlan, scale: float, out=None, lse=None):
     assert Sq == plan.Sq and Sk == plan.Sk and v.shape[0] == Sk
     if out is None:
         out = torch.empty(Sq, Hq, 128, dtype=torch.bfloat16, device=q.device)
-    if lse is None:
+    if not want_lse:
+        lse = None
+    elif lse is None:
         lse = torch.empty(Hq, Sq, dtype=torch.float32, device=q.device)
     _lib.call("attn_fwd", c_void_p(q.data_ptr()), c_ll(q.stride(0)), c_void_p(k.data_ptr()),
               c_ll(k.stride(0)), c_void_p(v.data_ptr()), c_ll(v.stride(0)),
-              c_void_p(out.data_ptr()), c_ll(out.stride(0)), c_void_p(lse.data_ptr()),
+              c_void_p(out.data_ptr()), c_ll(out.stride(0)), _optr(lse),
               c_void_p(plan.meta_q.data_ptr()), c_void_p(plan.meta_k.data_ptr()),
               c_void_p(plan.pair_list.data_ptr()), c_void_p(plan.pair_count.data_ptr()),
               c_int(Sq), c_int(Sk), c_int(Hq), c_int(Hkv), c_float(scale), *plan._mask_ptrs()[:2],
