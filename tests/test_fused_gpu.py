@@ -310,3 +310,31 @@ def test_rmsnorm_fwd_row_kernel(rows, H):
     ref = oracle.rmsnorm(x.float(), gain.float()[tg.clamp(min=0).repeat_interleave(128)[:rows].long()], 1e-6)
     assert ((y.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all()
     torch.testing.assert_close(rstd, torch.rsqrt(x.float().pow(2).mean(1) + 1e-6), rtol=1e-5, atol=0)
+
+
+@pytest.mark.parametrize("rows", [1, 15, 17, 300])                              # CTAs of 16 rows
+@pytest.mark.parametrize("n_q,n_kv", [(2, 1), (32, 8), (32, 4), (40, 9)])        # odd head counts, one and two steps per row
+def test_qknorm_rope_bwd_wide_equals_narrow(rows, n_q, n_kv):
+    """Rows that are only 8-byte aligned take the kernel of four elements per lane: the same gradients."""
+    from sensenova_u1_b200.config import tiny_mot
+    from sensenova_u1_b200.models import oracle
+    from sensenova_u1_b200.ops import fused
+    cfg = tiny_mot(head_dim=128, patch_size=16)
+    inv_t, inv_hw = (t.contiguous() for t in oracle.rope_inv_freq(cfg, DEV))
+    W = (n_q + 2 * n_kv) * 128
+    gains = (1 + 0.1 * torch.randn(3, 4, 64, device=DEV)).to(torch.bfloat16)
+    tg = torch.tensor([2, -1, 1], dtype=torch.int32, device=DEV)                 # -1: no gain gradient
+    pos3 = torch.randint(0, 3000, (3, rows), device=DEV, dtype=torch.int32)
+    out = []
+    for pad in (8, 4):
+        qkv, d = (torch.full((rows, W + pad), 9.0, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+        qkv[:, :W], d[:, :W] = _bf(rows, W, seed=rows), _bf(rows, W, seed=7)
+        dg = torch.zeros(3, 4, 64, device=DEV)
+        fused.qknorm_rope_bwd(qkv[:, :W], d[:, :W], gains, dg, tg, pos3, inv_t, inv_hw, n_q, n_kv, 1e-6)
+        assert (d[:, W:] == 9).all()
+        out.append((d[:, :W].float(), dg))
+    (a, da), (b, db) = out
+    assert torch.equal(a[:, (n_q + n_kv) * 128:], b[:, (n_q + n_kv) * 128:])     # v is not touched
+    # sums of 64 in another order: one rounding to bf16 apart (2^-7 of the value), cancellation near zero
+    assert ((a - b).abs() <= b.abs() * 2.0 ** -7 + 1e-4).all()
+    assert ((da - db).abs() <= db.abs() * 1e-4 + 1e-3).all() and (da[0] == 0).all()
