@@ -551,6 +551,30 @@ SNU1_API int snu1_moe_gather(const void* x, const int* dest, const int* top_idx,
   return kHostOk;
 }
 
+// Clears the rows of a that pad expert e's segment, [seg_start[e] + counts[e], seg_end[e]).  A weight gradient reduces over
+// whole segments, so these rows (and no others) have to be zero.
+namespace snu1 {
+__global__ void __launch_bounds__(256)
+    moe_zero_pads_kernel(__nv_bfloat16* __restrict__ a, const int* __restrict__ counts, const int* __restrict__ seg_start,
+                         const int* __restrict__ seg_end, int H, int max_rows) {
+  const int e = blockIdx.x, hv = H / 8;
+  const long long lo = (long long)(seg_start[e] + counts[e]) * hv, hi = (long long)min(seg_end[e], max_rows) * hv;
+  for (long long i = lo + threadIdx.x + blockIdx.y * 256; i < hi; i += 256 * gridDim.y)
+    reinterpret_cast<uint4*>(a)[i] = make_uint4(0, 0, 0, 0);
+}
+}  // namespace snu1
+SNU1_API int snu1_moe_zero_pads(void* a, const int* counts, const int* seg_start, const int* seg_end, int E, int H,
+                                int max_rows, void* stream) {
+  if (H % 8 || E <= 0 || max_rows <= 0) {
+    set_last_error("moe_zero_pads: bad sizes E=%d H=%d", E, H);
+    return kHostBadArg;
+  }
+  moe_zero_pads_kernel<<<dim3(E, 4), 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)a, counts, seg_start, seg_end, H,
+                                                                     max_rows);
+  SNU1_CUDA_CHECK(cudaGetLastError());
+  return kHostOk;
+}
+
 SNU1_API int snu1_moe_combine(const void* yp, const int* dest, const int* top_idx, const float* top_w,
                               const void* residual, void* y, int R, int K, int H, void* stream) {
   if (H % 8) {

@@ -14,7 +14,7 @@ import torch
 
 from ..data.batch import KIND_PAD, KIND_UND_IMG, PackedBatch
 from ..ops import fused, gemm, moe
-from ..ops.gemm import OUT_BF16_ACC, OUT_F32_STORE
+from ..ops.gemm import OUT_BF16_ACC, OUT_BF16_STORE, OUT_F32_STORE
 from .engine import MoTEngine
 
 
@@ -115,11 +115,11 @@ class MoEMoTEngine(MoTEngine):
             logits = gemm.gemm_nt(hb, p[s + f"moe_{br}.gate"], out=ws.get(f"moe.{br}.logits", (R, E), torch.float32),
                                   out_mode=OUT_F32_STORE)
             r = self._route(logits, K, lo, hi, br, _Prefixed(ws, f"moe.{br}."))
-            xp = ws.get(f"moe.{br}.xp", (r.max_rows, H), zero=True)
+            xp = moe.zero_pads(ws.get(f"moe.{br}.xp", (r.max_rows, H)), r)
             moe.gather(hb, r, xp)
             gu = gemm.gemm_nt(xp, p[s + f"moe_{br}.w13"], out=ws.get(f"moe.{br}.gu", (r.max_rows, 2 * Fe)),
                               tile_group=r.tile_group)
-            act = fused.swiglu_fwd(gu, ws.get(f"moe.{br}.act", (r.max_rows, Fe)))
+            act = fused.swiglu_fwd(gu, ws.get(f"moe.{br}.act", (r.max_rows, Fe)), rows_dev=r.total_rows)
             yp = gemm.gemm_nt(act, p[s + f"moe_{br}.w2"], out=ws.get(f"moe.{br}.yp", (r.max_rows, H)),
                               tile_group=r.tile_group)
             if out is not None:
@@ -296,26 +296,32 @@ class MoEMoTEngine(MoTEngine):
         S, H = dy.shape
         Fe = cfg.moe_intermediate_size
         d_h2 = ws.get("d_h", (S, H), zero=True)
+        wmode = self._wgrad_mode(l)
+        if wmode == OUT_BF16_STORE:              # a branch without rows in this batch has no product that would store
+            for br in ("gen", "und"):
+                if br not in a["moe"]:
+                    for n in ("gate", "w13", "w2"):
+                        g[s + f"moe_{br}.{n}"].zero_()
         for br, sv in a["moe"].items():
             r, lo, hi, E, K = sv["r"], sv["lo"], sv["hi"], sv["E"], sv["K"]
             R = hi - lo
-            d_yp = ws.get(f"moe.{br}.d_yp", (r.max_rows, H), zero=True)
+            d_yp = moe.zero_pads(ws.get(f"moe.{br}.d_yp", (r.max_rows, H)), r)
             dw = ws.get(f"moe.{br}.dw", (R, K), torch.float32)
             moe.combine_bwd(dy[lo:hi], sv["yp"], r, d_yp, dw)
             d_act = gemm.gemm_nn(d_yp, p[s + f"moe_{br}.w2"], out=ws.get(f"moe.{br}.d_act", (r.max_rows, Fe)),
                                  tile_group=r.tile_group)
             gemm.gemm_tn(d_yp, sv["act"], out=g[s + f"moe_{br}.w2"], k_begin=r.seg_start, k_end=r.seg_end,
-                         num_groups=E, out_mode=OUT_BF16_ACC)
-            d_gu = fused.swiglu_bwd(sv["gu"], d_act, ws.get(f"moe.{br}.d_gu", (r.max_rows, 2 * Fe)))
+                         num_groups=E, out_mode=wmode)
+            d_gu = fused.swiglu_bwd(sv["gu"], d_act, ws.get(f"moe.{br}.d_gu", (r.max_rows, 2 * Fe)), rows_dev=r.total_rows)
             d_xp = gemm.gemm_nn(d_gu, p[s + f"moe_{br}.w13"], out=ws.get(f"moe.{br}.d_xp", (r.max_rows, H)),
                                 tile_group=r.tile_group)
             gemm.gemm_tn(d_gu, sv["xp"], out=g[s + f"moe_{br}.w13"], k_begin=r.seg_start, k_end=r.seg_end,
-                         num_groups=E, out_mode=OUT_BF16_ACC)
+                         num_groups=E, out_mode=wmode)
             moe.gather_bwd(d_xp, r, d_h2[lo:hi])
             dlog = self._router_bwd(r, dw, br, E, K, ws.get(f"moe.{br}.dlog", (R, E)))
             hb = a["h2"][lo:hi]
             gemm.gemm_nn(dlog, p[s + f"moe_{br}.gate"], out=d_h2[lo:hi], out_mode=OUT_BF16_ACC)
-            gemm.gemm_tn(dlog, hb, out=g[s + f"moe_{br}.gate"], out_mode=OUT_BF16_ACC)
+            gemm.gemm_tn(dlog, hb, out=g[s + f"moe_{br}.gate"], out_mode=wmode)
         return d_h2
 
     _aux_grad_scale = 1.0

@@ -96,6 +96,13 @@ def gather(x, r: Routing, xp):
     return xp
 
 
+def zero_pads(a, r: Routing):
+    """Clears the rows of ``a`` [max_rows, H] that pad the experts' segments to 128 rows."""
+    _lib.call("moe_zero_pads", P(a), P(r.counts), P(r.seg_start), P(r.seg_end), c_int(r.E), c_int(a.shape[1]),
+              c_int(r.max_rows), ST())
+    return a
+
+
 def combine(yp, r: Routing, residual, y):
     _lib.call("moe_combine", P(yp), P(r.dest), P(r.top_idx), P(r.top_w), P(residual), P(y), c_int(r.R),
               c_int(r.K), c_int(y.shape[1]), ST())

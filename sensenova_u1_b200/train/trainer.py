@@ -134,11 +134,12 @@ class Trainer:
                        noise: Optional[Sequence[torch.Tensor]] = None):
         """Same step for batches that already live on the device; returns device scalars."""
         ce_norm, gen_norm = self._normalisers(batches)
-        # plain dense engine: the first micro-batch stores the layers' weight gradients, so they are not cleared
+        # one-rank-per-layer engines: the first micro-batch stores the layers' weight gradients, so they are not cleared
         store_first = (getattr(self, "store_first_enabled", True) and self.engine is not None
-                       and type(self.engine).__name__ == "MoTEngine" and self.wp is None
+                       and type(self.engine).__name__ in ("MoTEngine", "MoEMoTEngine") and self.wp is None
+                       and getattr(self.engine, "ep", None) is None
                        and getattr(self.engine, "cp", None) is None and getattr(self.engine, "tp", None) is None
-                       and not self.optim.cfg.frozen and not self.store.cfg.is_moe
+                       and not self.optim.cfg.frozen
                        and type(self.store).__name__ == "ParamStore")
         self.store.zero_grads(keep_layer_matrices=True) if store_first else self.store.zero_grads()
         acc = None
