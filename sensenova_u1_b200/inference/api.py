@@ -219,8 +219,9 @@ class NEOChatModel:
             image_size = (images[0].shape[2], images[0].shape[1])
         tags = "<image>\n" * len(images)
         tail = f"{prompts.THINK_START}\n\n{prompts.THINK_END}\n\n{prompts.IMG_START_TOKEN}"
-        full = self._embed_prompt(tokenizer, tags + prompt, images, system=prompts.SYSTEM_MESSAGE_FOR_GEN, tail=tail)
-        img_only = self._embed_prompt(tokenizer, tags, images, system=prompts.SYSTEM_MESSAGE_FOR_GEN, tail=tail)
+        embs = self._embed_images(images)               # both branches show the same pictures
+        full = self._embed_prompt(tokenizer, tags + prompt, images, system=prompts.SYSTEM_MESSAGE_FOR_GEN, tail=tail, embs=embs)
+        img_only = self._embed_prompt(tokenizer, tags, images, system=prompts.SYSTEM_MESSAGE_FOR_GEN, tail=tail, embs=embs)
         un_ids = _encode(tokenizer, prompts.render_chat([("user", ""), ("assistant", None)]) + prompts.IMG_START_TOKEN)
         sample = [full, (un_ids, None, None), img_only]
         return self.engine.denoise([sample] * batch_size, tuple(image_size), num_steps, cfg_scale, img_cfg_scale,
@@ -277,12 +278,22 @@ class NEOChatModel:
         return self.interleave_gen(tokenizer, prompt, images, **kw)[1]
 
     # ---- understanding ------------------------------------------------------------
-    def _embed_prompt(self, tokenizer, question: str, images: Sequence[torch.Tensor], system=None, tail: str = "",
-                      history: Sequence[Tuple[str, str]] = ()):
-        """Token ids, embeddings and (t,h,w) indexes of a prompt with ``<image>`` placeholders
-        (also inside ``tail``, the already generated part of the assistant turn)."""
+    def _embed_images(self, images: Sequence[torch.Tensor]):
+        """Understanding-branch embeddings of [3,H,W] pictures; the pixels are put into patch order on the device."""
         from ..data.batch import patchify_block_major
-        cfg, eng = self.cfg, self.engine
+        cfg, dev = self.cfg, self.store.device
+        embs = []
+        for im in images:
+            p16, px, py, _, _ = patchify_block_major(im.to(dev).float(), cfg.patch_size, cfg.merge_size)
+            embs.append(self.engine.vision_embed("und", p16.to(torch.bfloat16), px.to(dev), py.to(dev)))
+        return embs
+
+    def _embed_prompt(self, tokenizer, question: str, images: Sequence[torch.Tensor], system=None, tail: str = "",
+                      history: Sequence[Tuple[str, str]] = (), embs=None):
+        """Token ids, embeddings and (t,h,w) indexes of a prompt with ``<image>`` placeholders
+        (also inside ``tail``, the already generated part of the assistant turn).  ``embs``: :meth:`_embed_images` of
+        ``images``, for several prompts about the same pictures."""
+        cfg = self.cfg
         tp = cfg.token_pixels
         counts = [(im.shape[1] // tp) * (im.shape[2] // tp) for im in images]
         history, text, tail = prompts.expand_conversation(list(history), question, tail, counts)
@@ -295,12 +306,11 @@ class NEOChatModel:
         is_ctx = (ids == ctx_id)
         pos3 = self.get_thw_indexes(ids, [(im.shape[1] // tp, im.shape[2] // tp) for im in images], ctx_id)
         if images:
-            embs = []
-            for im in images:
-                p16, px, py, _, _ = patchify_block_major(im.float(), cfg.patch_size, cfg.merge_size)
-                embs.append(eng.vision_embed("und", p16.to(dev, torch.bfloat16), px.to(dev), py.to(dev)))
-            x = x.clone()
-            x[is_ctx.to(dev)] = torch.cat(embs)
+            rows = is_ctx.nonzero().view(-1)
+            embs = torch.cat(self._embed_images(images) if embs is None else embs)
+            if rows.numel() != embs.shape[0]:
+                raise ValueError(f"{rows.numel()} image tokens in the prompt, {embs.shape[0]} embeddings")
+            x.index_copy_(0, rows.to(dev), embs)        # x is this call's own copy of the embedding rows
         return ids, x, pos3
 
     def extract_feature(self, pixel_values, gen_model: bool = False, grid_hw=None) -> torch.Tensor:
@@ -355,23 +365,25 @@ class NEOChatModel:
     def get_thw_indexes(ids: torch.Tensor, grids: Sequence[Tuple[int, int]], ctx_id: int) -> torch.Tensor:
         """(t,h,w) per token: text advances t by one; all tokens of an image share the next t and
         carry their grid row / column (modeling_neo_chat.py:1977-1992)."""
-        n = ids.numel()
-        t = torch.zeros(n, dtype=torch.int32)
-        h = torch.zeros(n, dtype=torch.int32)
-        w = torch.zeros(n, dtype=torch.int32)
+        t, h, w = [], [], []
         cur, i, g = 0, 0, 0
         flags = (ids == ctx_id).tolist()
+        n = len(flags)
         while i < n:
             if not flags[i]:
-                t[i] = cur; cur += 1; i += 1
-                continue
-            gh, gw = grids[g]; g += 1
-            cnt = gh * gw
-            t[i:i + cnt] = cur
-            idx = torch.arange(cnt)
-            h[i:i + cnt] = (idx // gw).int(); w[i:i + cnt] = (idx % gw).int()
-            cur += 1; i += cnt
-        return torch.stack([t, h, w])
+                t.append(cur); h.append(0); w.append(0)
+                i += 1
+            else:
+                gh, gw = grids[g]; g += 1
+                cnt = gh * gw
+                if cnt > n - i:
+                    raise ValueError(f"image of {gh} x {gw} tokens, but {n - i} positions are left in the prompt")
+                t += [cur] * cnt
+                h += [j // gw for j in range(cnt)]
+                w += [j % gw for j in range(cnt)]
+                i += cnt
+            cur += 1
+        return torch.tensor([t, h, w], dtype=torch.int32)
 
     @staticmethod
     def _sampling(gc: dict) -> Optional[dict]:
