@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
       const uint64_t k_desc = make_smem_desc(smem_u32(sK), 0, 1024), v_desc = make_smem_desc(smem_u32(sV), 0, 1024);
       const uint64_t kt_desc = make_smem_desc(smem_u32(sK), HALF_BYTES, 1024);
       constexpr uint32_t tile = TILE_BYTES >> 4, half_tile = HALF_BYTES >> 4;
-      bool ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0, abort_flag, args.status, 3));
+      bool ok = mbar_wait_warp(q_full, 0, abort_flag, args.status, 3);
       auto issue_s = [&](int j) {
         const uint64_t kd = k_desc + (j & 1) * tile;
 #pragma unroll
@@ -280,14 +280,11 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
     const float dl = row_ok ? args.delta[(long long)head * args.Sq + row] : 0.f;
     const float sc2 = args.scale_log2, sc = args.scale;
     bool ok = true;
-    for (int j = 0; j < n && ok; ++j) {
+    for (int j = 0; j < n; ++j) {       // the whole list also after a time-out, see mbar_wait_warp
       const int entry = list[j];
       const bool partial = list_class(entry) != kTileFull;
       const int k0 = list_tile(entry) * 128 + half * 64;
-      if (!mbar_wait(s_full, j & 1, abort_flag, args.status, 5)) {
-        ok = false;
-        break;
-      }
+      ok &= mbar_wait(s_full, j & 1, abort_flag, args.status, 5);
       tc_fence_after();
       float p[64];
       {
@@ -339,14 +336,8 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
           p[c + 1] = fast_exp2(x1);
         }
       }
-      if (!mbar_wait(dp_full, j & 1, abort_flag, args.status, 5)) {
-        ok = false;
-        break;
-      }
-      if (j > 0 && !mbar_wait(ds_done, (j - 1) & 1, abort_flag, args.status, 5)) {
-        ok = false;
-        break;
-      }
+      ok &= mbar_wait(dp_full, j & 1, abort_flag, args.status, 5);
+      if (j > 0) ok &= mbar_wait(ds_done, (j - 1) & 1, abort_flag, args.status, 5);
       tc_fence_after();
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -382,7 +373,8 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_full);
     }
-    if (ok && mbar_wait(ds_done, (n - 1) & 1, abort_flag, args.status, 5)) {
+    ok &= mbar_wait(ds_done, (n - 1) & 1, abort_flag, args.status, 5);
+    if (__all_sync(0xffffffffu, ok)) {
       tc_fence_after();
 #pragma unroll 1
       for (int c = half * 2; c < half * 2 + 2; ++c) {
@@ -565,7 +557,7 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
       const uint64_t qt_desc = make_smem_desc(smem_u32(sQ), SUB_HALF, 1024), dot_desc = make_smem_desc(smem_u32(sdO), SUB_HALF, 1024);
       const uint64_t pt_desc = make_smem_desc(smem_u32(sPT), 0, 1024), dst_desc = make_smem_desc(smem_u32(sdST), 0, 1024);
       constexpr uint32_t sub = SUB_TILE >> 4;
-      bool ok = __all_sync(0xffffffffu, mbar_wait(kv_full, 0, abort_flag, args.status, 3));
+      bool ok = mbar_wait_warp(kv_full, 0, abort_flag, args.status, 3);
       auto issue_sdp = [&](int i) {
         const int s = i & 1, qs = i % DKV_STAGES;
         const uint64_t qd = q_desc + qs * sub, dod = do_desc + qs * sub;
@@ -648,15 +640,12 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
     TokMeta mk = krow_ok ? args.meta_k[krow] : TokMeta{-2, 0, 0, kFlagBlocked};
     const float sc2 = args.scale_log2, sc = args.scale;
     bool ok = true;
-    for (int i = 0; i < n && ok; ++i) {
+    for (int i = 0; i < n; ++i) {
       const int s = i & 1;
       int qrow0, qh, entry;
       decode(i, qrow0, qh, entry);
       const bool fast = list_class(entry) == kTileFull && tile_rows_ok;
-      if (!mbar_wait(&sdp_full[s], (i >> 1) & 1, abort_flag, args.status, 5)) {
-        ok = false;
-        break;
-      }
+      ok &= mbar_wait(&sdp_full[s], (i >> 1) & 1, abort_flag, args.status, 5);
       tc_fence_after();
       uint32_t st[32], dp[32];
       tmem_ld_32x32b_x32(tmem_ST + s * 64 + half * 32 + lane_sel, st);
@@ -701,10 +690,7 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
           dk[c >> 1] = pack_bf16x2(d0, d1);
         }
       }
-      if (i > 0 && !mbar_wait(pds_done, (i - 1) & 1, abort_flag, args.status, 5)) {
-        ok = false;
-        break;
-      }
+      if (i > 0) ok &= mbar_wait(pds_done, (i - 1) & 1, abort_flag, args.status, 5);
 #pragma unroll
       for (int ch = 0; ch < 4; ++ch) {
         const uint32_t off = swz128_offset(rloc, half * 4 + ch);
@@ -716,7 +702,8 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(pds_full);
     }
-    if (ok && mbar_wait(pds_done, (n - 1) & 1, abort_flag, args.status, 5)) {
+    ok &= mbar_wait(pds_done, (n - 1) & 1, abort_flag, args.status, 5);
+    if (__all_sync(0xffffffffu, ok)) {
       tc_fence_after();
       // each of the two warps of a lane quarter writes half of the 128 output columns
 #pragma unroll 1

@@ -356,16 +356,13 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
     const float sc = args.scale_log2;
     bool ok = true;
     int cnt = 0;  // key tiles this query tile has processed
-    for (int j = 0; j < n && ok; ++j) {
+    for (int j = 0; j < n; ++j) {        // the whole list also after a time-out, see mbar_wait_warp
       const int entry = list[j];
       const int cls_t = (entry >> (24 + 2 * t)) & 3;
       if (cls_t == kTileSkip) continue;
       const bool partial = cls_t != kTileFull;
       const int k0 = list_tile(entry) * BKV;
-      if (!mbar_wait(&s_full[t], cnt & 1, abort_flag, args.status, 5)) {
-        ok = false;
-        break;
-      }
+      ok &= mbar_wait(&s_full[t], cnt & 1, abort_flag, args.status, 5);
       tc_fence_after();
       float sv[128];
       {
@@ -470,10 +467,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
       l = l * alpha + sum;
       m = m_new;
       if (cnt > 0) {
-        if (!mbar_wait(&pv_done[t], (cnt - 1) & 1, abort_flag, args.status, 5)) {
-          ok = false;
-          break;
-        }
+        ok &= mbar_wait(&pv_done[t], (cnt - 1) & 1, abort_flag, args.status, 5);
         tc_fence_after();
       }
 #pragma unroll
@@ -509,6 +503,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
       if (lane == 0) mbar_arrive(&p_full[t]);
       ++cnt;
     }
+    if (cnt > 0) ok &= mbar_wait(&pv_done[t], (cnt - 1) & 1, abort_flag, args.status, 5);
+    ok = __all_sync(0xffffffffu, ok);
     if (cnt == 0) {
       // no key tile at all for this query tile: zero output
       if (ok && row < args.Sq) {
@@ -518,7 +514,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
         for (int i = 0; i < 16; ++i) op[i] = z;
         args.lse[(long long)head * args.Sq + row] = __int_as_float(0x7f800000);
       }
-    } else if (ok && mbar_wait(&pv_done[t], (cnt - 1) & 1, abort_flag, args.status, 5)) {
+    } else if (ok) {
       tc_fence_after();
       const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll 1

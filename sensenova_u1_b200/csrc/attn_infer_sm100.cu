@@ -76,7 +76,7 @@ __device__ __forceinline__ bool count_wait(const int* c, int target, volatile in
     int v;
     asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     if (v >= target) return true;
-    if ((spins & 0x3ff) == 0x3ff) {
+    if ((spins & 0x3ff) == 1) {
       if (*abort_flag) return false;
       const uint64_t now = globaltimer_ns();
       if (t0 == 0) t0 = now;
@@ -200,46 +200,46 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
       const uint64_t q_desc = make_smem_desc(smem_u32(sQ), 0, 1024);
       const uint64_t k_desc = make_smem_desc(smem_u32(sK), 0, 1024);
       const uint64_t v_desc = make_smem_desc(smem_u32(sV), HALF_BYTES, 1024);
-      bool ok = mbar_wait(q_full, 0, abort_flag, args.status, 3);
+      bool ok = mbar_wait(q_full, 0, abort_flag, args.status, 3);   // this lane's; see mbar_wait_warp
       int s_cnt[2] = {0, 0};   // S products issued per query tile
       int pv_cnt[2] = {0, 0};  // PV products issued per query tile
-      auto issue_s = [&](int entry, int j, int t) -> bool {
-        if (((entry >> (24 + 2 * t)) & 3) == kTileSkip) return true;
-        // the softmax warps must have drained the previous S of this tile
-        if (!mbar_wait(&s_empty[t], (s_cnt[t] & 1) ^ 1, abort_flag, args.status, 2)) return false;
-        tc_fence_after();
-        const uint64_t qd = q_desc + t * (TILE_BYTES >> 4), kd = k_desc + (j % K_STAGES) * (TILE_BYTES >> 4);
-        __syncwarp();
-        if (elect_one()) {
+      auto issue_s = [&](int entry, int j, int t) {
+        if (((entry >> (24 + 2 * t)) & 3) != kTileSkip) {
+          // the softmax warps must have drained the previous S of this tile
+          ok &= mbar_wait(&s_empty[t], (s_cnt[t] & 1) ^ 1, abort_flag, args.status, 2);
+          tc_fence_after();
+          const uint64_t qd = q_desc + t * (TILE_BYTES >> 4), kd = k_desc + (j % K_STAGES) * (TILE_BYTES >> 4);
+          __syncwarp();
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            constexpr uint32_t half = HALF_BYTES >> 4;
-            const uint32_t off = (k >> 2) * half + (k & 3) * 2;
-            umma_bf16_ss(tmem_base + t * 128, qd + off, kd + off, idesc_s, k > 0 ? 1u : 0u);
+            for (int k = 0; k < 8; ++k) {
+              constexpr uint32_t half = HALF_BYTES >> 4;
+              const uint32_t off = (k >> 2) * half + (k & 3) * 2;
+              umma_bf16_ss(tmem_base + t * 128, qd + off, kd + off, idesc_s, k > 0 ? 1u : 0u);
+            }
+            umma_commit(&s_full[t]);
           }
-          umma_commit(&s_full[t]);
+          __syncwarp();
+          ++s_cnt[t];
         }
-        __syncwarp();
-        ++s_cnt[t];
-        return true;
       };
-      auto issue_pv = [&](int entry, int j, int t) -> bool {
-        if (((entry >> (24 + 2 * t)) & 3) == kTileSkip) return true;
-        if (!mbar_wait(&p_full[t], pv_cnt[t] & 1, abort_flag, args.status, 2)) return false;
-        tc_fence_after();
-        const uint64_t vd = v_desc + (j % V_STAGES) * (TILE_BYTES >> 4);
-        const uint32_t p_tmem = tmem_base + (t ^ 1) * 128;      // in the other tile's score columns
-        const uint32_t acc0 = pv_cnt[t] > 0 ? 1u : 0u;
-        __syncwarp();
-        if (elect_one()) {
+      auto issue_pv = [&](int entry, int j, int t) {
+        if (((entry >> (24 + 2 * t)) & 3) != kTileSkip) {
+          ok &= mbar_wait(&p_full[t], pv_cnt[t] & 1, abort_flag, args.status, 2);
+          tc_fence_after();
+          const uint64_t vd = v_desc + (j % V_STAGES) * (TILE_BYTES >> 4);
+          const uint32_t p_tmem = tmem_base + (t ^ 1) * 128;      // in the other tile's score columns
+          const uint32_t acc0 = pv_cnt[t] > 0 ? 1u : 0u;
+          __syncwarp();
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            umma_bf16_ts(tmem_base + 256 + t * 128, p_tmem + k * 8, vd + k * (2048 >> 4), idesc_pv, k > 0 ? 1u : acc0);
-          umma_commit(&pv_done[t]);
+            for (int k = 0; k < 8; ++k)
+              umma_bf16_ts(tmem_base + 256 + t * 128, p_tmem + k * 8, vd + k * (2048 >> 4), idesc_pv, k > 0 ? 1u : acc0);
+            umma_commit(&pv_done[t]);
+          }
+          __syncwarp();
+          ++pv_cnt[t];
         }
-        __syncwarp();
-        ++pv_cnt[t];
-        return true;
       };
       auto release = [&](uint64_t* bar) {
         if (elect_one()) umma_commit(bar);
@@ -250,25 +250,28 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
       // stored over an S that has been read.  The two tiles run half a step apart: one takes exponentials while the
       // other loads, reduces and stores.
       int e = list[0], e1 = n > 1 ? list[1] : 0;      // entries of this step and the next (read a step ahead)
-      ok = ok && mbar_wait(&k_full[0], 0, abort_flag, args.status, 3) && issue_s(e, 0, 0) && issue_s(e, 0, 1);
-      if (ok) release(&k_empty[0]);
-      if (ok && n > 1) ok = mbar_wait(&k_full[1], 0, abort_flag, args.status, 3);
-      if (ok) ok = mbar_wait(&v_full[0], 0, abort_flag, args.status, 3);
-      for (int j = 0; j < n && ok; ++j) {
+      ok &= mbar_wait(&k_full[0], 0, abort_flag, args.status, 3);
+      issue_s(e, 0, 0);
+      issue_s(e, 0, 1);
+      release(&k_empty[0]);
+      if (n > 1) ok &= mbar_wait(&k_full[1], 0, abort_flag, args.status, 3);
+      ok &= mbar_wait(&v_full[0], 0, abort_flag, args.status, 3);
+      for (int j = 0; j < n; ++j) {      // the whole list also after a time-out
         const bool more = j + 1 < n;
         const int e2 = j + 2 < n ? list[j + 2] : 0;
-        if (more) ok = issue_s(e1, j + 1, 0);
-        ok = ok && issue_pv(e, j, 0);
-        if (more && ok) {
-          ok = issue_s(e1, j + 1, 1);
-          if (ok) release(&k_empty[(j + 1) % K_STAGES]);
+        if (more) issue_s(e1, j + 1, 0);
+        issue_pv(e, j, 0);
+        if (more) {
+          issue_s(e1, j + 1, 1);
+          release(&k_empty[(j + 1) % K_STAGES]);
         }
-        ok = ok && issue_pv(e, j, 1);
-        if (!ok || !more) break;
-        release(&v_empty[j % V_STAGES]);
-        // the next step's operands, waited for while the products just issued run
-        if (j + 2 < n) ok = mbar_wait(&k_full[(j + 2) % K_STAGES], ((j + 2) / K_STAGES) & 1, abort_flag, args.status, 3);
-        ok = ok && mbar_wait(&v_full[(j + 1) % V_STAGES], ((j + 1) / V_STAGES) & 1, abort_flag, args.status, 3);
+        issue_pv(e, j, 1);
+        if (more) {
+          release(&v_empty[j % V_STAGES]);
+          // the next step's operands, waited for while the products just issued run
+          if (j + 2 < n) ok &= mbar_wait(&k_full[(j + 2) % K_STAGES], ((j + 2) / K_STAGES) & 1, abort_flag, args.status, 3);
+          ok &= mbar_wait(&v_full[(j + 1) % V_STAGES], ((j + 1) / V_STAGES) & 1, abort_flag, args.status, 3);
+        }
         e = e1;
         e1 = e2;
       }
@@ -298,16 +301,13 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
     int next = n > 0 ? list[0] : 0;          // read a step ahead
     // score tiles of the other query tile that are issued before PV_t(j): key tiles 0 .. j of B for A, 0 .. j + 1 of A for B
     int other = t == 1 && ((next >> 24) & 3) != kTileSkip;
-    for (int j = 0; j < n && ok; ++j) {
+    for (int j = 0; j < n; ++j) {        // the whole list also after a time-out, see mbar_wait_warp
       const int entry = next;
       next = j + 1 < n ? list[j + 1] : 0;
       other += t == 0 ? ((entry >> 26) & 3) != kTileSkip : ((next >> 24) & 3) != kTileSkip;
       const int cls_t = (entry >> (24 + 2 * t)) & 3;
       if (cls_t == kTileSkip) continue;
-      if (!mbar_wait(&s_full[t], cnt & 1, abort_flag, args.status, 5)) {
-        ok = false;
-        break;
-      }
+      ok &= mbar_wait(&s_full[t], cnt & 1, abort_flag, args.status, 5);
       tc_fence_after();
       float sv[2][32];   // [columns 0-63, 64-127][4 i + 2 row + e]
       {
@@ -412,17 +412,9 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
         unpack_f32x2(add_f32x2(acc[r][0], acc[r][1]), s0, s1);
         l[r] = l[r] * alpha[r] + (s0 + s1);      // of this thread's columns; summed over the four threads at the end
       }
-      if (cnt > 0) {
-        if (!mbar_wait(&pv_done[t], (cnt - 1) & 1, abort_flag, args.status, 5)) {
-          ok = false;
-          break;
-        }
-      }
+      if (cnt > 0) ok &= mbar_wait(&pv_done[t], (cnt - 1) & 1, abort_flag, args.status, 5);
       // the other tile's warps have read the scores that P goes over
-      if (!count_wait(&drained[t ^ 1], 8 * other, abort_flag, args.status, 5)) {
-        ok = false;
-        break;
-      }
+      ok &= count_wait(&drained[t ^ 1], 8 * other, abort_flag, args.status, 5);
       tc_fence_after();
       tmem_st_16x128b_x16(tmem_P, pk);
       if (cnt > 0 && rescale) {
@@ -451,7 +443,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1)
     }
     // Output rows leave through this warp's rows of the query tile's buffer (no product reads it any more), so that 16
     // lanes store one row's 256 bytes.
-    if (ok && cnt > 0) ok = mbar_wait(&pv_done[t], (cnt - 1) & 1, abort_flag, args.status, 5);
+    if (cnt > 0) ok &= mbar_wait(&pv_done[t], (cnt - 1) & 1, abort_flag, args.status, 5);
+    ok = __all_sync(0xffffffffu, ok);
     if (ok) {
       tc_fence_after();
 #pragma unroll

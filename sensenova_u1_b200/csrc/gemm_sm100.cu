@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       if (tc.skip) continue;
       const int acc = tile_it & 1;
       const uint32_t acc_ph = (tile_it >> 1) & 1;
-      if (!mbar_wait(&acc_full[acc], acc_ph, abort_flag, args.status, 4)) {
+      if (!mbar_wait_warp(&acc_full[acc], acc_ph, abort_flag, args.status, 4)) {
         ok = false;
         break;
       }
@@ -606,7 +606,7 @@ __device__ __forceinline__ bool mbar_wait_cl(uint64_t* bar, uint32_t parity, vol
   uint64_t t0 = globaltimer_ns();
   uint32_t spins = 0;
   while (!mbar_try_wait_cl(bar, parity)) {
-    if ((++spins & 0x3ff) == 0) {
+    if ((spins++ & 0x3ff) == 0) {
       if (*abort_flag) return false;
       if (globaltimer_ns() - t0 > kLocalWaitNs) {
         *abort_flag = 1;
@@ -893,7 +893,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       for (int ps = 0; ps < pu.npass && ok; ++ps) {
         const int acc = tile_it & 1;
         const uint32_t acc_ph = (tile_it >> 1) & 1;
-        if (!mbar_wait_cl(&acc_full[acc], acc_ph, abort_flag, args.status, 4)) {
+        if (!__all_sync(0xffffffffu, mbar_wait_cl(&acc_full[acc], acc_ph, abort_flag, args.status, 4))) {
           ok = false;
           break;
         }

@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
     bool ok = true;
     for (int i = 0; i < c_hi - c_lo; ++i) {
       const int s = i % C::STAGES;
-      if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], (i / C::STAGES) & 1, abort_flag, args.status, 3))) {
+      if (!mbar_wait_warp(&full_bar[s], (i / C::STAGES) & 1, abort_flag, args.status, 3)) {
         ok = false;
         break;
       }
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
   if (warp >= 2) {
     const int quarter = warp & 3;
     const int wr = quarter * 32 + lane;
-    ok = mbar_wait(acc_full, 0, abort_flag, args.status, 4);
+    ok = mbar_wait_warp(acc_full, 0, abort_flag, args.status, 4);
     if (ok) {
       tc_fence_after();
       const uint32_t ta = tmem_base + ((uint32_t)(quarter * 32) << 16);
