@@ -8,6 +8,8 @@
 // 352-506, 573-660 (host-synchronising split sizes, argsort / index permute, grouped_gemm.ops.permute);
 // inference block src/sensenova_u1/models/neo_unify/modeling_qwen3_moe.py:51-119.
 // Here split sizes never leave the device.
+#include <float.h>
+
 #include "host_common.h"
 #include "sm100_common.cuh"
 
@@ -57,7 +59,9 @@ __device__ __forceinline__ RoutedSlot route_row(const float* __restrict__ logits
     v[i] *= inv;
     const int e = lane + 32 * i;
     if (probs_out && e < E) probs_out[e] = v[i];
-    sc[i] = e < E ? v[i] + (sel_bias ? sel_bias[e] : 0.f) : -INFINITY;
+    // -inf marks what has been taken: a score without a value (NaN logits) counts as the lowest finite one, so that a row
+    // takes K different experts whatever it holds
+    sc[i] = e < E ? fmaxf(v[i] + (sel_bias ? sel_bias[e] : 0.f), -FLT_MAX) : -INFINITY;
   }
   float wsum = 0.f;
   my_w = 0.f;
@@ -82,7 +86,6 @@ __device__ __forceinline__ RoutedSlot route_row(const float* __restrict__ logits
         be = oe;
       }
     }
-    be = min(be, E - 1);                              // no finite score left (NaN logits)
     const float pw = __shfl_sync(0xffffffffu, v[be >> 5], be & 31);     // the chosen expert's probability
     if ((be & 31) == lane) sc[be >> 5] = -INFINITY;  // remove from further rounds
     if (lane == k) {

@@ -71,3 +71,26 @@ def test_one_cta_path_equals_the_general_path(monkeypatch):
         outs.append(eng._moe_ffn(W, x, x, UND, torch.empty_like(x)).float())
     # two bf16 roundings of the experts' outputs may differ by an ulp each
     assert ((outs[0] - outs[1]).abs() <= outs[1].abs() * 2.0 ** -7 + 2e-2).all()
+
+
+@pytest.mark.parametrize("R,E,K,bad", [(32, 32, 8, 17), (32, 128, 8, 20), (32, 256, 16, 31), (5, 3, 2, 5), (200, 128, 8, 60)])
+@pytest.mark.parametrize("what", [float("nan"), float("inf"), float("-inf")])
+def test_rows_without_a_finite_score(R, E, K, bad, what):
+    """A row of NaN (or whose softmax is NaN) still takes K different experts: no expert gets more rows than there are, and
+    every slot lies inside the permuted buffer.  The other rows are not affected."""
+    from sensenova_u1_b200.ops import _lib, moe
+    g = torch.Generator(device="cuda").manual_seed(R + E)
+    good = torch.randn(R, E, device="cuda", generator=g)
+    logits = good.clone()
+    logits[:bad] = what
+    logits[0, 1:] = good[0, 1:]                                            # one row with a single bad score
+    for route in ([moe.route] if R > 32 else [moe.route, lambda x, k, n: moe.route_few(x, k, n, _Bufs())]):
+        r, ref = route(logits, K, True), route(good, K, True)
+        _lib.check_status()
+        idx, dest = r.top_idx.cpu(), r.dest.cpu()
+        assert ((0 <= idx) & (idx < E)).all() and all(len(set(row)) == K for row in idx.tolist())
+        assert (dest >= 0).all() and (dest < r.max_rows).all() and dest.unique().numel() == R * K
+        tiles = r.tile_group.cpu()
+        assert torch.equal(tiles[(dest // 128).view(-1).long()], idx.view(-1))     # every slot in a tile of its expert
+        assert torch.equal(r.top_idx[bad:], ref.top_idx[bad:]) and torch.equal(r.top_w[bad:], ref.top_w[bad:])
+        assert torch.isnan(r.top_w[1:bad]).all()                            # what the row held goes on into its output
