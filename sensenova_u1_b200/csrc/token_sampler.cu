@@ -243,26 +243,34 @@ __global__ void __launch_bounds__(THREADS) top_k_top_p_kernel(const Args a) {
       const int i = 2 * tid + j;
       e[j] = i < larger ? expf(from_key(s.key_all[i]) - mx) : 0.f;
     }
-    auto scan = [&](float x) {                          // inclusive, over the block
+    // sum over the block before the thread's own, and with it.  The former is never the latter less x: that leaves a
+    // rounding instead of 0 before the first, and the likeliest token would go at a top_p below it
+    auto scan = [&](float x, float& before) {
+      float incl = x;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const float t = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += t;
+        const float t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
       }
+      before = __shfl_up_sync(0xffffffffu, incl, 1);
+      if (lane == 0) before = 0.f;
       __syncthreads();
-      if (lane == 31) s.scan[warp] = x;
+      if (lane == 31) s.scan[warp] = incl;
       __syncthreads();
-      for (int w = 0; w < warp; ++w) x += s.scan[w];
-      return x;
+      float base = 0.f;
+      for (int w = 0; w < warp; ++w) base += s.scan[w];
+      before += base;
+      return incl + base;
     };
-    const float incl = scan(e[0] + e[1]);
+    float b0, unused;
+    const float incl = scan(e[0] + e[1], b0);
     if (tid == THREADS - 1) s.sum = incl;
     __syncthreads();
     const float above = s.sum, sum = above + ties * e_tie;
     __syncthreads();
-    const float b0 = incl - e[0] - e[1], b1 = incl - e[1];
+    const float b1 = b0 + e[0];
     const bool k0 = !(b0 / sum > a.top_p) || a.top_p >= 1.f, k1 = !(b1 / sum > a.top_p) || a.top_p >= 1.f;
-    const float kept = scan((k0 ? e[0] : 0.f) + (k1 ? e[1] : 0.f));
+    const float kept = scan((k0 ? e[0] : 0.f) + (k1 ? e[1] : 0.f), unused);
     if (tid == THREADS - 1) {
       int keep = ties;
       if (a.top_p < 1.f) {

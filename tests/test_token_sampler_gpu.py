@@ -55,3 +55,13 @@ def test_ties_signed_zeros_and_infinities(monkeypatch):
     assert torch.equal(got, (1 / noise[:, :251]).argmax(1)) or torch.equal(got, (1 / noise[:, :250]).argmax(1))
     bad = torch.full((2, 64), float("nan"), device="cuda")
     assert ((0 <= fused.sample_top_k_top_p(bad, noise[:2, :64].contiguous(), 1.0, 5, 0.9))).all()
+
+
+@pytest.mark.parametrize("k", [2, 50, 1024])
+@pytest.mark.parametrize("p", [1e-9, 1e-30, 0.0])      # below any rounding of a sum of probabilities
+def test_tiny_top_p_is_greedy(k, p, monkeypatch):
+    """Nothing comes before the most likely token, so it stays whatever ``top_p`` is."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    lg = torch.randn(64, 5000, device="cuda", generator=g)
+    got, ref = _both(lg, dict(do_sample=True, top_k=k, top_p=p or 1e-300), 1, monkeypatch)
+    assert torch.equal(got, lg.argmax(-1)) and torch.equal(ref, got)
