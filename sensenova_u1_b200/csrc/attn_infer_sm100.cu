@@ -76,7 +76,7 @@ __device__ __forceinline__ bool count_wait(const int* c, int target, volatile in
     int v;
     asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     if (v >= target) return true;
-    if ((spins & 0x3ff) == 1) {
+    if ((spins & 0x3ff) == 32) {
       if (*abort_flag) return false;
       const uint64_t now = globaltimer_ns();
       if (t0 == 0) t0 = now;

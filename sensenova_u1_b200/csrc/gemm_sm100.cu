@@ -603,12 +603,14 @@ __device__ __forceinline__ bool mbar_try_wait_cl(uint64_t* bar, uint32_t parity)
 __device__ __forceinline__ bool mbar_wait_cl(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
                                              int where) {
   if (mbar_try_wait_cl(bar, parity)) return true;
-  uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;
   uint32_t spins = 0;
   while (!mbar_try_wait_cl(bar, parity)) {
-    if ((spins++ & 0x3ff) == 0) {
+    if ((++spins & 0x3ff) == 32) {       // soon, when some role has given up already; short waits read no clock
       if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > kLocalWaitNs) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > kLocalWaitNs) {
         *abort_flag = 1;
         report_status(status, kWaitTimeout, where);
         return false;
