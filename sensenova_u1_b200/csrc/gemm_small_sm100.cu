@@ -344,6 +344,9 @@ static int launch_gemm_small_any(const void* x, const void* w, void* c, int M, i
     split = 1;
     while (split < 8 && (long long)tiles * mt * split * 2 <= fit && chunks / (split * 2) >= (tn >= 64 ? 12 : 3)) split *= 2;
   }
+  // every part needs a chunk (a CTA without one has no product that would set its accumulator), a cluster has 8 CTAs at most
+  split = split < chunks ? split : chunks;
+  split = split < 8 ? split : 8;
   CUtensorMap tmW, tmX;
   int rc;
   {
@@ -395,12 +398,24 @@ int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K
 
 }  // namespace snu1
 
-// The same product with the reduction split given (0: chosen by size); snu1_gemm_bf16 comes here by itself.
+// The same product with the reduction split given (0: chosen by size; more parts than the reduction has 64s, or than 8, are
+// not made); snu1_gemm_bf16 comes to launch_gemm_small by itself, with the checks of its own.
 SNU1_API int snu1_gemm_small(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
                              long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
                              void* stream) {
-  return snu1::launch_gemm_small(x, w, c, M, N, K, ldx, ldw, ldc, f32_out, residual, ldr, alpha, split, 0, 0,
-                                 reinterpret_cast<cudaStream_t>(stream));
+  using namespace snu1;
+  if (M <= 0 || N <= 0 || N % 8 || K <= 0 || K % 8 || ldx % 8 || ldw % 8 || ldc % (f32_out ? 4 : 8) ||
+      (M + 127) / 128 > 65535 || (reinterpret_cast<uintptr_t>(c) & 15) != 0) {
+    set_last_error("gemm_small: M=%d N=%d K=%d ldx=%lld ldw=%lld ldc=%lld (N, K, ldx, ldw multiples of 8, ldc of %d, y 16-byte "
+                   "aligned)", M, N, K, ldx, ldw, ldc, f32_out ? 4 : 8);
+    return kHostBadArg;
+  }
+  if (residual != nullptr && (f32_out || ldr % 8 || (reinterpret_cast<uintptr_t>(residual) & 15) != 0)) {
+    set_last_error("gemm_small: a residual needs a bf16 result, 16-byte alignment and a stride of a multiple of 8");
+    return kHostBadArg;
+  }
+  return launch_gemm_small(x, w, c, M, N, K, ldx, ldw, ldc, f32_out, residual, ldr, alpha, split, 0, 0,
+                           reinterpret_cast<cudaStream_t>(stream));
 }
 
 // Expert products of a few rows: row tile t (rows 128 t .. 128 t + rows - 1 of x and y, rows <= 128) times the weights of

@@ -43,6 +43,41 @@ def test_few_rows_take_the_weight_streaming_kernel():
     assert ((a - b).abs() <= b.abs() * 2.0 ** -7 + 1e-2).all()      # two roundings of nearly the same fp32 sum
 
 
+def _streamed(x, w, out, split=0, f32=1, residual=None, **wrong):
+    """The exported entry point; ``wrong``: arguments in place of the operands' own."""
+    from sensenova_u1_b200.ops import _lib
+    from sensenova_u1_b200.ops._lib import c_float, c_int, c_ll, c_void_p
+    P = lambda t: c_void_p(None if t is None else t.data_ptr())
+    v = dict(N=w.shape[0], K=x.shape[1], ldx=x.stride(0), ldw=w.stride(0), ldc=out.stride(0), ldr=0 if residual is None else residual.stride(0))
+    v.update(wrong)
+    _lib.call("gemm_small", P(x), P(w), P(out), c_int(x.shape[0]), c_int(v["N"]), c_int(v["K"]), c_ll(v["ldx"]), c_ll(v["ldw"]),
+              c_ll(v["ldc"]), c_int(f32), P(residual), c_ll(v["ldr"]), c_float(1.0), c_int(split), c_void_p(_lib.stream()))
+    return out
+
+
+@pytest.mark.parametrize("K", [8, 64, 72, 200])               # 1, 1, 2 and 4 pieces of 64 for up to 8 CTAs
+@pytest.mark.parametrize("split", [2, 5, 8, 16, 100])
+def test_split_of_a_short_reduction(K, split):
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x, w = (torch.randn(n, K, device="cuda", generator=g).to(torch.bfloat16) for n in (20, 256))
+    out = _streamed(x, w, torch.full((20, 256), float("nan"), device="cuda"), split)
+    ref = x.double() @ w.double().t()
+    # fp32 sums of at most 13 tensor-core steps, each off by at most one unit in the last place of a partial sum
+    assert (out - ref).norm() / ref.norm() < 13 * 2.0 ** -23
+
+
+def test_entry_point_refuses_what_the_kernel_cannot_address():
+    x, w = (torch.zeros(n, 64, device="cuda", dtype=torch.bfloat16) for n in (20, 256))
+    bf, f = torch.zeros(20 * 256 + 16, device="cuda", dtype=torch.bfloat16), torch.zeros(20 * 256 + 8, device="cuda")
+    for kw in (dict(N=250), dict(K=60), dict(ldx=60), dict(ldw=60), dict(ldc=258), dict(K=0), dict(N=0),
+               dict(out=f[1:1 + 20 * 256]), dict(out=bf[4:4 + 20 * 256], f32=0), dict(residual=bf[:20 * 256]),
+               dict(f32=0, out=bf[:20 * 256], residual=bf[4:4 + 20 * 256]),
+               dict(f32=0, out=bf[:20 * 256], residual=bf[:20 * 256], ldr=252)):
+        kw = {k: v.view(20, 256) if torch.is_tensor(v) else v for k, v in kw.items()}
+        with pytest.raises(RuntimeError):
+            _streamed(x, w, kw.pop("out", f[:20 * 256].view(20, 256)), **kw)
+
+
 @pytest.mark.parametrize("M", [1, 17, 64, 128, 129, 300, 1000])        # weight-streaming kernel up to 128 rows, pair kernel beyond
 @pytest.mark.parametrize("F,K", [(24, 72), (64, 512), (200, 1096), (768, 2048), (3072, 1024)])   # ragged and whole column tiles
 @pytest.mark.parametrize("static", [False, True])
