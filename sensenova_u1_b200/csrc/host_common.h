@@ -32,6 +32,7 @@ int num_sms();
   do {                                                                                 \
     cudaError_t _e = (expr);                                                           \
     if (_e != cudaSuccess) {                                                           \
+      cudaGetLastError(); /* a refused launch is not the next call's error */          \
       ::snu1::set_last_error("%s failed: %s (%s:%d)", #expr, cudaGetErrorString(_e),   \
                              __FILE__, __LINE__);                                      \
       return ::snu1::kHostCuda;                                                        \

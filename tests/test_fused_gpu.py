@@ -338,3 +338,18 @@ def test_qknorm_rope_bwd_wide_equals_narrow(rows, n_q, n_kv):
     # sums of 64 in another order: one rounding to bf16 apart (2^-7 of the value), cancellation near zero
     assert ((a - b).abs() <= b.abs() * 2.0 ** -7 + 1e-4).all()
     assert ((da - db).abs() <= db.abs() * 1e-4 + 1e-3).all() and (da[0] == 0).all()
+
+
+def test_refused_launch_does_not_fail_the_next_call():
+    from sensenova_u1_b200.ops import _lib, attention as A, fused
+    i, f = torch.zeros(3, dtype=torch.int32, device=DEV), torch.zeros(64, device=DEV)
+    x = torch.zeros(8192, device=DEV, dtype=torch.bfloat16)
+    rows = torch.zeros(1, dtype=torch.long, device=DEV)
+    n_q = 16 * 65536                                                              # more CTAs than a grid's y can have: not launched
+    with pytest.raises(_lib.NativeLibraryError):
+        _lib.call("qknorm_rope_cache", fused.P(x), _lib.c_ll(8), fused.P(x), _lib.c_ll(8), fused.P(x), fused.P(x), _lib.c_ll(1),
+                  fused.P(rows), fused.P(x), fused.P(i), fused.P(f), fused.P(f), _lib.c_int(1), _lib.c_int(n_q), _lib.c_int(1),
+                  _lib.c_float(1e-6), fused.ST())
+    meta = A.make_meta(torch.zeros(5, device=DEV), torch.arange(5, device=DEV))
+    A.build_plan(meta)                                                            # looks at the runtime's last error
+    torch.cuda.synchronize()
