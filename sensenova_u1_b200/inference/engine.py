@@ -290,7 +290,8 @@ class InferenceEngine:
         if (lg.is_cuda and lg.dim() == 2 and 0 < lg.shape[0] < 65536 and 0 < k < lg.shape[-1] and k <= fused.SAMPLER_MAX_K
                 and lg.shape[-1] <= fused.SAMPLER_MAX_VOCAB):
             # the same draw in one launch: top-k first bounds what has to be sorted
-            return fused.sample_top_k_top_p(lg, torch.empty_like(lg).exponential_(1.0), t, k, p_)
+            noise = torch.empty(lg.shape, dtype=lg.dtype, device=lg.device).exponential_(1.0)    # in row order for any strides
+            return fused.sample_top_k_top_p(lg, noise, t, k, p_)
         if t != 1.0:
             lg = lg / t
         if 0 < k < lg.shape[-1]:

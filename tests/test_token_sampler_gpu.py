@@ -65,3 +65,12 @@ def test_tiny_top_p_is_greedy(k, p, monkeypatch):
     lg = torch.randn(64, 5000, device="cuda", generator=g)
     got, ref = _both(lg, dict(do_sample=True, top_k=k, top_p=p or 1e-300), 1, monkeypatch)
     assert torch.equal(got, lg.argmax(-1)) and torch.equal(ref, got)
+
+
+def test_logits_of_any_strides(monkeypatch):
+    """Columns first, every other column, one row repeated: the same draws as the separate operations."""
+    g = torch.Generator(device="cuda").manual_seed(2)
+    base = torch.randn(4000, 6, device="cuda", generator=g)
+    for lg in (base.t(), base.t().contiguous()[:, ::2], base[:, 0].expand(5, 4000)):
+        a, b = _both(lg, dict(do_sample=True, temperature=0.9, top_k=40, top_p=0.95), 4, monkeypatch)
+        assert torch.equal(a, b)
