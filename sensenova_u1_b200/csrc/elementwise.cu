@@ -637,9 +637,9 @@ __global__ void __launch_bounds__(QC_THREADS, 2)
         v[i] *= rstd;
         dxh[i] = dnorm * (is_k ? gk[i] : gq[i]);
         dot2[i >> 2] += dxh[i] * v[i];
-        const float a = dnorm * v[i];          // zero for the heads past the last (loaded as zeros)
-        if (is_k) acc_k[i] += a;
-        else acc_q[i] += a;
+        const float a = dnorm * v[i];
+        if (!is_k) acc_q[i] += a;
+        else if (h < nheads) acc_k[i] += a;    // past the last head v is 0 * rstd, not a number where eps is 0
       }
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) {

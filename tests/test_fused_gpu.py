@@ -353,3 +353,26 @@ def test_refused_launch_does_not_fail_the_next_call():
     meta = A.make_meta(torch.zeros(5, device=DEV), torch.arange(5, device=DEV))
     A.build_plan(meta)                                                            # looks at the runtime's last error
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("pad", [8, 4])                                          # both kernels
+def test_qknorm_rope_bwd_odd_heads_without_eps(pad):
+    """Lanes of the last pair of heads that own no head add nothing to the gain gradients, also where 1 / sqrt(0 + eps) of
+    their empty head is infinite."""
+    from sensenova_u1_b200.ops import fused
+    rows, n_q, n_kv = 20, 4, 1
+    W = (n_q + 2 * n_kv) * 128
+    qkv, d = (torch.zeros(rows, W + pad, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    qkv[:, :W], d[:, :W] = _bf(rows, W, seed=1), _bf(rows, W, seed=2)
+    gains = torch.ones(1, 4, 64, device=DEV, dtype=torch.bfloat16)
+    dg = torch.zeros(1, 4, 64, device=DEV)
+    zero = torch.zeros(32, device=DEV)                                            # no rotation
+    fused.qknorm_rope_bwd(qkv[:, :W], d[:, :W], gains, dg, None, torch.zeros(3, rows, device=DEV, dtype=torch.int32), zero,
+                          zero[:16], n_q, n_kv, 0.0)
+    x = qkv[:, :W].double().view(rows, -1, 2, 64)[:, :n_q + n_kv]
+    xhat = x * x.pow(2).mean(-1, keepdim=True).rsqrt()
+    dn = (_bf(rows, W, seed=2).double().view(rows, -1, 2, 64)[:, :n_q + n_kv] * xhat).sum(0)      # [heads, half, 64]
+    want = torch.stack([dn[:n_q, 0].sum(0), dn[:n_q, 1].sum(0), dn[n_q:, 0].sum(0), dn[n_q:, 1].sum(0)])
+    # fp32 sums of at most 80 products of about 4, each rounded a handful of times
+    assert (dg[0] - want).abs().max() < 80 * 16 * 2.0 ** -22
+    assert torch.isfinite(d).all()
