@@ -72,6 +72,7 @@ class InferenceEngine:
         self.vc: List[torch.Tensor] = []
         self.stats = torch.zeros(4 + 4 * 592, dtype=torch.float32, device=self.dev)   # sums + per-block partials
         self._graph = self._capture_stream = None     # last captured decode step, for its memory (see _capture)
+        self._graph_bytes = 0
         self.sp = None      # sequence-parallel sampling state (enable_sequence_parallel)
 
     def enable_sequence_parallel(self, group) -> None:
@@ -403,32 +404,59 @@ class InferenceEngine:
         self.last_decode_steps, self.last_decode_graph = done, graph is not None
         return out
 
+    GRAPH_POOL_LIMIT = 256 << 20     # bytes that a decode graph may keep from one request to the next
+
     def _capture(self, fn):
         """CUDA graph of ``fn()``.  Its temporaries come from the memory pool of the graph before it, which is kept (and
-        never replayed again) for that purpose: ``torch.cuda.graph`` collects garbage and empties the allocator's cache
-        first, and every request then paid for returning that memory to the driver and asking for it again (5 - 400 ms
-        on a shared host)."""
-        cur, old = torch.cuda.current_stream(), self._graph
-        if self._capture_stream is None:             # always the same one: the pool's free blocks belong to a stream
-            self._capture_stream = torch.cuda.Stream()
-        self._capture_stream.wait_stream(cur)
-        graph = torch.cuda.CUDAGraph()
-        try:
-            with torch.cuda.stream(self._capture_stream):
-                graph.capture_begin(pool=None if old is None else old.pool())
-                try:
-                    fn()
-                finally:
-                    graph.capture_end()
-        except torch.cuda.OutOfMemoryError:          # the cache holds what the pool needs: let torch empty it first
-            self._graph = old = None
-            torch.cuda.synchronize()
+        never replayed again) for that purpose: ``torch.cuda.graph`` empties the allocator's cache first, and every request
+        then paid for returning that memory to the driver and asking for it again (5 - 400 ms on a shared host).  A pool that
+        has grown past ``GRAPH_POOL_LIMIT`` is not kept: it goes back to the allocator with its request's graph."""
+        with torch.cuda.device(self.dev):
+            cur, old = torch.cuda.current_stream(), self._graph
+            if self._capture_stream is None:         # always the same one: the pool's free blocks belong to a stream
+                self._capture_stream = torch.cuda.Stream(self.dev)
+            self._capture_stream.wait_stream(cur)
+            before = self._reserved()
             graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph):
-                fn()
-        cur.wait_stream(self._capture_stream)
-        self._graph = graph
+            try:
+                self._record(graph, old, fn)
+            except torch.cuda.OutOfMemoryError:      # the cache holds what the pool needs: let torch empty it first
+                graph = None
+            if graph is None:                        # here the error no longer holds on to the broken capture's memory
+                self.release_decode_memory()
+                old = None
+                torch.cuda.synchronize()
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, stream=self._capture_stream):
+                    before = self._reserved()
+                    fn()
+            cur.wait_stream(self._capture_stream)
+            self._graph_bytes += max(0, self._reserved() - before)
+            self._graph = graph
+            if self._graph_bytes > self.GRAPH_POOL_LIMIT:
+                self.release_decode_memory()
         return graph
+
+    def _reserved(self) -> int:
+        # memory_reserved() without its flat copy of all counters
+        return torch.cuda.memory_stats_as_nested_dict(self.dev)["reserved_bytes"]["all"]["current"]
+
+    def _record(self, graph, old, fn):
+        with torch.cuda.stream(self._capture_stream):
+            graph.capture_begin(pool=None if old is None else old.pool())
+            try:
+                fn()
+            except BaseException:
+                try:
+                    graph.capture_end()
+                except RuntimeError:                 # a broken capture: what broke it is the error to report
+                    pass
+                raise
+            graph.capture_end()
+
+    def release_decode_memory(self) -> None:
+        """Gives the memory that the last decode graph keeps for the next one back to the allocator."""
+        self._graph, self._graph_bytes = None, 0
 
     # --------------------------------------------------------------- generation
     @torch.no_grad()
