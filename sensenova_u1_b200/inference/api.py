@@ -368,7 +368,7 @@ class NEOChatModel:
         t, h, w = [], [], []
         cur, i, g = 0, 0, 0
         flags = (ids == ctx_id).tolist()
-        n = len(flags)
+        n = ids.numel()
         while i < n:
             if not flags[i]:
                 t.append(cur); h.append(0); w.append(0)

@@ -362,6 +362,19 @@ def test_prompt_embedding_places_pictures_of_history_question_and_partial_answer
         m._embed_prompt(tok, "no placeholder", [img(1, 1)])
 
 
+def test_position_indexes_of_text_and_pictures():
+    import pytest
+    import torch
+    from sensenova_u1_b200.inference.api import NEOChatModel
+    thw = NEOChatModel.get_thw_indexes
+    got = thw(torch.tensor([7, 3, 3, 3, 3, 8, 3, 9]), [(2, 2), (1, 1)], 3)
+    assert got.tolist() == [[0, 1, 1, 1, 1, 2, 3, 4], [0, 0, 0, 1, 1, 0, 0, 0], [0, 0, 1, 0, 1, 0, 0, 0]] and got.dtype == torch.int32
+    assert thw(torch.tensor([], dtype=torch.long), [], 3).shape == (3, 0)
+    for ids, grids in (([7, 3, 3], [(2, 2)]), ([3], []), ([[7, 8, 9]], [(1, 1)]), ([[7, 8, 9]], [])):   # too few tokens, no grid,
+        with pytest.raises((ValueError, IndexError)):                                                  # a batch of prompts
+            thw(torch.tensor(ids), grids, 3)
+
+
 def test_chat_adds_picture_tags_only_when_nothing_marks_them():
     import types
     import torch
