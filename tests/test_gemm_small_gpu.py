@@ -33,16 +33,6 @@ def test_small_rows(M, N, K, split):
         assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + 1e-2).all()
 
 
-def test_few_rows_take_the_weight_streaming_kernel():
-    """``gemm_nt`` at 128 rows (this kernel) and at 129 (the pair kernel) on the same operands."""
-    from sensenova_u1_b200.ops import gemm
-    g = torch.Generator(device="cuda").manual_seed(0)
-    x = torch.randn(129, 4096, device="cuda", generator=g).to(torch.bfloat16)
-    w = torch.randn(4096, 4096, device="cuda", generator=g).to(torch.bfloat16)
-    a, b = gemm.gemm_nt(x[:128], w).double(), gemm.gemm_nt(x, w)[:128].double()
-    assert ((a - b).abs() <= b.abs() * 2.0 ** -7 + 1e-2).all()      # two roundings of nearly the same fp32 sum
-
-
 def _streamed(x, w, out, split=0, f32=1, residual=None, **wrong):
     """The exported entry point; ``wrong``: arguments in place of the operands' own."""
     from sensenova_u1_b200.ops import _lib
@@ -53,6 +43,20 @@ def _streamed(x, w, out, split=0, f32=1, residual=None, **wrong):
     _lib.call("gemm_small", P(x), P(w), P(out), c_int(x.shape[0]), c_int(v["N"]), c_int(v["K"]), c_ll(v["ldx"]), c_ll(v["ldw"]),
               c_ll(v["ldc"]), c_int(f32), P(residual), c_ll(v["ldr"]), c_float(1.0), c_int(split), c_void_p(_lib.stream()))
     return out
+
+
+@pytest.mark.parametrize("M", [1, 16, 32, 33, 128])
+def test_few_rows_take_the_weight_streaming_kernel(M):
+    """``gemm_nt`` up to 128 rows has this kernel's bits (a reduction in several parts), at 129 rows the pair kernel's."""
+    from sensenova_u1_b200.ops import gemm
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x = torch.randn(129, 4096, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(4096, 4096, device="cuda", generator=g).to(torch.bfloat16)
+    few, many = (gemm.gemm_nt(t, w, out_mode=gemm.OUT_F32_STORE) for t in (x[:M], x))
+    assert torch.equal(few, _streamed(x[:M], w, torch.empty_like(few)))
+    assert not torch.equal(few, many[:M])                      # so that equal bits mean the same kernel
+    # the same products in another order: K / 16 steps of fp32 sums on both sides
+    assert (few - many[:M]).norm() / many[:M].norm() < 2 * 4096 / 16 * 2.0 ** -23
 
 
 @pytest.mark.parametrize("K", [8, 64, 72, 200])               # 1, 1, 2 and 4 pieces of 64 for up to 8 CTAs
@@ -108,3 +112,35 @@ def test_linear_swiglu_grouped():
     ref = fused.swiglu_fwd(gu, torch.empty(7 * 128, F, device="cuda", dtype=torch.bfloat16))
     keep = (tg >= 0).repeat_interleave(128)
     assert torch.equal(out[keep], ref[keep]) and (out[~keep] == 7).all()
+
+
+def test_static_weights_written_just_before_a_request():
+    """A weight declared static may be read before the kernel in front of the product has finished: new values that were
+    written right before a prompt and a decode step are the ones they use."""
+    from sensenova_u1_b200.config import tiny_mot
+    from sensenova_u1_b200.inference.engine import InferenceEngine
+    from sensenova_u1_b200.models.params import ParamStore
+    cfg = tiny_mot(head_dim=128, patch_size=16)
+    store = ParamStore(cfg, device="cuda:0", with_grads=False)
+    store.init_weights(3)
+    eng = InferenceEngine(cfg, store)
+    names = [n for n, t in store.p.items() if n.startswith("layers.0.") and t.dim() == 3]
+    first = {n: store.p[n].clone() for n in names}
+    second = {n: torch.randn_like(store.p[n]) * 0.05 for n in names}
+    want = []
+    for wait in (True, False):
+        for rep in range(1 if wait else 10):
+            for values in (first, second):
+                for n in names:
+                    store.p[n].copy_(values[n])
+                if wait:
+                    torch.cuda.synchronize()
+                lay, h = eng.prefill([torch.arange(5, 25)], reserve_image_tokens=8)
+                got = (h.clone(), eng.decode(lay, h, 1), eng.kc[0].clone(), eng.kc[1].clone())
+                if wait:
+                    want.append(got)
+                else:
+                    ref = want[0 if values is first else 1]
+                    assert torch.equal(got[0], ref[0]) and got[1] == ref[1]
+                    assert torch.equal(got[2], ref[2]) and torch.equal(got[3], ref[3])
+    assert not torch.equal(want[0][0], want[1][0])
