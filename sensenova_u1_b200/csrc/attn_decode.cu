@@ -49,22 +49,6 @@ struct Args {
   float scale_log2;
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
-  uint32_t ra;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(p)), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
-  return v;
-}
 __device__ __forceinline__ uint64_t bf16x2_to_f32x2(uint32_t u) {
   return pack_f32x2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
 }
@@ -114,7 +98,7 @@ __global__ void __launch_bounds__(THREADS, 2) attn_decode_kernel(const Args a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane & 7, grp = warp * 4 + (lane >> 3);
   const int row = blockIdx.z;
-  const int rank = a.split > 1 ? (int)cluster_rank() : 0;
+  const int rank = a.split > 1 ? (int)cluster_ctarank() : 0;
   const int rep = a.Hq / a.Hkv, per_kv = rep / HG;
   const int kvh = blockIdx.y / per_kv;
   const int h0 = kvh * rep + (blockIdx.y % per_kv) * HG;
@@ -290,7 +274,7 @@ __global__ void __launch_bounds__(THREADS, 2) attn_decode_kernel(const Args a) {
       c_l[h] = lc;
     }
   }
-  if (a.split > 1) cluster_sync();
+  if (a.split > 1) cluster_sync_all();
   else __syncthreads();
   // every CTA of the cluster finishes its share of the HG x 128 outputs, two at a time
   constexpr int PAIRS = HG * 64;
@@ -303,20 +287,20 @@ __global__ void __launch_bounds__(THREADS, 2) attn_decode_kernel(const Args a) {
       lt = c_l[h];
     } else {
       float mt = -INFINITY;
-      for (int r = 0; r < a.split; ++r) mt = fmaxf(mt, ld_cluster(&c_m[h], r));
+      for (int r = 0; r < a.split; ++r) mt = fmaxf(mt, ld_cluster(c_m[h], r));
       x = y = lt = 0.f;
       for (int r = 0; r < a.split; ++r) {
-        const float mr = ld_cluster(&c_m[h], r);
+        const float mr = ld_cluster(c_m[h], r);
         const float f = mr == -INFINITY ? 0.f : fast_exp2(mr - mt);
-        x += f * ld_cluster(&c_acc[h][c], r);
-        y += f * ld_cluster(&c_acc[h][c + 1], r);
-        lt += f * ld_cluster(&c_l[h], r);
+        x += f * ld_cluster(c_acc[h][c], r);
+        y += f * ld_cluster(c_acc[h][c + 1], r);
+        lt += f * ld_cluster(c_l[h], r);
       }
     }
     const float inv = lt > 0.f ? 1.f / lt : 0.f;       // a row without keys gives zeros
     *reinterpret_cast<uint32_t*>(a.o + row * a.ldo + (long long)(h0 + h) * 128 + c) = pack_bf16x2(x * inv, y * inv);
   }
-  if (a.split > 1) cluster_sync();   // nobody leaves while its partial result is read
+  if (a.split > 1) cluster_sync_all();   // nobody leaves while its partial result is read
 }
 
 template <int HG>

@@ -61,26 +61,6 @@ struct Args {
   int* status;
 };
 
-__device__ __forceinline__ uint32_t cta_in_cluster() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
-  uint32_t ra;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(ra)
-               : "memory");
-  return v;
-}
-
 // SWIGLU: w holds args.N gate rows and then as many up rows; a tile is 64 of each and gives 64 columns of
 // silu(gate) * up (both rounded to bf16 first, as when the projection was stored).
 template <int TN, bool SWIGLU, bool DEEP>
@@ -100,7 +80,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = (int)cta_in_cluster();
+  const int rank = (int)cluster_ctarank();
   constexpr int CN = SWIGLU ? BW / 2 : BW;      // columns of y per tile
   const int n0 = (blockIdx.x / args.split) * CN;
   int m0 = blockIdx.y * TN, w0 = 0;
@@ -218,7 +198,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
       tc_fence_before();
     }
   }
-  cluster_sync();
+  cluster_sync_all();
   if (warp >= 2) {
     pdl_wait();
     // this CTA finishes rows [r_lo, r_hi) of the tile: 8 outputs per thread and step
@@ -282,7 +262,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
     }
   }
   tc_fence_before();
-  cluster_sync();
+  cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, C::TMEM);

@@ -55,25 +55,6 @@ struct Shared {
   int tie_keep;
 };
 
-__device__ __forceinline__ uint32_t rank_in_cluster() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-template <typename T>
-__device__ __forceinline__ T remote(const T& x, uint32_t rank) {
-  static_assert(sizeof(T) == 4, "32-bit values");
-  uint32_t ra, v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(&x)), "r"(rank));
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(ra) : "memory");
-  T out;
-  memcpy(&out, &v, 4);
-  return out;
-}
 // order-preserving integer of a float; NaN above everything (as sorting does), -0 equal to 0
 __device__ __forceinline__ unsigned to_key(float x) {
   if (x != x) return 0xffffffffu;
@@ -105,7 +86,7 @@ __device__ __forceinline__ void block_best(Shared& s, float& v, int& i) {
 __global__ void __launch_bounds__(THREADS) top_k_top_p_kernel(const Args a) {
   extern __shared__ unsigned keys[];
   __shared__ Shared s;
-  const uint32_t rank = rank_in_cluster();
+  const uint32_t rank = cluster_ctarank();
   const int row = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int lo = (int)((long long)a.V * rank / CTAS), n = (int)((long long)a.V * (rank + 1) / CTAS) - lo;
   for (int i = tid; i < 4 * 256; i += THREADS) s.hist[0][i] = 0;
@@ -129,10 +110,10 @@ __global__ void __launch_bounds__(THREADS) top_k_top_p_kernel(const Args a) {
       const unsigned same = __match_any_sync(0xffffffffu, d);      // most logits share a few digits
       if (in && (same & ((1u << lane) - 1)) == 0) atomicAdd(&s.hist[p][d], __popc(same));
     }
-    cluster_sync();
+    cluster_sync_all();
     if (tid < 256) {
       unsigned t = 0;
-      for (int r = 0; r < CTAS; ++r) t += remote(s.hist[p][tid], r);
+      for (int r = 0; r < CTAS; ++r) t += ld_cluster(s.hist[p][tid], r);
       s.total[tid] = t;
     }
     __syncthreads();
@@ -197,15 +178,15 @@ __global__ void __launch_bounds__(THREADS) top_k_top_p_kernel(const Args a) {
     }
     if (tid == 0) s.ties = all;
   }
-  cluster_sync();
+  cluster_sync_all();
   if (rank == 0) {
     // gather, sort by (value, -index), softmax and cut
     int at = 0;
     for (int r = 0; r < CTAS; ++r) {
-      const int c = remote(s.count, r);
+      const int c = ld_cluster(s.count, r);
       for (int i = tid; i < c; i += THREADS) {
-        s.key_all[at + i] = remote(s.key[i], r);
-        s.idx_all[at + i] = remote(s.idx[i], r);
+        s.key_all[at + i] = ld_cluster(s.key[i], r);
+        s.idx_all[at + i] = ld_cluster(s.idx[i], r);
       }
       at += c;
     }
@@ -296,13 +277,13 @@ __global__ void __launch_bounds__(THREADS) top_k_top_p_kernel(const Args a) {
       s.draw_idx = bi;
     }
   }
-  cluster_sync();
+  cluster_sync_all();
   // ties of the k-th value that stay, ranked by index over the cluster
   {
-    const int keep = remote(s.tie_keep, 0);
-    const float pt = remote(s.tie_prob, 0);
+    const int keep = ld_cluster(s.tie_keep, 0);
+    const float pt = ld_cluster(s.tie_prob, 0);
     int before = tie_rank;
-    for (uint32_t r = 0; r < rank; ++r) before += remote(s.ties, r);
+    for (uint32_t r = 0; r < rank; ++r) before += ld_cluster(s.ties, r);
     float bv = 0.f;
     int bi = -1;
     if (my_ties > 0 && before < keep)
@@ -321,14 +302,14 @@ __global__ void __launch_bounds__(THREADS) top_k_top_p_kernel(const Args a) {
       s.cta_idx = bi;
     }
   }
-  cluster_sync();
+  cluster_sync_all();
   if (rank == 0 && tid == 0) {
     float bv = s.draw_val;
     int bi = s.draw_idx;
-    for (int r = 0; r < CTAS; ++r) take(bv, bi, remote(s.cta_val, r), remote(s.cta_idx, r));
+    for (int r = 0; r < CTAS; ++r) take(bv, bi, ld_cluster(s.cta_val, r), ld_cluster(s.cta_idx, r));
     a.out[row] = bi < 0 ? 0 : bi;
   }
-  cluster_sync();      // nobody leaves while its shared memory is read
+  cluster_sync_all();      // nobody leaves while its shared memory is read
 }
 
 }  // namespace tok
