@@ -8,9 +8,10 @@
 //
 // The kernel of attn_fwd_sm100.cu stays for callers that want the row log-sum-exp, i.e. a backward pass: the rows of a
 // warp decide together when the running maximum moves, and with 16 rows to a warp instead of 32 P is rounded at other
-// scales.  Outputs stay as close to fp64, but the bits differ, and a training run would no longer repeat what it did
-// before.  Made to decide over 32 rows and to add row sums in the same order (bit-equal), this kernel is as slow as that
-// one (full 8192: 1037 us).
+// scales.  Outputs are as close to fp32 softmax, but their bits differ, while every bf16 value of a training step is the
+// same as before this kernel came (only sums by fp32 atomics vary: loss, gains, biases).  That holds for one step: those
+// sums make the second differ from run to run (first-layer gradients by up to 1e-2), with either kernel.  Made to decide
+// over 32 rows and to add row sums in the same order (bit-equal), this kernel is as slow as that one (full 8192: 1037 us).
 #include "attn_common.cuh"
 #include "host_common.h"
 

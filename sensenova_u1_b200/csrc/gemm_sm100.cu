@@ -1123,8 +1123,15 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
     return kHostBadArg;
   }
   const int G = group_mode == 0 ? 1 : num_groups;
-  // Up to 128 rows of A, plain y = x W^T: the weight-streaming kernel.  Its times against the pair kernel stand in
-  // gemm_small_sm100.cu; at 256 rows and 24576 x 4096 weights it loses (76.7 against 58.0 us).
+  // Up to 128 rows of A, plain y = x W^T: the weight-streaming kernel.  us, weights cold in L2, streaming / pair:
+  //   rows                  64         128         129         256         512
+  //   24576 x 4096     41.8/59.1   45.8/59.1   67.7/58.8   77.6/62.4    128/82.8
+  //   151936 x 4096     216/252     260/254     469/270     497/275    1025/575
+  //   6144 x 4096      16.6/31.1   19.1/31.1   23.8/30.9   24.7/30.7   34.3/32.9
+  //   4096 x 4096      13.5/29.6   15.4/29.1   17.7/29.5   17.8/30.1   24.6/30.3
+  //   4096 x 12288     26.7/74.7   28.7/68.3   35.7/68.5   35.7/67.8   57.6/67.1
+  // The line is right for weights whose tiles fill the chip; for the others it lies too low (a second row tile reads the
+  // weights again, but from L2).
   if (M <= 128 && group_mode == 0 && !a_mn && !b_mn && (out_mode == 0 || out_mode == 2) && comm == nullptr &&
       (g_pair_mode != 0 || swiglu) && K > 0)
     return launch_gemm_small(A, B, C, M, N, K, lda, ldb, ldc, out_mode == 2, residual, ldr, alpha, 0, w_static, swiglu,

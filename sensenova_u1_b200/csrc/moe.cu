@@ -482,9 +482,8 @@ static int grid_1d(long long total, int block) {
 
 using namespace snu1;
 
-// counts [E] must be zero on entry.  max_tiles = number of 128-row tiles of the permuted buffer.
-// The same for at most 32 rows without the training outputs (no probabilities, no counts): top_idx, top_w [R,K],
-// tile_group [max_tiles] (expert of every 128-row tile, -1 beyond the last), dest [R,K].
+// Routing of at most 32 rows (a warp per row of one CTA) without the training outputs (no probabilities, no counts):
+// top_idx, top_w [R,K], tile_group [max_tiles] (expert of every 128-row tile, -1 beyond the last), dest [R,K].
 SNU1_API int snu1_moe_route_few(const float* logits, int R, int E, int K, int norm_topk, int* top_idx, float* top_w,
                                 int max_tiles, int* tile_group, int* dest, void* stream) {
   if (R < 1 || R > 32 || E > kMaxExperts || K > kMaxTopK || K > E || K < 1 || max_tiles < (R * K < E ? R * K : E)) {
@@ -496,6 +495,7 @@ SNU1_API int snu1_moe_route_few(const float* logits, int R, int E, int K, int no
   return kHostOk;
 }
 
+// counts [E] must be zero on entry.  max_tiles = number of 128-row tiles of the permuted buffer.
 static int moe_route_impl(const float* logits, int R, int E, int K, int norm_topk, float* probs,
                           int* top_idx, float* top_w, int* counts, const int* row_valid, int max_tiles,
                           int* seg_start, int* seg_end, int* tile_group, int* total_rows, int* dest,
