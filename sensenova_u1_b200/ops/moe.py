@@ -76,7 +76,9 @@ def route(logits: torch.Tensor, K: int, norm_topk: bool = True, row_valid=None, 
                    lse, row_class, cc)
 
 
-FEW_ROWS = 32     # rows that one CTA routes, see route_few
+# Rows that one CTA routes, a warp each (route_few).  Whole expert block (128 experts, 8 per row, 768 x 2048), us, few / general
+# path: 1 row 37 / 71, 8 rows 111 / 156, 24 rows 199 / 235, 32 rows 221 / 267; beyond, general only: 33 rows 263, 64 rows 287.
+FEW_ROWS = 32
 
 
 def route_few(logits: torch.Tensor, K: int, norm_topk: bool, ws) -> Routing:
