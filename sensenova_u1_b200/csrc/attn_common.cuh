@@ -141,4 +141,8 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   return d;
 }
 
+__device__ __forceinline__ uint64_t bf16x2_to_f32x2(uint32_t u) {
+  return pack_f32x2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+}
+
 }  // namespace snu1

@@ -49,10 +49,6 @@ struct Args {
   float scale_log2;
 };
 
-__device__ __forceinline__ uint64_t bf16x2_to_f32x2(uint32_t u) {
-  return pack_f32x2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
-}
-
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }

@@ -199,6 +199,10 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
       "r"(y), "r"(z), "r"(w)
       : "memory");
 }
+// Asks for [p, p + bytes) to be brought into L2 (a hint: nothing waits for it).  Both multiples of 16.
+__device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
 // generic-proxy writes to smem that the async proxy (UMMA / TMA) will read
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

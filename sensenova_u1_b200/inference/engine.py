@@ -23,7 +23,7 @@ from ..data.batch import apply_time_schedule
 from ..models import oracle
 from ..models.engine import Workspace
 from ..models.params import GEN, UND, ParamStore
-from ..ops import _lib, attention as attn_ops, fused, gemm
+from ..ops import _lib, attention as attn_ops, decode_stack, fused, gemm
 from ..ops._lib import c_float, c_int, c_void_p
 
 CFG_NORMS = {"none": 0, "global": 1, "channel": 2, "cfg_zero_star": 3}
@@ -74,6 +74,7 @@ class InferenceEngine:
         self._graph = self._capture_stream = None     # last captured decode step, for its memory (see _capture)
         self._graph_bytes = 0
         self.sp = None      # sequence-parallel sampling state (enable_sequence_parallel)
+        self._stack = None  # scratch of the whole-stack decode kernel
 
     def enable_sequence_parallel(self, group) -> None:
         """Splits the image tokens of :meth:`denoise` over the ranks of ``group`` (all of which run the same
@@ -134,6 +135,9 @@ class InferenceEngine:
         if self.offload is not None:
             self.offload.set_phase("prefix" if branch == UND else "denoise")
         static = self.offload is None           # offloaded weights arrive from a copy stream between the kernels
+        if (static and isinstance(plan, DecodeRows) and not cfg.is_moe
+                and decode_stack.takes(R, H, cfg.ffn_size, cfg.num_heads, cfg.num_kv_heads, plan.max_keys)):
+            return self._decode_layers(x, branch, pos3, plan, kv_rows, kv_len)
         h1, h2, x1 = (ws.get(n, (R, H)) for n in ("i.h1", "i.h2", "i.x1"))
         xo = [ws.get(f"i.x{i}", (R, H)) for i in range(2)]
         qkv, qk = ws.get("i.qkv", (R, qd + 2 * kd)), ws.get("i.qk", (R, qd + kd))
@@ -186,6 +190,18 @@ class InferenceEngine:
             else:
                 x = self._moe_ffn(WE, h2, x1, branch, xo[l & 1])
         return x
+
+    def _decode_layers(self, x, branch, pos3, plan, kv_rows, kv_len):
+        """:meth:`layers` for one new token of a few documents: one launch for the whole stack."""
+        cfg, p = self.cfg, self.p
+        if self._stack is None:
+            self._stack = decode_stack.Scratch(self.dev)
+        names = [f"layers.{l}.{{}}" for l in range(cfg.num_layers)]
+        table = [tuple(p[n.format(w)][branch] for w in ("wqkv", "wo", "w13", "w2", "attn_norm", "qk_norm", "ffn_norm"))
+                 + (self.kc[l], self.vc[l]) for l, n in enumerate(names)]
+        return decode_stack.decode_stack(x, table, self.ws.get("i.x0", tuple(x.shape)), self._stack, cfg.num_heads,
+                                         cfg.num_kv_heads, cfg.ffn_size, plan, kv_rows, pos3, kv_len, self.inv_t, self.inv_hw,
+                                         cfg.rms_eps, self.scale)
 
     def _moe_ffn(self, W, h2, x1, branch, out):
         """Dropless top-k expert FFN of one branch: device-side routing, tokens gathered into expert

@@ -1,0 +1,82 @@
+"""The whole-stack decode kernel (csrc/decode_stack.cu) against the kernels it stands in for and against fp64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(seed=3, **kw):
+    from sensenova_u1_b200.config import tiny_mot
+    from sensenova_u1_b200.inference import engine as E
+    from sensenova_u1_b200.models.params import ParamStore
+    cfg = tiny_mot(head_dim=128, patch_size=16, **kw)
+    store = ParamStore(cfg, device="cuda:0", with_grads=False)
+    store.init_weights(seed)
+    return E, cfg, E.InferenceEngine(cfg, store)
+
+
+# rings of 5 and 6 stages, one to many tiles per CTA, CTAs without rows, one to many parts per document
+SIZES = [dict(hidden_size=1024, num_heads=8, num_kv_heads=2, ffn_size=1024, num_layers=1),
+         dict(hidden_size=2048, num_heads=8, num_kv_heads=2, ffn_size=3072, num_layers=3),
+         dict(hidden_size=1024, num_heads=16, num_kv_heads=2, ffn_size=12288, num_layers=2)]
+
+
+@pytest.mark.parametrize("size", range(len(SIZES)))
+@pytest.mark.parametrize("lens", [(1,), (64,), (700,), (3000,), (9, 70), (300, 1)])
+def test_stack_equals_the_layers_one_by_one(size, lens, monkeypatch):
+    E, cfg, eng = _engine(**SIZES[size])
+    docs = [torch.arange(5, 5 + n) % cfg.vocab_size for n in lens]
+
+    def step(stack):
+        monkeypatch.setattr(E.decode_stack, "takes", lambda *a: stack)
+        lay, h = eng.prefill(docs, reserve_image_tokens=4)
+        dev = eng.dev
+        pos = torch.tensor([x.next_pos for x in lay], dtype=torch.int32, device=dev)
+        rows = torch.tensor([x.img_start for x in lay], device=dev)
+        mq = E.attn_ops.make_meta(torch.arange(len(lay), dtype=torch.int32, device=dev), pos)
+        eng._meta_k.index_copy_(0, rows, mq)
+        plan = E.DecodeRows(mq, eng._meta_k, torch.tensor([x.kv_start for x in lay], dtype=torch.int32, device=dev), max(lens) + 4)
+        x = eng.p["embed_tokens"][7:7 + len(lay)].contiguous()
+        out = eng.layers(x, E.UND, torch.stack([pos, pos * 0, pos * 0]), plan, rows, eng._meta_k.shape[0]).clone()
+        E._lib.check_status()
+        return out, [t.clone() for t in eng.kc + eng.vc], rows
+    want, cache, rows = step(False)
+    for _ in range(2):                                          # the barrier and the tickets are whole again after a launch
+        got, cache2, _ = step(True)
+        # the same roundings to bf16 at the same places (half a unit in the last place each), on sums in another order: a
+        # rounding that falls the other way is one unit, 2^-7, of one element; a handful of stages per layer compound
+        assert (got.double() - want.double()).norm() <= 2.0 ** -7 * cfg.num_layers * want.double().norm()
+        for a, b in zip(cache2, cache):
+            other = torch.ones(a.shape[0], dtype=torch.bool, device="cuda")
+            other[rows] = False
+            assert torch.equal(a[other], b[other])              # nothing else in the cache is touched
+            assert (a[rows].double() - b[rows].double()).norm() <= 2.0 ** -7 * cfg.num_layers * b[rows].double().norm()
+    monkeypatch.undo()
+
+
+@pytest.mark.parametrize("spoil", ["type", "shape", "stride"])
+def test_operands_of_other_forms_are_refused(spoil):
+    E, cfg, eng = _engine(**SIZES[0])
+    lay, h = eng.prefill([torch.arange(5, 9)], reserve_image_tokens=4)
+    dev = eng.dev
+    one = torch.tensor([4], dtype=torch.int32, device=dev)
+    plan = E.DecodeRows(E.attn_ops.make_meta(one * 0, one), eng._meta_k, one * 0, 8)
+    pos3 = torch.stack([one, one * 0, one * 0])
+    x = eng.p["embed_tokens"][7:8].contiguous()
+    if spoil == "type":
+        x = x.float()
+    elif spoil == "shape":
+        pos3 = pos3[:2].contiguous()
+    else:
+        pos3 = pos3.repeat(1, 2)[:, ::2]
+    with pytest.raises(ValueError):
+        eng._decode_layers(x, E.UND, pos3, plan, torch.tensor([4], device=dev), eng._meta_k.shape[0])
+
+
+def test_takes_refuses_what_the_kernel_is_not_built_for():
+    from sensenova_u1_b200.ops.decode_stack import takes
+    assert takes(1, 4096, 12288, 32, 8, 3072) and takes(2, 4096, 12288, 32, 8, 1) and takes(2, 1024, 1024, 8, 2, 9)
+    for bad in ((0, 1024, 1024, 8, 2, 9), (3, 1024, 1024, 8, 2, 9), (1, 1024, 32768, 8, 2, 9), (2, 16384, 4096, 32, 8, 9),
+                (1, 512, 1024, 8, 2, 9), (1, 1024, 1536, 8, 2, 9), (1, 1024, 0, 8, 2, 9), (1, 1024, 1024, 8, 4, 9),
+                (1, 1024, 1024, 4, 1, 9), (1, 1024, 1024, 8, 3, 9), (1, 4096, 12288, 32, 8, 3073)):
+        assert not takes(*bad)
