@@ -16,7 +16,7 @@ tools/key_mappings.json).  q/k/v and gate/up projections are stored fused.
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import Dict, Iterator, List, Tuple
+from typing import Dict, Iterator, List, Optional, Tuple
 
 import torch
 
@@ -204,17 +204,22 @@ class ParamStore:
                     n = min(step, flat.numel() - i)
                     flat[i:i + n] = (torch.randn(n, device=self.device, generator=g) * sd).to(self.dtype)
 
-    def zero_grads(self, keep_layer_matrices: bool = False) -> None:
+    def zero_grads(self, keep_layer_matrices: bool = False, keep: Optional[Dict[str, List[Tuple[int, int]]]] = None) -> None:
         """Clears the gradient arenas.  ``keep_layer_matrices``: the decoder layers' matrices are left as they are,
         for a caller whose first micro-batch *stores* those gradients instead of adding to them (saves clearing and
-        re-reading two bytes per parameter and step)."""
+        re-reading two bytes per parameter and step).  ``keep``: sorted ranges per arena that are left as well."""
         for a, t in self.grad_arena.items():
+            parts = [(0, self.sizes[a])]
             if a == "mat" and keep_layer_matrices:
-                for key, lo, hi in self.buckets("mat"):
-                    if not key.startswith("layer."):
-                        t[lo:hi].zero_()
-            else:
-                t.zero_()
+                parts = [(lo, hi) for key, lo, hi in self.buckets("mat") if not key.startswith("layer.")]
+            for lo, hi in parts:
+                for s, e in (keep or {}).get(a) or []:
+                    if lo < e and s < hi:
+                        if s > lo:
+                            t[lo:s].zero_()
+                        lo = e
+                if lo < hi:
+                    t[lo:hi].zero_()
 
     def named_parameters(self) -> Iterator[Tuple[str, torch.Tensor]]:
         for s in self.specs:

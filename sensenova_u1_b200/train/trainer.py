@@ -106,6 +106,7 @@ class Trainer:
                 self.engine.on_backward_begin = self.wp.begin_micro_backward
                 self.engine.on_layer_backward_begin = self._wp_layer_backward
         self._last_micro = True
+        self._cleared = set()           # matrix buckets whose frozen gradients this step has dropped
         self.profile_events = None      # set to a list to collect CUDA events around every optimizer step
 
     # ---------------------------------------------------------------------
@@ -139,9 +140,12 @@ class Trainer:
                        and type(self.engine).__name__ in ("MoTEngine", "MoEMoTEngine") and self.wp is None
                        and getattr(self.engine, "ep", None) is None
                        and getattr(self.engine, "cp", None) is None and getattr(self.engine, "tp", None) is None
-                       and not self.optim.cfg.frozen
                        and type(self.store).__name__ == "ParamStore")
-        self.store.zero_grads(keep_layer_matrices=True) if store_first else self.store.zero_grads()
+        if store_first:
+            # frozen ranges are cleared after the backward pass instead, whatever it left there
+            self.store.zero_grads(keep_layer_matrices=True, keep=self.optim.cfg.frozen)
+        else:
+            self.store.zero_grads()
         acc = None
         if self.wp is not None:
             self.wp.begin_step()
@@ -161,8 +165,11 @@ class Trainer:
             acc = out if acc is None else {k: acc[k] + out[k] for k in acc}
         if self.optim.cfg.frozen:
             for a in self.store.sizes:
-                if a != "mat" or self.engine is None:      # matrix buckets were cleared as they became ready
-                    self._clear_frozen(a, 0, self.store.sizes[a])
+                for name, lo, hi in self.store.buckets(a):
+                    if a != "mat" or name not in self._cleared:     # matrix buckets were cleared as they became ready
+                        self._clear_frozen(a, lo, hi)
+            self._cleared.clear()
+            self.optim.frozen_cleared = True
         self.sync_tp_replicated_grads()
         if getattr(self.engine, "sel_bias", None):
             self.engine.update_selection_bias(self.dp_group)
@@ -228,6 +235,7 @@ class Trainer:
                 for name, lo, hi in self.store.buckets("mat"):
                     if name == bucket:
                         self._clear_frozen("mat", lo, hi)
+                        self._cleared.add(name)
             self.optim.reduce_bucket("mat", bucket)
 
     def _weights_needed(self, bucket: str) -> None:
