@@ -8,6 +8,7 @@ tokenizer works) or with ``encode(text) -> list[int]`` and ``decode(list[int]) -
 from __future__ import annotations
 
 import json
+import re
 from dataclasses import dataclass, field
 from pathlib import Path
 from typing import List, Optional, Sequence, Tuple
@@ -17,6 +18,7 @@ import torch
 from ..config import ModelConfig
 from ..models.params import ParamStore
 from . import prompts
+from .engine import upload
 from .images import load_image_native, smart_resize  # noqa: F401  (re-exported: the reference's utils expose them next to the model)
 
 __version__ = "0.1.0"
@@ -285,7 +287,7 @@ class NEOChatModel:
         embs = []
         for im in images:
             p16, px, py, _, _ = patchify_block_major(im.to(dev).float(), cfg.patch_size, cfg.merge_size)
-            embs.append(self.engine.vision_embed("und", p16.to(torch.bfloat16), px.to(dev), py.to(dev)))
+            embs.append(self.engine.vision_embed("und", p16.to(torch.bfloat16), *upload(dev, px, py)))
         return embs
 
     def _embed_prompt(self, tokenizer, question: str, images: Sequence[torch.Tensor], system=None, tail: str = "",
@@ -302,15 +304,15 @@ class NEOChatModel:
         ctx_id = int(_encode(tokenizer, prompts.IMG_CONTEXT_TOKEN)[-1])
         self.img_context_token_id = ctx_id
         dev = self.store.device
-        x = self.store.p["embed_tokens"].index_select(0, ids.to(dev))
-        is_ctx = (ids == ctx_id)
+        rows = (ids == ctx_id).nonzero().view(-1)
+        dev_ids, dev_rows = upload(dev, ids, rows)
+        x = self.store.p["embed_tokens"].index_select(0, dev_ids)
         pos3 = self.get_thw_indexes(ids, [(im.shape[1] // tp, im.shape[2] // tp) for im in images], ctx_id)
         if images:
-            rows = is_ctx.nonzero().view(-1)
             embs = torch.cat(self._embed_images(images) if embs is None else embs)
             if rows.numel() != embs.shape[0]:
                 raise ValueError(f"{rows.numel()} image tokens in the prompt, {embs.shape[0]} embeddings")
-            x.index_copy_(0, rows.to(dev), embs)        # x is this call's own copy of the embedding rows
+            x.index_copy_(0, dev_rows, embs)        # x is this call's own copy of the embedding rows
         return ids, x, pos3
 
     def extract_feature(self, pixel_values, gen_model: bool = False, grid_hw=None) -> torch.Tensor:
@@ -327,7 +329,7 @@ class NEOChatModel:
             n = int(gh) * int(gw)
             px, py = patch_grid_positions(int(gh), int(gw), m)
             embs.append(self.engine.vision_embed("gen" if gen_model else "und", pixel_values[off:off + n].to(dev, torch.bfloat16),
-                                                 px.to(dev), py.to(dev)))
+                                                 *upload(dev, px, py)))
             off += n
         return torch.cat(embs)
 
@@ -447,12 +449,16 @@ class NEOChatModel:
         m = cfg.merge_size
         grids = [] if grid_hw is None else [(int(h) // m, int(w) // m) for h, w in torch.as_tensor(grid_hw).tolist()]
         pos3 = self.get_thw_indexes(ids, grids, self.img_context_token_id)
-        x = self.store.p["embed_tokens"].index_select(0, ids.to(dev))
+        rows = (ids == self.img_context_token_id).nonzero().view(-1)
+        dev_ids, dev_rows = upload(dev, ids, rows)
+        x = self.store.p["embed_tokens"].index_select(0, dev_ids)
         if pixel_values is not None or visual_features is not None:
             if visual_features is None:
                 visual_features = self.extract_feature(pixel_values, grid_hw=grid_hw)
-            x = x.clone()
-            x[(ids == self.img_context_token_id).to(dev)] = visual_features.reshape(-1, x.shape[1]).to(x.dtype)
+            visual_features = visual_features.reshape(-1, x.shape[1]).to(x.dtype)
+            if visual_features.shape[0] not in (1, rows.numel()):
+                raise RuntimeError(f"{rows.numel()} image tokens in the prompt, {visual_features.shape[0]} embeddings")
+            x.index_copy_(0, dev_rows, visual_features.expand(rows.numel(), -1))       # x is this call's own copy
         eos = gc.get("eos_token_id")
         stops = tuple(eos) if isinstance(eos, (list, tuple)) else ((int(eos),) if eos is not None else ())
         out = self._generate_ids(ids, x, pos3, int(gc.get("max_new_tokens", 256) or 256), stops, self._sampling(gc))
@@ -466,19 +472,17 @@ class ByteTokenizer:
     def __init__(self, vocab_size: int = 1024):
         self.specials = {s: 256 + i for i, s in enumerate(prompts.SPECIAL_TOKENS + [prompts.IM_START, prompts.IM_END])}
         self.inv = {v: k for k, v in self.specials.items()}
+        self._special = re.compile("|".join(map(re.escape, self.specials)))
         if vocab_size < 256 + len(self.specials):
             raise ValueError("vocabulary too small")
 
     def encode(self, text: str) -> List[int]:
         out, i = [], 0
-        while i < len(text):
-            for s, t in self.specials.items():
-                if text.startswith(s, i):
-                    out.append(t); i += len(s)
-                    break
-            else:
-                out += list(text[i].encode("utf-8")); i += 1
-        return out
+        for m in self._special.finditer(text):
+            out += text[i:m.start()].encode("utf-8")
+            out.append(self.specials[m.group()])
+            i = m.end()
+        return out + list(text[i:].encode("utf-8"))
 
     def __call__(self, text, **kw):
         return {"input_ids": self.encode(text)}

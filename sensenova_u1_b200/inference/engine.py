@@ -33,6 +33,27 @@ def _pad128(n):
     return (n + 127) // 128 * 128
 
 
+def upload(device, *tensors):
+    """Host tensors on the device, in one copy from pinned memory that nothing waits for.  (A copy from pageable memory
+    waits for all work of the stream: with ten of them per request, the device idled 2 - 8 ms while the host prepared
+    indexes, launches and the decode graph.)  Tensors that are on a device already are only moved if needed."""
+    device = torch.device(device)
+    host = [t for t in tensors if not t.is_cuda]
+    if device.type != "cuda" or not host:
+        return [t.to(device) for t in tensors]
+    offsets, n = [], 0
+    for t in host:
+        offsets.append(n)
+        n += (t.numel() * t.element_size() + 15) // 16 * 16
+    buf = torch.empty(max(n, 16), dtype=torch.uint8, pin_memory=True)
+    at = lambda b, t, o: b[o:o + t.numel() * t.element_size()].view(t.dtype).view(t.shape)
+    for t, o in zip(host, offsets):
+        at(buf, t, o).copy_(t)
+    dev = buf.to(device, non_blocking=True)
+    it = iter([at(dev, t, o) for t, o in zip(host, offsets)])
+    return [t.to(device) if t.is_cuda else next(it) for t in tensors]
+
+
 @dataclass
 class DocLayout:
     """Row ranges of one document inside the per-layer KV buffer."""
@@ -251,33 +272,37 @@ class InferenceEngine:
             layouts.append(DocLayout(kv_pos, n, kv_pos + n, n))
             kv_pos += n + reserve_image_tokens
         self.alloc_cache(_pad128(kv_pos))
-        R = sum(lens)
-        ids = torch.cat([d.to(self.dev) for d in docs_ids]).long()
-        x = self.p["embed_tokens"].index_select(0, ids) if docs_embeds is None else torch.cat(list(docs_embeds))
-        doc = torch.cat([torch.full((n,), i, dtype=torch.int32) for i, n in enumerate(lens)]).to(self.dev)
+        # indexes and metadata are made on the host (they come from it) and go up together
+        doc = torch.repeat_interleave(torch.arange(n_docs, dtype=torch.int32), torch.tensor(lens))
         if docs_pos3 is None:
-            pos = torch.cat([torch.arange(n, dtype=torch.int32) for n in lens]).to(self.dev)
-            pos3 = torch.stack([pos, torch.zeros_like(pos), torch.zeros_like(pos)]).contiguous()
+            pos = torch.cat([torch.arange(n, dtype=torch.int32) for n in lens])
+            pos3 = torch.stack([pos, torch.zeros_like(pos), torch.zeros_like(pos)])
             img = None
         else:
-            pos3 = torch.cat(list(docs_pos3), dim=1).to(self.dev).int().contiguous()
+            pos3 = torch.cat([p.cpu() for p in docs_pos3], dim=1).int().contiguous()
             pos = pos3[0]
             # tokens that share a t index with a neighbour belong to one image: bidirectional
             img = ((pos3[1] > 0) | (pos3[2] > 0) | (torch.roll(pos, 1) == pos) | (torch.roll(pos, -1) == pos)).int() * (pos + 1)
-        kv_rows = torch.cat([torch.arange(lay.kv_start, lay.kv_start + n) for lay, n in zip(layouts, lens)]).to(self.dev)
+        kv_rows = torch.cat([torch.arange(lay.kv_start, lay.kv_start + n) for lay, n in zip(layouts, lens)])
         # keys: cache rows [0, kv_pos); rows not written yet are blocked
-        mk = torch.zeros(kv_pos, 4, dtype=torch.int32, device=self.dev)
+        mk = torch.zeros(kv_pos, 4, dtype=torch.int32)
         mk[:, 0] = -7
         mk[:, 3] = attn_ops.FLAG_BLOCKED
         mq = attn_ops.make_meta(doc, pos, img)
         mk[kv_rows] = mq
-        plan = attn_ops.build_plan(mq, mk.contiguous())
+        self._meta_host = mk                         # as the prefill left it: decoding advances the device's copy
+        ends = torch.tensor(lens).cumsum(0) - 1
+        for lay, t in zip(layouts, pos[ends].tolist()):
+            lay.next_pos = t + 1
+        ids = None
+        if docs_embeds is None:
+            ids = torch.cat([d.to(docs_ids[0].device) for d in docs_ids]).long()
+        pos3, kv_rows, mk, mq, last, *ids = upload(self.dev, pos3, kv_rows, mk, mq, ends, *([] if ids is None else [ids]))
+        x = self.p["embed_tokens"].index_select(0, ids[0]) if docs_embeds is None else torch.cat(list(docs_embeds))
+        plan = attn_ops.build_plan(mq, mk)
         x = self.layers(x.contiguous(), UND, pos3, plan, kv_rows, kv_pos)
-        last = torch.tensor([sum(lens[:i + 1]) - 1 for i in range(n_docs)], device=self.dev)
         self._meta_k = mk
         self._doc_starts = [lay.kv_start for lay in layouts]
-        for lay, n in zip(layouts, lens):
-            lay.next_pos = int(pos3[0][sum(lens[:layouts.index(lay)]) + n - 1]) + 1
         return layouts, x.index_select(0, last)
 
     # ------------------------------------------------------------ text decoding
@@ -341,21 +366,24 @@ class InferenceEngine:
         if max_new_tokens <= 0:
             return [[] for _ in range(n_docs)]
         dev = self.dev
+        pos, kv_rows, doc, first = upload(
+            dev, torch.tensor([lay.next_pos for lay in layouts], dtype=torch.int32), torch.tensor([lay.img_start for lay in layouts]),
+            torch.arange(n_docs, dtype=torch.int32), torch.tensor(self._doc_starts[:n_docs], dtype=torch.int32))
         st = {
             "h": last_hidden.contiguous().clone(),
             "out": torch.full((n_docs, max_new_tokens), -1, dtype=torch.long, device=dev),
             "step": torch.zeros(1, dtype=torch.long, device=dev),
-            "pos": torch.tensor([lay.next_pos for lay in layouts], dtype=torch.int32, device=dev),
-            "kv_rows": torch.tensor([lay.img_start for lay in layouts], dtype=torch.long, device=dev),
-            "doc": torch.arange(n_docs, dtype=torch.int32, device=dev),
+            "pos": pos,
+            "kv_rows": kv_rows,
+            "doc": doc,
         }
         kv_len = self._meta_k.shape[0]
         # Documents are numbered by their place in the last prefill: when the layouts are those documents in order, row
         # d reads cache rows [kv_start, its own] and nothing else can be visible to it, so its keys are split over CTAs.
         # Any other selection of layouts takes the tile plan, which looks at every cache row.
-        first = None
-        if [lay.kv_start for lay in layouts] == self._doc_starts[:n_docs]:
-            first = torch.tensor(self._doc_starts[:n_docs], dtype=torch.int32, device=dev)
+        if [lay.kv_start for lay in layouts] != self._doc_starts[:n_docs]:
+            first = None
+        else:
             max_keys = max(lay.img_start - lay.kv_start for lay in layouts) + max_new_tokens
         if sampling and float(sampling.get("repetition_penalty", 1.0) or 1.0) != 1.0:
             vocab = self.p["lm_head"].shape[0]
@@ -567,14 +595,18 @@ class InferenceEngine:
         ww = torch.arange(tw, dtype=torch.int32).view(1, tw).expand(th, tw).reshape(-1)
         # rows are grouped by branch: [all conditional images | all unconditional | all image-only]
         order = [i for k in range(nb) for i in range(n_docs) if i % nb == k]
-        pos3 = torch.cat([torch.stack([torch.full((T,), layouts[i].next_pos, dtype=torch.int32), hh, ww]) for i in order],
-                         dim=1).to(self.dev).contiguous()
-        kv_rows = torch.cat([torch.arange(layouts[i].img_start, layouts[i].img_start + T) for i in order]).to(self.dev)
-        doc = torch.cat([torch.full((T,), i, dtype=torch.int32) for i in order]).to(self.dev)
-        big = torch.full_like(doc, 1 << 28)
-        mq = attn_ops.make_meta(doc, big)
-        mk = self._meta_k.clone()
+        pos3 = torch.cat([torch.stack([torch.full((T,), layouts[i].next_pos, dtype=torch.int32), hh, ww]) for i in order], dim=1)
+        kv_rows = torch.cat([torch.arange(layouts[i].img_start, layouts[i].img_start + T) for i in order])
+        doc = torch.cat([torch.full((T,), i, dtype=torch.int32) for i in order])
+        mk = self._meta_host.clone()
         mk[kv_rows] = attn_ops.make_meta(doc, torch.zeros_like(doc))
+        m, ps = cfg.merge_size, cfg.patch_size
+        ty = hh.view(-1, 1, 1) * m + torch.arange(m, dtype=torch.int32).view(1, m, 1)
+        tx = ww.view(-1, 1, 1) * m + torch.arange(m, dtype=torch.int32).view(1, 1, m)
+        py = ty.expand(T, m, m).reshape(-1).repeat(batch_size)
+        px = tx.expand(T, m, m).reshape(-1).repeat(batch_size)
+        pos3, kv_rows, mq, mk, px, py = upload(self.dev, pos3, kv_rows, attn_ops.make_meta(doc, torch.full_like(doc, 1 << 28)), mk,
+                                               px, py)
         publish = None
         if sp is not None:
             # my rows: the slice [s0, s0 + Tl) of every document, in the same document order
@@ -583,7 +615,7 @@ class InferenceEngine:
             kv_rows = kv_rows.index_select(0, loc)
             mq = mq.index_select(0, loc).contiguous()
             publish = [(j * Tl, Tl, layouts[i].img_start + s0) for j, i in enumerate(order)]
-        plan = attn_ops.build_plan(mq, mk.contiguous())
+        plan = attn_ops.build_plan(mq, mk)
         kv_len = mk.shape[0]
         ns = min(math.sqrt(T / float(cfg.noise_scale_base_image_seq_len)) * cfg.noise_scale
                  if cfg.noise_scale_mode in ("resolution", "dynamic", "dynamic_sqrt") else cfg.noise_scale,
@@ -593,13 +625,8 @@ class InferenceEngine:
             noise = torch.randn(batch_size, 3, Hh, W, device=self.dev, generator=g)
         img = ns * noise.float()
         z = img.reshape(batch_size, 3, th, tp, tw, tp).permute(0, 2, 4, 3, 5, 1).reshape(batch_size * T, cfg.token_dim).contiguous()
-        m, ps = cfg.merge_size, cfg.patch_size
         patches = z.reshape(batch_size * T, m, ps, m, ps, 3).permute(0, 1, 3, 5, 2, 4).reshape(
             batch_size * T * m * m, cfg.patch_dim).to(torch.bfloat16).contiguous()
-        ty = hh.view(-1, 1, 1) * m + torch.arange(m, dtype=torch.int32).view(1, m, 1)
-        tx = ww.view(-1, 1, 1) * m + torch.arange(m, dtype=torch.int32).view(1, 1, m)
-        py = ty.expand(T, m, m).reshape(-1).repeat(batch_size).to(self.dev).contiguous()
-        px = tx.expand(T, m, m).reshape(-1).repeat(batch_size).to(self.dev).contiguous()
         ts = torch.linspace(0.0, 1.0, num_steps + 1)
         ts = apply_time_schedule(ts, T, cfg, timestep_shift=timestep_shift).tolist()
         ns_emb = None
@@ -630,7 +657,7 @@ class InferenceEngine:
             else:  # outside the guidance interval only the conditional documents run
                 sub = slice(0, BTl)
                 if plan_c is None:
-                    plan_c = attn_ops.build_plan(mq[sub].contiguous(), mk.contiguous())
+                    plan_c = attn_ops.build_plan(mq[sub].contiguous(), mk)
                 h = self.layers(emb.contiguous(), GEN, pos3[:, sub].contiguous(), plan_c, kv_rows[sub], kv_len,
                                 publish[:batch_size] if publish is not None else None)
             hf = self.final_norm(h, GEN)
