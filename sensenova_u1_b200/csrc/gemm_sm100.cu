@@ -1123,16 +1123,22 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
     return kHostBadArg;
   }
   const int G = group_mode == 0 ? 1 : num_groups;
-  // Up to 128 rows of A, plain y = x W^T: the weight-streaming kernel.  us, weights cold in L2, streaming / pair:
-  //   rows                  64         128         129         256         512
-  //   24576 x 4096     41.8/59.1   45.8/59.1   67.7/58.8   77.6/62.4    128/82.8
-  //   151936 x 4096     216/252     260/254     469/270     497/275    1025/575
-  //   6144 x 4096      16.6/31.1   19.1/31.1   23.8/30.9   24.7/30.7   34.3/32.9
-  //   4096 x 4096      13.5/29.6   15.4/29.1   17.7/29.5   17.8/30.1   24.6/30.3
-  //   4096 x 12288     26.7/74.7   28.7/68.3   35.7/68.5   35.7/67.8   57.6/67.1
-  // The line is right for weights whose tiles fill the chip; for the others it lies too low (a second row tile reads the
-  // weights again, but from L2).
-  if (M <= 128 && group_mode == 0 && !a_mn && !b_mn && (out_mode == 0 || out_mode == 2) && comm == nullptr &&
+  // Few rows of A, plain y = x W^T: the weight-streaming kernel, up to 128 rows always, beyond (up to 1024, where a row tile
+  // more reads the weights again from L2) as long as its 128 x 128 tiles are one wave: the 256 x 256 tiles of the pair kernel
+  // are then at most half of what the chip takes at once.  Beyond 128 rows only for an inference engine's weights (w_static):
+  // a reduction in parts has other roundings, which training amplifies from step to step.  us, weights cold in L2, streaming /
+  // pair:
+  //   rows                  64         128         129         256         384         512         1024
+  //   24576 x 4096     41.8/59.1   45.8/59.1   67.7/58.8   77.6/62.4               128/82.8
+  //   151936 x 4096     216/252     260/254     469/270     497/275                1025/575
+  //   8192 x 4096                              23.2/27.2   23.7/27.3        -/28.5
+  //   6144 x 4096      16.6/31.1   19.1/31.1   21.7/27.1   22.7/27.8   23.1/28.2        -/28.5
+  //   4096 x 4096      13.5/29.6   15.4/29.1   14.4/26.0   15.5/26.0   21.9/26.3   22.0/26.4        -/27.8
+  //   4096 x 12288     26.7/74.7   28.7/68.3   32.2/62.1   32.7/62.2   54.5/62.0   54.3/62.5        -/74.1
+  //   2048 x 4096      10.5/27.5   12.5/27.6   10.6/25.8   12.2/25.8   14.9/26.0   15.2/26.0   21.8/26.3
+  //   128 x 2048                                9.6/14.6    9.8/14.7    9.8/14.7    9.8/14.7    9.8/14.7
+  const bool few = M <= 128 || (M <= 1024 && w_static && !swiglu && (long long)((N + 127) / 128) * ((M + 127) / 128) <= num_sms());
+  if (few && group_mode == 0 && !a_mn && !b_mn && (out_mode == 0 || out_mode == 2) && comm == nullptr &&
       (g_pair_mode != 0 || swiglu) && K > 0)
     return launch_gemm_small(A, B, C, M, N, K, lda, ldb, ldc, out_mode == 2, residual, ldr, alpha, 0, w_static, swiglu,
                              stream);

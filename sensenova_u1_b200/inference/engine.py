@@ -112,11 +112,11 @@ class InferenceEngine:
     def vision_embed(self, br: str, patches, px, py):
         cfg, p = self.cfg, self.p
         m2 = cfg.merge_size ** 2
-        a1 = gemm.gemm_nt(patches, p[f"vision_{br}.patch_w"], residual=p[f"vision_{br}.patch_b"])
+        a1 = gemm.gemm_nt(patches, p[f"vision_{br}.patch_w"], residual=p[f"vision_{br}.patch_b"], w_static=True)
         fused.gelu_fwd(a1, a1)
         r1 = fused.rope2d(a1, torch.empty_like(a1), px, py, self.inv_v)
         return gemm.gemm_nt(r1.view(r1.shape[0] // m2, m2 * cfg.vision_hidden), p[f"vision_{br}.merge_w"],
-                            residual=p[f"vision_{br}.merge_b"])
+                            residual=p[f"vision_{br}.merge_b"], w_static=True)
 
     def scalar_embed(self, name, t):
         p = self.p
@@ -665,9 +665,9 @@ class InferenceEngine:
                 # convolutional decoder: cuDNN convolutions on the token grids (not a tcgen05 path)
                 x_pred = oracle.pixel_head(self.p, hf, [(th, tw)] * (hf.shape[0] // T), cfg).to(torch.bfloat16).contiguous()
             else:
-                a1 = gemm.gemm_nt(hf, self.p["fm_head.w1"], residual=self.p["fm_head.b1"])
+                a1 = gemm.gemm_nt(hf, self.p["fm_head.w1"], residual=self.p["fm_head.b1"], w_static=True)
                 fused.gelu_fwd(a1, a1)
-                x_pred = gemm.gemm_nt(a1, self.p["fm_head.w2"], residual=self.p["fm_head.b2"])
+                x_pred = gemm.gemm_nt(a1, self.p["fm_head.w2"], residual=self.p["fm_head.b2"], w_static=True)
             if par is not None:
                 from ..parallel.symm import peer_put
                 buf = par["x"][step & 1]                     # two buffers: a slow peer may still read the other

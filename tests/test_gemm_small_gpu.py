@@ -144,3 +144,24 @@ def test_static_weights_written_just_before_a_request():
                     assert torch.equal(got[0], ref[0]) and got[1] == ref[1]
                     assert torch.equal(got[2], ref[2]) and torch.equal(got[3], ref[3])
     assert not torch.equal(want[0][0], want[1][0])
+
+
+@pytest.mark.parametrize("N,K,M,streams", [(4096, 1096, 512, True), (4096, 1096, 513, False), (2048, 1096, 1024, True),
+                                           (2048, 1096, 1025, False), (128, 520, 1000, True), (6144, 520, 384, True),
+                                           (6144, 520, 385, False), (18944, 200, 128, True), (18944, 200, 129, False)])
+def test_one_wave_of_tiles_takes_the_weight_streaming_kernel(N, K, M, streams):
+    """An engine's weights up to 1024 rows, while 128 x 128 tiles are one wave (148 SMs)."""
+    from sensenova_u1_b200.ops import _lib, gemm
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the line is drawn by the number of SMs")
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w, r = (torch.randn(n, k, device="cuda", generator=g).to(torch.bfloat16) for n, k in ((M, K), (N, K), (M, N)))
+    y = gemm.gemm_nt(x, w, residual=r, w_static=True)
+    f = gemm.gemm_nt(x, w, out_mode=gemm.OUT_F32_STORE, w_static=True)
+    one = _streamed(x, w, torch.empty_like(f))
+    _lib.check_status()
+    ref = x.double() @ w.double().t()
+    # fp32 sums of K / 16 tensor-core steps, each off by at most one unit in the last place of a partial sum
+    assert (f - ref).norm() / ref.norm() < K / 16 * 2.0 ** -23 + 1e-6
+    assert ((y.double() - ref - r.double()).abs() <= (ref + r.double()).abs() * 2.0 ** -8 + 1e-2).all()
+    assert torch.equal(f, one) or not streams
