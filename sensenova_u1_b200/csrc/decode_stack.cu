@@ -516,11 +516,15 @@ __device__ __forceinline__ void attend(const Args& a, Smem& s, float* red, const
     named_bar_sync(1, CT);                                   // the unit before has left the buffers
     const int sp = t.sp, hgp = t.hgp, m = t.m, kvh = t.kvh, h0 = hgp * HG, k_lo = t.lo, k_hi = t.hi;
     const long long last = t.last;
+    const int4 mqr = *reinterpret_cast<const int4*>(a.meta_q + m);
+    const TokMeta mq{mqr.x, mqr.y, mqr.z, mqr.w};
     if (warp < (HG + 2) / 2) {
       // q heads, the key and the value of this row: 16 lanes of 8 elements each
       const int head = grp;
       const int src = head < HG ? h0 + head : head == HG ? a.Hq + kvh : a.Hq + a.Hkv + kvh;
       const uint2* qp = a.qkv + ((long long)m * (a.Hq + 2 * a.Hkv) + src) * 64 + sub * 4;
+      const __nv_bfloat16* gp = L.qk_norm + (head >= HG ? 128 : 0) + (sub >= 8 ? 64 : 0) + (sub & 7) * 8;
+      const uint4 gr = __ldg(reinterpret_cast<const uint4*>(gp));
       uint4 w0, w1;
       poll(a, s, [&]() {
         w0 = ld_words(qp);
@@ -528,8 +532,6 @@ __device__ __forceinline__ void attend(const Args& a, Smem& s, float* red, const
         return w0.y == in && w0.w == in && w1.y == in && w1.w == in;
       });
       const uint4 raw = make_uint4(w0.x, w0.z, w1.x, w1.z);
-      const __nv_bfloat16* gp = L.qk_norm + (head >= HG ? 128 : 0) + (sub >= 8 ? 64 : 0) + (sub & 7) * 8;
-      const uint4 gr = __ldg(reinterpret_cast<const uint4*>(gp));
       float v[8], g[8], o[8];
       unpack8(raw, v);
       unpack8(gr, g);
@@ -576,8 +578,6 @@ __device__ __forceinline__ void attend(const Args& a, Smem& s, float* red, const
         q2[h][i] = pack_f32x2(f.x, f.y);
         acc[h][i] = 0ull;
       }
-    const int4 mqr = *reinterpret_cast<const int4*>(a.meta_q + m);
-    const TokMeta mq{mqr.x, mqr.y, mqr.z, mqr.w};
     float mx = -INFINITY, l = 0.f;                           // of this lane's head, over the keys of its group
     for (int k0 = k_lo; k0 < k_hi; k0 += GROUPS * U) {
       if (k0 != k_lo) load_keys(a, L, t, k0, x);

@@ -318,14 +318,16 @@ class InferenceEngine:
         generated tokens; positive logits divided by the penalty, negative ones multiplied), then, with ``do_sample``,
         temperature, top-k and nucleus (top-p) filtering and a draw by the exponential-race form of categorical
         sampling (argmax of p / Exp(1)), which stays on the device and is capturable in a CUDA graph."""
+        best = lambda x: (decode_stack.argmax_rows(x) if x.is_cuda and x.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1
+                          and x.stride(0) >= x.shape[1] and 0 < x.shape[0] < 65536 and x.shape[1] > 0 else x.argmax(-1))
         if not sampling:
-            return logits.argmax(-1)
+            return best(logits)
         lg = logits.float()
         rp = float(sampling.get("repetition_penalty", 1.0) or 1.0)
         if seen is not None and rp != 1.0:
             lg = torch.where(seen, torch.where(lg > 0, lg / rp, lg * rp), lg)
         if not sampling.get("do_sample", False):
-            return lg.argmax(-1)
+            return best(lg)
         t = float(sampling.get("temperature", 1.0) or 1.0)
         k = int(sampling.get("top_k", 0) or 0)
         p_ = float(sampling.get("top_p", 1.0) or 1.0)
@@ -366,17 +368,11 @@ class InferenceEngine:
         if max_new_tokens <= 0:
             return [[] for _ in range(n_docs)]
         dev = self.dev
-        pos, kv_rows, doc, first = upload(
+        pos, kv_rows, first = upload(
             dev, torch.tensor([lay.next_pos for lay in layouts], dtype=torch.int32), torch.tensor([lay.img_start for lay in layouts]),
-            torch.arange(n_docs, dtype=torch.int32), torch.tensor(self._doc_starts[:n_docs], dtype=torch.int32))
-        st = {
-            "h": last_hidden.contiguous().clone(),
-            "out": torch.full((n_docs, max_new_tokens), -1, dtype=torch.long, device=dev),
-            "step": torch.zeros(1, dtype=torch.long, device=dev),
-            "pos": pos,
-            "kv_rows": kv_rows,
-            "doc": doc,
-        }
+            torch.tensor(self._doc_starts[:n_docs], dtype=torch.int32))
+        rows = decode_stack.Rows(pos, kv_rows, self.cfg.hidden_size, max_new_tokens)
+        st = {"h": last_hidden.contiguous().clone()}
         kv_len = self._meta_k.shape[0]
         # Documents are numbered by their place in the last prefill: when the layouts are those documents in order, row
         # d reads cache rows [kv_start, its own] and nothing else can be visible to it, so its keys are split over CTAs.
@@ -396,26 +392,18 @@ class InferenceEngine:
             nxt = self._pick_token(logits, sampling, st.get("seen"))
             if "seen" in st:
                 st["seen"].scatter_(1, nxt.view(-1, 1), True)
-            st["out"].index_copy_(1, st["step"], nxt.view(-1, 1))
-            x = self.p["embed_tokens"].index_select(0, nxt)
-            zero = torch.zeros_like(st["pos"])
-            pos3 = torch.stack([st["pos"], zero, zero]).contiguous()
-            mq = attn_ops.make_meta(st["doc"], st["pos"])
-            self._meta_k.index_copy_(0, st["kv_rows"], mq)
-            plan = (DecodeRows(mq, self._meta_k, first, max_keys) if first is not None
-                    else attn_ops.build_plan(mq, self._meta_k))
-            h = self.layers(x.contiguous(), UND, pos3, plan, st["kv_rows"], kv_len)
-            st["h"].copy_(h)
-            st["pos"].add_(1)
-            st["kv_rows"].add_(1)
-            st["step"].add_(1)
+            rows.advance(nxt, self.p["embed_tokens"], self._meta_k)
+            plan = (DecodeRows(rows.meta_q, self._meta_k, first, max_keys) if first is not None
+                    else attn_ops.build_plan(rows.meta_q, self._meta_k))
+            # the same buffer after every step: the captured step reads what it (or the eager one) has left there
+            st["h"] = self.layers(rows.x, UND, rows.pos3, plan, rows.kv_rows, kv_len)
 
         done = 0
         graph = None
         stops = set(int(t) for t in stop_ids)
 
         def finished():
-            toks = st["out"][:, :done].tolist()
+            toks = rows.out[:, :done].tolist()
             return all(any(t in stops for t in row) for row in toks) if stops else False
 
         if sampling and sampling.get("do_sample", False) and sampling.get("seed") is not None and dev.type == "cuda":
@@ -432,7 +420,7 @@ class InferenceEngine:
             else:
                 step_fn()
             done += 1
-        toks = st["out"][:, :done].tolist()
+        toks = rows.out[:, :done].tolist()
         out = []
         for row in toks:
             cut = len(row)

@@ -62,3 +62,45 @@ def decode_stack(x, layers, out, scratch: Scratch, heads: int, kv_heads: int, ff
               P(scratch.count), P(plan.meta_q), P(plan.meta_k), P(plan.first), P(kv_rows), P(pos3), P(inv_t), P(inv_hw),
               c_int(plan.max_keys), c_float(eps), c_float(scale), c_void_p(_lib.stream()))
     return out
+
+
+# ---- between the LM head and the layers (csrc/decode_step.cu) -----------------------------------------------------
+def argmax_rows(x):
+    """``x.argmax(-1)`` of fp32 rows: NaN counts as largest, of equal elements the first."""
+    rows, V = x.shape
+    if x.dtype != torch.float32 or x.stride(1) != 1 or (rows > 1 and x.stride(0) < V):
+        raise ValueError("argmax_rows takes fp32 rows")
+    out = torch.empty(rows, dtype=torch.long, device=x.device)
+    _lib.call("argmax_rows", c_void_p(x.data_ptr()), c_ll(max(x.stride(0), V)), c_int(rows), c_int(V), c_void_p(out.data_ptr()),
+              c_void_p(_lib.stream()))
+    return out
+
+
+class Rows:
+    """Device state of a decode: what the step in progress reads (``x``, ``pos3``, ``meta_q``, ``kv_rows``) and what
+    :meth:`advance` needs to make it from the next tokens."""
+
+    def __init__(self, pos, kv_rows, hidden: int, new: int):
+        """``pos`` (int32) / ``kv_rows`` (int64): position and cache row of every document's first new token."""
+        n, dev = pos.numel(), pos.device
+        if pos.dtype != torch.int32 or kv_rows.dtype != torch.int64 or kv_rows.numel() != n:
+            raise ValueError("positions are int32 and cache rows int64, one per document")
+        self.pos0, self.row0 = pos.contiguous(), kv_rows.contiguous()
+        self.out = torch.full((n, new), -1, dtype=torch.long, device=dev)
+        self.done = torch.zeros(n, dtype=torch.int32, device=dev)
+        self.x = torch.empty(n, hidden, dtype=torch.bfloat16, device=dev)
+        self.pos3 = torch.empty(3, n, dtype=torch.int32, device=dev)
+        self.meta_q = torch.empty(n, 4, dtype=torch.int32, device=dev)
+        self.kv_rows = torch.empty(n, dtype=torch.int64, device=dev)
+
+    def advance(self, tokens, embed, meta_k):
+        """Tokens (int64 [docs]) are stored; their embeddings, positions, cache rows and metadata become the step's."""
+        n, H = self.x.shape
+        if (tokens.dtype != torch.int64 or tokens.numel() != n or not tokens.is_contiguous() or embed.dtype != torch.bfloat16
+                or embed.shape[1] != H or not embed.is_contiguous() or meta_k.dtype != torch.int32 or meta_k.shape[1] != 4
+                or not meta_k.is_contiguous()):
+            raise ValueError("advance: tokens int64 [docs], embedding [vocab, hidden], metadata int32 [rows, 4]")
+        P = lambda t: c_void_p(t.data_ptr())
+        _lib.call("decode_advance", P(tokens), P(embed), c_int(embed.shape[0]), c_int(H), c_int(n), c_int(meta_k.shape[0]), P(self.done),
+                  P(self.pos0), P(self.row0), P(self.out), c_int(self.out.shape[1]), P(self.x), P(self.pos3), P(self.meta_q),
+                  P(meta_k), P(self.kv_rows), c_void_p(_lib.stream()))
