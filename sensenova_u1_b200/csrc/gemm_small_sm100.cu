@@ -58,6 +58,7 @@ struct Args {
   int w_static;       // w may be read before the preceding kernel has finished
   const int* tile_group;   // experts: weight set of row tile blockIdx.y (negative: unused tile); null: one weight set
   int w_rows;         // rows of w per weight set
+  int x_shared;       // experts: every tile reads rows 0 .. of x (one row that all of them share)
   int* status;
 };
 
@@ -94,6 +95,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
     m0 = blockIdx.y * 128;
     w0 = g * args.w_rows;
   }
+  const int x0 = args.x_shared ? 0 : m0;
   const int chunks = (args.K + BK - 1) / BK;
   const int c_lo = (int)((long long)chunks * rank / args.split);
   const int c_hi = (int)((long long)chunks * (rank + 1) / args.split);
@@ -132,13 +134,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
       pdl_wait();
       pdl_trigger();
       for (int i = 0; i < pre; ++i)
-        tma_load_2d(smem + i * C::STAGE + W_STAGE, &tmX, &full_bar[i], (c_lo + i) * BK, m0);
+        tma_load_2d(smem + i * C::STAGE + W_STAGE, &tmX, &full_bar[i], (c_lo + i) * BK, x0);
       for (int i = pre; i < n; ++i) {
         const int s = i % C::STAGES;
         if (!mbar_wait(&empty_bar[s], ((i / C::STAGES) & 1) ^ 1, abort_flag, args.status, 1)) break;
         mbar_expect_tx(&full_bar[s], C::STAGE);
         load_w(s, c_lo + i);
-        tma_load_2d(smem + s * C::STAGE + W_STAGE, &tmX, &full_bar[s], (c_lo + i) * BK, m0);
+        tma_load_2d(smem + s * C::STAGE + W_STAGE, &tmX, &full_bar[s], (c_lo + i) * BK, x0);
       }
     }
     __syncwarp();
@@ -306,7 +308,7 @@ static int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const Args& a,
 static int launch_gemm_small_any(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw,
                                  long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
                                  int w_static, int swiglu, const int* tile_group, int tiles_m, int w_rows,
-                                 long long w_total, cudaStream_t st) {
+                                 long long w_total, int x_shared, cudaStream_t st) {
   using namespace gsmall;
   const int tn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   const int mt = tiles_m > 0 ? tiles_m : (M + tn - 1) / tn;
@@ -336,7 +338,7 @@ static int launch_gemm_small_any(const void* x, const void* w, void* c, int M, i
     if ((rc = encode_tmap_bf16(&tmW, w, 2, dims, strides, box)) != kHostOk) return rc;
   }
   {
-    uint64_t dims[2] = {(uint64_t)K, tiles_m > 0 ? (uint64_t)tiles_m * 128 : (uint64_t)M};
+    uint64_t dims[2] = {(uint64_t)K, tiles_m > 0 && !x_shared ? (uint64_t)tiles_m * 128 : (uint64_t)M};
     uint64_t strides[1] = {(uint64_t)ldx * 2};
     uint32_t box[2] = {BK, (uint32_t)tn};
     if ((rc = encode_tmap_bf16(&tmX, x, 2, dims, strides, box)) != kHostOk) return rc;
@@ -346,6 +348,7 @@ static int launch_gemm_small_any(const void* x, const void* w, void* c, int M, i
   a.M = tiles_m > 0 ? tiles_m * 128 : M;
   a.tile_group = tile_group;
   a.w_rows = w_rows;
+  a.x_shared = x_shared;
   a.N = N;
   a.K = K;
   a.split = split;
@@ -373,7 +376,7 @@ int launch_gemm_small(const void* x, const void* w, void* c, int M, int N, int K
                       long long ldc, int f32_out, const void* residual, long long ldr, float alpha, int split,
                       int w_static, int swiglu, cudaStream_t st) {
   return launch_gemm_small_any(x, w, c, M, N, K, ldx, ldw, ldc, f32_out, residual, ldr, alpha, split, w_static, swiglu,
-                               nullptr, 0, 0, (long long)N * (swiglu ? 2 : 1), st);
+                               nullptr, 0, 0, (long long)N * (swiglu ? 2 : 1), 0, st);
 }
 
 }  // namespace snu1
@@ -400,11 +403,12 @@ SNU1_API int snu1_gemm_small(const void* x, const void* w, void* c, int M, int N
 
 // Expert products of a few rows: row tile t (rows 128 t .. 128 t + rows - 1 of x and y, rows <= 128) times the weights of
 // expert tile_group[t], w[experts][w_rows][K] contiguous; tiles with a negative entry are skipped.  swiglu: w_rows = 2 N,
-// y = silu(gate) * up, else w_rows = N.  Rows of a tile past those in use are computed from whatever x holds there.
+// y = silu(gate) * up, else w_rows = N.  x_shared: x has the one set of rows that every tile reads.  Rows of a tile past those in
+// use are computed from whatever x holds there.
 // One token, 8 of 128 experts, 768 x 2048: gate / up with activation 37.4 (pair kernel over padded tiles) -> 12 us, down
 // 23.6 -> 8 us (floors 7.6 and 3.8).
 SNU1_API int snu1_gemm_experts(const void* x, const void* w, void* y, int tiles, int rows, int N, int K, long long ldx,
-                               long long ldy, const int* tile_group, int experts, int swiglu, void* stream) {
+                               long long ldy, const int* tile_group, int experts, int swiglu, int x_shared, void* stream) {
   using namespace snu1;
   if (tiles <= 0 || tiles > 65535 || rows <= 0 || rows > 128 || N <= 0 || N % 8 || K <= 0 || K % 8 || ldx % 8 || ldy % 8 ||
       experts <= 0 || tile_group == nullptr || (reinterpret_cast<uintptr_t>(y) & 15) != 0) {
@@ -414,5 +418,5 @@ SNU1_API int snu1_gemm_experts(const void* x, const void* w, void* y, int tiles,
   }
   const int w_rows = swiglu ? 2 * N : N;
   return launch_gemm_small_any(x, w, y, rows, N, K, ldx, K, ldy, 0, nullptr, 0, 1.0f, 0, 0, swiglu, tile_group, tiles,
-                               w_rows, (long long)experts * w_rows, reinterpret_cast<cudaStream_t>(stream));
+                               w_rows, (long long)experts * w_rows, x_shared, reinterpret_cast<cudaStream_t>(stream));
 }

@@ -329,6 +329,91 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ yp, const i
   }
 }
 
+// The same for a few rows, and the norm that follows: h = rmsnorm(y) * gain.  A CTA per row, y stays in registers.  A decode step of
+// one row is bound by its chain of short launches; this is one less per layer, and a single row is read in place by its experts,
+// another one less: a request of 24 tokens, 8 layers with 128 experts of 768 x 2048: 19.1 -> 17.6 ms.
+constexpr int CN_THREADS = 256, CN_VEC = 4;      // up to 8192 columns
+__global__ void __launch_bounds__(CN_THREADS)
+    moe_combine_norm_kernel(const __nv_bfloat16* __restrict__ yp, const int* __restrict__ dest, const int* __restrict__ top_idx,
+                            const float* __restrict__ top_w, const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ y,
+                            const __nv_bfloat16* __restrict__ gain, __nv_bfloat16* __restrict__ h, int K, int H, float eps) {
+  __shared__ float scratch[CN_THREADS / 32];
+  const long long row = blockIdx.x;
+  const int hv = H / 8;
+  float acc[CN_VEC][8];
+  uint4 g[CN_VEC];
+#pragma unroll
+  for (int j = 0; j < CN_VEC; ++j)
+    if (threadIdx.x + j * CN_THREADS < hv) g[j] = __ldg(reinterpret_cast<const uint4*>(gain) + threadIdx.x + j * CN_THREADS);
+  pdl_wait();
+  pdl_trigger();
+  auto add = [](float (&a)[8], const uint4& u, float w) {
+    const uint32_t v[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      a[2 * e] += w * __uint_as_float(v[e] << 16);
+      a[2 * e + 1] += w * __uint_as_float(v[e] & 0xffff0000u);
+    }
+  };
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < CN_VEC; ++j) {
+    const int c = threadIdx.x + j * CN_THREADS;
+    if (c >= hv) break;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[j][e] = 0.f;
+    add(acc[j], reinterpret_cast<const uint4*>(residual + row * H)[c], 1.f);
+    for (int k0 = 0; k0 < K; k0 += 4) {
+      uint4 u[4];
+      float w[4];
+      bool ok[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const long long rk = row * K + min(k0 + i, K - 1);
+        ok[i] = k0 + i < K && top_idx[rk] >= 0;
+        w[i] = top_w[rk];
+        if (ok[i]) u[i] = reinterpret_cast<const uint4*>(yp + (long long)dest[rk] * H)[c];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (ok[i]) add(acc[j], u[i], w[i]);
+    }
+    uint4 o;
+    o.x = pack_bf16x2(acc[j][0], acc[j][1]);
+    o.y = pack_bf16x2(acc[j][2], acc[j][3]);
+    o.z = pack_bf16x2(acc[j][4], acc[j][5]);
+    o.w = pack_bf16x2(acc[j][6], acc[j][7]);
+    reinterpret_cast<uint4*>(y + row * H)[c] = o;
+    const uint32_t v[4] = {o.x, o.y, o.z, o.w};        // the norm sees the stored values
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      acc[j][2 * e] = __uint_as_float(v[e] << 16);
+      acc[j][2 * e + 1] = __uint_as_float(v[e] & 0xffff0000u);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss += acc[j][e] * acc[j][e];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float t = 0.f;
+#pragma unroll
+  for (int i = 0; i < CN_THREADS / 32; ++i) t += scratch[i];
+  const float rstd = rsqrtf(t / H + eps);
+#pragma unroll
+  for (int j = 0; j < CN_VEC; ++j) {
+    const int c = threadIdx.x + j * CN_THREADS;
+    if (c >= hv) break;
+    const uint32_t v[4] = {g[j].x, g[j].y, g[j].z, g[j].w};
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      o[e] = pack_bf16x2(acc[j][2 * e] * rstd * __uint_as_float(v[e] << 16), acc[j][2 * e + 1] * rstd * __uint_as_float(v[e] & 0xffff0000u));
+    reinterpret_cast<uint4*>(h + row * H)[c] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
 // backward of combine: dyp[dest] = w * dy[row];  dw[row,k] = <dy[row], yp[dest]>.  One warp per (row,k).
 __global__ void __launch_bounds__(256)
     moe_combine_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ yp,
@@ -492,6 +577,19 @@ SNU1_API int snu1_moe_route_few(const float* logits, int R, int E, int K, int no
   }
   SNU1_CUDA_CHECK(launch_pdl(moe_route_few_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, logits, R, E, K, norm_topk,
                              top_idx, top_w, max_tiles, tile_group, dest));
+  return kHostOk;
+}
+
+// snu1_moe_combine with a residual, and h = rmsnorm(y) * gain: H <= 8192.
+SNU1_API int snu1_moe_combine_norm(const void* yp, const int* dest, const int* top_idx, const float* top_w, const void* residual,
+                                   void* y, const void* gain, void* h, int R, int K, int H, float eps, void* stream) {
+  if (R < 1 || K < 1 || H < 8 || H % 8 || H > CN_THREADS * CN_VEC * 8 || residual == nullptr) {
+    set_last_error("moe_combine_norm: R=%d K=%d H=%d (a multiple of 8 up to 8192)", R, K, H);
+    return kHostBadArg;
+  }
+  SNU1_CUDA_CHECK(launch_pdl(moe_combine_norm_kernel, dim3(R), dim3(CN_THREADS), 0, (cudaStream_t)stream, (const __nv_bfloat16*)yp, dest,
+                             top_idx, top_w, (const __nv_bfloat16*)residual, (__nv_bfloat16*)y, (const __nv_bfloat16*)gain,
+                             (__nv_bfloat16*)h, K, H, eps));
   return kHostOk;
 }
 

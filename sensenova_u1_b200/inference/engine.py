@@ -23,7 +23,7 @@ from ..data.batch import apply_time_schedule
 from ..models import oracle
 from ..models.engine import Workspace
 from ..models.params import GEN, UND, ParamStore
-from ..ops import _lib, attention as attn_ops, decode_stack, fused, gemm
+from ..ops import _lib, attention as attn_ops, decode_stack, fused, gemm, moe
 from ..ops._lib import c_float, c_int, c_void_p
 
 CFG_NORMS = {"none": 0, "global": 1, "channel": 2, "cfg_zero_star": 3}
@@ -170,6 +170,7 @@ class InferenceEngine:
         act = None
         if not cfg.is_moe:
             act = ws.get("i.act", (R, cfg.ffn_size))
+        normed = False
         for l in range(cfg.num_layers):
             s = f"layers.{l}."
             if self.offload is not None:
@@ -178,7 +179,9 @@ class InferenceEngine:
             else:
                 W = lambda n: p[s + n][branch]
                 WE = lambda n: p[s + n]                     # expert mixtures are whole tensors of one branch
-            fused.rmsnorm_fwd(x, W("attn_norm"), None, h1, None, cfg.rms_eps)
+            if not normed:
+                fused.rmsnorm_fwd(x, W("attn_norm"), None, h1, None, cfg.rms_eps)
+            normed = False
             gemm.gemm_nt(h1, W("wqkv"), out=qkv, w_static=static)
             if publish is None:
                 fused.qknorm_rope_cache(qkv, qf, self.kc[l], self.vc[l], kv_rows, W("qk_norm"), pos3, self.inv_t,
@@ -209,7 +212,9 @@ class InferenceEngine:
                 gemm.linear_swiglu(h2, W("w13"), out=act, w_static=static)
                 x = gemm.gemm_nt(act, W("w2"), out=xo[l & 1], residual=x1, w_static=static)
             else:
-                x = self._moe_ffn(WE, h2, x1, branch, xo[l & 1])
+                # the next layer's norm rides on the experts' combination when few rows are routed
+                gain = p[f"layers.{l + 1}.attn_norm"][branch] if static and R <= moe.FEW_ROWS and l + 1 < cfg.num_layers else None
+                x, normed = self._moe_ffn(WE, h2, x1, branch, xo[l & 1], gain, h1), gain is not None
         return x
 
     def _decode_layers(self, x, branch, pos3, plan, kv_rows, kv_len):
@@ -224,11 +229,11 @@ class InferenceEngine:
                                          cfg.num_kv_heads, cfg.ffn_size, plan, kv_rows, pos3, kv_len, self.inv_t, self.inv_hw,
                                          cfg.rms_eps, self.scale)
 
-    def _moe_ffn(self, W, h2, x1, branch, out):
+    def _moe_ffn(self, W, h2, x1, branch, out, gain=None, h=None):
         """Dropless top-k expert FFN of one branch: device-side routing, tokens gathered into expert
         segments, one grouped GEMM per projection, weighted combine + residual (the reference loops
-        over experts in Python: src/sensenova_u1/models/neo_unify/modeling_qwen3_moe.py:51-119)."""
-        from ..ops import moe
+        over experts in Python: src/sensenova_u1/models/neo_unify/modeling_qwen3_moe.py:51-119).  With ``gain`` the norm of
+        the result goes to ``h`` as well."""
         cfg, p, ws = self.cfg, self.p, self.ws
         br = "und" if branch == UND else "gen"
         K = cfg.num_experts_per_tok if branch == UND else cfg.gen_num_experts_per_tok
@@ -241,18 +246,24 @@ class InferenceEngine:
             # Decoding: the experts' weights are streamed like those of any short product, only the experts in use.
             # One token (8 of 128 experts, 768 x 2048), whole block: 99 -> 45 us.
             r = moe.route_few(logits, K, cfg.norm_topk_prob, ws)
-            xp = moe.gather(h2, r, ws.get("i.moe.xp", (r.max_rows, H)))
+            # one row: every expert in use reads it where it is
+            xp = h2 if R == 1 else moe.gather(h2, r, ws.get("i.moe.xp", (r.max_rows, H)))
             act = gemm.gemm_experts(xp, W(f"moe_{br}.w13"), ws.get("i.moe.act", (r.max_rows, Fe)), r.tile_group, R, swiglu=True)
             yp = gemm.gemm_experts(act, W(f"moe_{br}.w2"), ws.get("i.moe.yp", (r.max_rows, H)), r.tile_group, R)
-            return moe.combine(yp, r, x1, out)
-        r = moe.route(logits, K, cfg.norm_topk_prob)
-        # rows between the experts' segments are never read: nothing is cleared
-        xp = ws.get("i.moe.xp", (r.max_rows, H))
-        moe.gather(h2, r, xp)
-        act = gemm.linear_swiglu(xp, W(f"moe_{br}.w13"), out=ws.get("i.moe.act", (r.max_rows, Fe)),
-                                 tile_group=r.tile_group)
-        yp = gemm.gemm_nt(act, W(f"moe_{br}.w2"), out=ws.get("i.moe.yp", (r.max_rows, H)), tile_group=r.tile_group)
-        return moe.combine(yp, r, x1, out)
+            if gain is not None and H <= 8192:
+                return moe.combine_norm(yp, r, x1, out, gain, h, cfg.rms_eps)
+        else:
+            r = moe.route(logits, K, cfg.norm_topk_prob)
+            # rows between the experts' segments are never read: nothing is cleared
+            xp = ws.get("i.moe.xp", (r.max_rows, H))
+            moe.gather(h2, r, xp)
+            act = gemm.linear_swiglu(xp, W(f"moe_{br}.w13"), out=ws.get("i.moe.act", (r.max_rows, Fe)),
+                                     tile_group=r.tile_group)
+            yp = gemm.gemm_nt(act, W(f"moe_{br}.w2"), out=ws.get("i.moe.yp", (r.max_rows, H)), tile_group=r.tile_group)
+        moe.combine(yp, r, x1, out)
+        if gain is not None:
+            fused.rmsnorm_fwd(out, gain, None, h, None, cfg.rms_eps)
+        return out
 
     def final_norm(self, x, branch):
         return fused.rmsnorm_fwd(x, self.p["final_norm"][branch], None, torch.empty_like(x), None, self.cfg.rms_eps)

@@ -132,16 +132,18 @@ def linear_swiglu(x, w13, out=None, *, tile_group=None, w_static=False):
 
 def gemm_experts(x, w, out, tile_group, rows: int, swiglu: bool = False):
     """Expert products of a few rows: rows ``128 t .. 128 t + rows - 1`` of ``x`` / ``out`` belong to expert
-    ``tile_group[t]`` (negative: unused tile); ``w[E,N,K]`` (``swiglu``: ``[E,2N,K]`` = gate rows, then up rows)."""
+    ``tile_group[t]`` (negative: unused tile); ``w[E,N,K]`` (``swiglu``: ``[E,2N,K]`` = gate rows, then up rows).
+    ``x`` of just ``rows`` rows: every tile reads the same ones."""
     _check(x, "x"); _check(w, "w"); _check(out, "out")
     E, Nw, K = w.shape
     N = Nw // 2 if swiglu else Nw
     tiles = tile_group.numel()
-    if not w.is_contiguous() or x.shape != (tiles * 128, K) or out.shape != (tiles * 128, N) or not 0 < rows <= 128:
-        raise ValueError("expert products need contiguous weights and 128 rows of x and out per tile")
+    shared = x.shape == (rows, K)
+    if not w.is_contiguous() or not (shared or x.shape == (tiles * 128, K)) or out.shape != (tiles * 128, N) or not 0 < rows <= 128:
+        raise ValueError("expert products need contiguous weights and 128 rows of x (or rows that all tiles share) and out per tile")
     _lib.call("gemm_experts", c_void_p(x.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), c_int(tiles),
               c_int(rows), c_int(N), c_int(K), c_ll(x.stride(0)), c_ll(out.stride(0)), c_void_p(tile_group.data_ptr()),
-              c_int(E), c_int(1 if swiglu else 0), c_void_p(_lib.stream()))
+              c_int(E), c_int(1 if swiglu else 0), c_int(1 if shared else 0), c_void_p(_lib.stream()))
     return out
 
 

@@ -111,6 +111,16 @@ def combine(yp, r: Routing, residual, y):
     return y
 
 
+def combine_norm(yp, r: Routing, residual, y, gain, h, eps: float):
+    """:func:`combine` and ``h = rmsnorm(y) * gain`` in one launch, a CTA per row."""
+    H = y.shape[1]
+    if not (residual.is_contiguous() and y.is_contiguous() and h.is_contiguous() and gain.numel() == H and h.shape == y.shape == residual.shape):
+        raise ValueError("combine_norm takes contiguous rows")
+    _lib.call("moe_combine_norm", P(yp), P(r.dest), P(r.top_idx), P(r.top_w), P(residual), P(y), P(gain), P(h), c_int(r.R), c_int(r.K),
+              c_int(H), c_float(eps), ST())
+    return y
+
+
 def combine_bwd(dy, yp, r: Routing, dyp, dw):
     _lib.call("moe_combine_bwd", P(dy), P(yp), P(r.dest), P(r.top_idx), P(r.top_w), P(dyp), P(dw), c_int(r.R),
               c_int(r.K), c_int(dy.shape[1]), ST())

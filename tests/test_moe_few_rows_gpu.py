@@ -94,3 +94,36 @@ def test_rows_without_a_finite_score(R, E, K, bad, what):
         assert torch.equal(tiles[(dest // 128).view(-1).long()], idx.view(-1))     # every slot in a tile of its expert
         assert torch.equal(r.top_idx[bad:], ref.top_idx[bad:]) and torch.equal(r.top_w[bad:], ref.top_w[bad:])
         assert torch.isnan(r.top_w[1:bad]).all()                            # what the row held goes on into its output
+
+
+@pytest.mark.parametrize("R,K,H", [(1, 1, 8), (3, 8, 2048), (32, 5, 8192), (2, 6, 2056)])
+def test_combination_and_norm(R, K, H):
+    from sensenova_u1_b200.ops import moe
+    g = torch.Generator(device="cuda").manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    yp, res, gain = rnd(R * K * 128, H), rnd(R, H), rnd(H)
+    r = moe.route_few(torch.randn(R, 16, device="cuda", generator=g), K, True, _Bufs())
+    y, h = torch.empty_like(res), torch.empty_like(res)
+    moe.combine_norm(yp, r, res, y, gain, h, 1e-6)
+    want = moe.combine(yp, r, res, torch.empty_like(res))
+    assert torch.equal(y, want)
+    ref = want.double() * (want.double().pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt() * gain.double()
+    # fp32 arithmetic, one rounding to bf16: half a unit in the last place, 2^-8 of the value
+    assert ((h.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-6).all()
+
+
+@pytest.mark.parametrize("rows", [1, 17])
+def test_experts_that_share_their_rows(rows):
+    from sensenova_u1_b200.ops import gemm
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    tg = torch.tensor([3, 0, -1, 4], dtype=torch.int32, device="cuda")
+    x = torch.randn(rows, 520, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(5, 400, 520, device="cuda", generator=g).to(torch.bfloat16)
+    each = torch.zeros(4 * 128, 520, device="cuda", dtype=torch.bfloat16)
+    each.view(4, 128, 520)[:, :rows] = x
+    for swiglu, n in ((False, 400), (True, 200)):
+        a, b = (gemm.gemm_experts(t, w, torch.full((4 * 128, n), 7.0, device="cuda", dtype=torch.bfloat16), tg, rows, swiglu=swiglu)
+                for t in (x, each))
+        used = torch.zeros(4 * 128, dtype=torch.bool, device="cuda")
+        used.view(4, 128)[:, :rows] = True
+        assert torch.equal(a[used], b[used]) and (a.view(4, 128, n)[2] == 7).all()
