@@ -16,13 +16,14 @@
 // these shapes fill a fraction of the chip; floor = weight bytes at 6.65 TB/s):
 //   N x K            rows 1: before  now  floor    rows 24: before  now    rows 128: before  now
 //   6144 x 4096             27.8   11.5    7.6              27.6   12.9              29.0   16.7
-//   4096 x 4096             27.4    8.2    5.0              27.5   10.3              27.6   13.7
+//   4096 x 4096             27.4    8.2    5.0              27.5    9.7              27.6   13.2
 //   24576 x 4096            63.4   35.2   30.3              54.1   36.3              56.1   43.5
-//   4096 x 12288            66.5   18.0   15.1              66.3   20.4              66.5   25.3
+//   4096 x 12288            66.5   18.0   15.1              66.3   20.2              66.5   25.0
 //   151936 x 4096          335.5  188.2  187.2             263.5  228.4             280.8  263.8
 #include <string.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "host_common.h"
 #include "sm100_common.cuh"
@@ -168,8 +169,31 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
     if (ok && elect_one()) umma_commit(acc_full);
     __syncwarp();
   }
-  // partial sums: tensor memory -> [row of x][128 weight rows] in this CTA's ring (all of its products have retired)
   const int rows = min(TN, args.M - m0);
+  // This CTA finishes rows [r_lo, r_hi) of the tile: 8 outputs per thread and step, two steps at a time where a thread has several.
+  // What bounds it is latency (other CTAs' sums, residual), so the first residual is read while the products still run, and a
+  // step's sums are asked for together: the number of parts is known to the loop.  They are asked for step by step, so that the
+  // steps share them out over the cluster; part by part all CTAs wait for the same one (128 rows, 4096 x 4096: 15.8 us).  Residual
+  // and sums one after the other / this, us: 24 rows 4096 x 4096 10.4 / 9.7, x 12288 21.2 / 20.2; 128 rows 13.6 / 13.2 and
+  // 26.4 / 25.0; 256 rows 18.2 / 15.8 and 36.6 / 33.2.  Four steps at a time: 13.5 and 25.3 at 128 rows, 15.8 and 32.8 at 256.
+  constexpr int BATCH = TN >= 64 ? 2 : 1;
+  const int v_hi = rows * (rank + 1) / args.split * (CN / 8);
+  const int tid = (int)threadIdx.x - 64;
+  int vb = rows * rank / args.split * (CN / 8);
+  uint4 res[BATCH];
+  auto load_res = [&]() {
+#pragma unroll
+    for (int i = 0; i < BATCH; ++i) {
+      const int vi = vb + tid + 128 * i, n = n0 + (vi % (CN / 8)) * 8;
+      if (vi < v_hi && n < args.N)
+        res[i] = *reinterpret_cast<const uint4*>(args.residual + (long long)(m0 + vi / (CN / 8)) * args.ldr + n);
+    }
+  };
+  if (warp >= 2) {
+    pdl_wait();
+    if (args.residual != nullptr) load_res();
+  }
+  // partial sums: tensor memory -> [row of x][128 weight rows] in this CTA's ring (all of its products have retired)
   float* part = reinterpret_cast<float*>(smem);
   bool ok = true;
   if (warp >= 2) {
@@ -202,58 +226,85 @@ __global__ void __launch_bounds__(NUM_THREADS, 2)
   }
   cluster_sync_all();
   if (warp >= 2) {
-    pdl_wait();
-    // this CTA finishes rows [r_lo, r_hi) of the tile: 8 outputs per thread and step
-    const int r_lo = rows * rank / args.split, r_hi = rows * (rank + 1) / args.split;
-    const int tid = threadIdx.x - 64;
     const uint32_t part_addr = smem_u32(part);
-    auto sum8 = [&](int r, int c, float (&o)[8]) {
+    // PARTS: how many CTAs share the reduction, 0 = args.split
+    auto finish = [&](auto parts) {
+      constexpr int PARTS = decltype(parts)::value;
+      auto sums = [&](int c, float (&o)[BATCH][8]) {      // in the order of the parts
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = 0.f;
-      for (int s = 0; s < args.split; ++s) {
-        const float4 a = ld_cluster_f4(part_addr + (r * BW + c) * 4, s);
-        const float4 b = ld_cluster_f4(part_addr + (r * BW + c) * 4 + 16, s);
-        o[0] += a.x; o[1] += a.y; o[2] += a.z; o[3] += a.w;
-        o[4] += b.x; o[5] += b.y; o[6] += b.z; o[7] += b.w;
-      }
-    };
-    for (int v = r_lo * (CN / 8) + tid; v < r_hi * (CN / 8) && ok; v += 128) {
-      const int r = v / (CN / 8), c8 = (v % (CN / 8)) * 8;
-      const int n = n0 + c8;
-      if (n >= args.N) continue;
-      float o[8];
-      sum8(r, c8, o);
-      if (SWIGLU) {
-        float up[8];
-        sum8(r, CN + c8, up);
+        for (int i = 0; i < BATCH; ++i) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = silu_mul(round_bf16(o[j]), round_bf16(up[j]));
-      } else {
+          for (int j = 0; j < 8; ++j) o[i][j] = 0.f;
+          if (vb + 128 * i >= v_hi) continue;
+          const int vi = min(vb + tid + 128 * i, v_hi - 1);      // a thread past the last step reads what it does not use
+          const uint32_t at = part_addr + ((vi / (CN / 8)) * BW + c + (vi % (CN / 8)) * 8) * 4;
+          auto add = [&](const float4& a, const float4& b) {
+            o[i][0] += a.x; o[i][1] += a.y; o[i][2] += a.z; o[i][3] += a.w;
+            o[i][4] += b.x; o[i][5] += b.y; o[i][6] += b.z; o[i][7] += b.w;
+          };
+          if constexpr (PARTS > 0) {
+            float4 a[PARTS], b[PARTS];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] *= args.alpha;
-      }
-      const long long m = m0 + r;
-      if (args.f32_out) {
-        float4* cp = reinterpret_cast<float4*>(reinterpret_cast<float*>(args.C) + m * args.ldc + n);
-        cp[0] = make_float4(o[0], o[1], o[2], o[3]);
-        cp[1] = make_float4(o[4], o[5], o[6], o[7]);
-      } else {
-        if (args.residual != nullptr) {
-          const uint4 u = *reinterpret_cast<const uint4*>(args.residual + m * args.ldr + n);
-          const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+            for (int s = 0; s < PARTS; ++s) {
+              a[s] = ld_cluster_f4(at, s);
+              b[s] = ld_cluster_f4(at + 16, s);
+            }
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 f = __bfloat1622float2(h[j]);
-            o[2 * j] += f.x;
-            o[2 * j + 1] += f.y;
+            for (int s = 0; s < PARTS; ++s) add(a[s], b[s]);
+          } else {
+            for (int s = 0; s < args.split; ++s) add(ld_cluster_f4(at, s), ld_cluster_f4(at + 16, s));
           }
         }
-        uint4 u;
-        u.x = pack_bf16x2(o[0], o[1]);
-        u.y = pack_bf16x2(o[2], o[3]);
-        u.z = pack_bf16x2(o[4], o[5]);
-        u.w = pack_bf16x2(o[6], o[7]);
-        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(args.C) + m * args.ldc + n) = u;
+      };
+      for (bool first = true; vb < v_hi; vb += 128 * BATCH, first = false) {
+        if (!first && args.residual != nullptr) load_res();
+        float out[BATCH][8];
+        sums(0, out);
+        if (SWIGLU) {
+          float up[BATCH][8];
+          sums(CN, up);
+#pragma unroll
+          for (int i = 0; i < BATCH; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) out[i][j] = silu_mul(round_bf16(out[i][j]), round_bf16(up[i][j]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < BATCH; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) out[i][j] *= args.alpha;
+        }
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+          const int vi = vb + tid + 128 * i, n = n0 + (vi % (CN / 8)) * 8;
+          if (vi >= v_hi || n >= args.N) continue;
+          float (&o)[8] = out[i];
+          const long long m = m0 + vi / (CN / 8);
+          if (args.f32_out) {
+            float4* cp = reinterpret_cast<float4*>(reinterpret_cast<float*>(args.C) + m * args.ldc + n);
+            cp[0] = make_float4(o[0], o[1], o[2], o[3]);
+            cp[1] = make_float4(o[4], o[5], o[6], o[7]);
+            continue;
+          }
+          if (args.residual != nullptr) {
+            const uint32_t u[4] = {res[i].x, res[i].y, res[i].z, res[i].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              o[2 * j] += __uint_as_float(u[j] << 16);
+              o[2 * j + 1] += __uint_as_float(u[j] & 0xffff0000u);
+            }
+          }
+          *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(args.C) + m * args.ldc + n) =
+              make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
+        }
+      }
+    };
+    if (ok) {
+      switch (args.split) {
+        case 1: finish(std::integral_constant<int, 1>()); break;
+        case 2: finish(std::integral_constant<int, 2>()); break;
+        case 4: finish(std::integral_constant<int, 4>()); break;
+        case 8: finish(std::integral_constant<int, 8>()); break;
+        default: finish(std::integral_constant<int, 0>());
       }
     }
   }

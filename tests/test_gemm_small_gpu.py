@@ -165,3 +165,19 @@ def test_one_wave_of_tiles_takes_the_weight_streaming_kernel(N, K, M, streams):
     assert (f - ref).norm() / ref.norm() < K / 16 * 2.0 ** -23 + 1e-6
     assert ((y.double() - ref - r.double()).abs() <= (ref + r.double()).abs() * 2.0 ** -8 + 1e-2).all()
     assert torch.equal(f, one) or not streams
+
+
+@pytest.mark.parametrize("split", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("M", [1, 24, 33, 64, 100, 128, 130])          # no, one and several steps of two per thread, ragged
+@pytest.mark.parametrize("N,K", [(136, 1096), (4096, 520)])
+def test_residual_joins_the_same_sums(M, N, K, split):
+    g = torch.Generator(device="cuda").manual_seed(M + split)
+    x, w, r = (torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16) for s in ((M, K), (N, K), (M, N)))
+    sums = _streamed(x, w, torch.full((M, N), float("nan"), device="cuda"), split)
+    guard = torch.full((M + 1, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    guard[:M] = r                                                       # in place, as a layer may have it
+    _streamed(x, w, guard[:M], split, f32=0, residual=guard[:M])
+    # one fp32 addition and one rounding behind the sums of the same parts in the same order
+    assert torch.equal(guard[:M], (sums + r.float()).to(torch.bfloat16)) and (guard[M] == 7).all()
+    exact = x.double() @ w.double().t()
+    assert (sums.double() - exact).abs().max() <= K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t()).max()
