@@ -80,3 +80,35 @@ def test_takes_refuses_what_the_kernel_is_not_built_for():
                 (1, 512, 1024, 8, 2, 9), (1, 1024, 1536, 8, 2, 9), (1, 1024, 0, 8, 2, 9), (1, 1024, 1024, 8, 4, 9),
                 (1, 1024, 1024, 4, 1, 9), (1, 1024, 1024, 8, 3, 9), (1, 4096, 12288, 32, 8, 3073)):
         assert not takes(*bad)
+
+
+def test_two_engines_on_two_streams():
+    """Whole-chip cooperative launches of two engines in two threads: each runs alone on the device, whichever comes first."""
+    import threading
+    E, cfg, one = _engine(**SIZES[1])
+    two = E.InferenceEngine(cfg, one.store)
+    docs = [torch.arange(5, 5 + n) % cfg.vocab_size for n in (60, 200)]
+
+    def request(eng, doc):
+        lay, h = eng.prefill([doc], reserve_image_tokens=24)
+        return eng.decode(lay, h, 24)
+    want = [request(e, d) for e, d in zip((one, two), docs)]
+    got, errors = [[], []], []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()), torch.no_grad():
+                for _ in range(4):
+                    # eager steps: a capture would not let the other thread allocate meanwhile
+                    lay, h = (one, two)[i].prefill([docs[i]], reserve_image_tokens=24)
+                    got[i].append((one, two)[i].decode(lay, h, 24, use_graph=False))
+        except Exception as e:                            # noqa: BLE001 - reported below
+            errors.append(e)
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    E._lib.check_status()
+    assert not errors and got == [[want[0]] * 4, [want[1]] * 4]
