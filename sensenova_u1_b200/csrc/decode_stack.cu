@@ -692,6 +692,9 @@ __device__ __forceinline__ void attend(const Args& a, Smem& s, float* red, const
         }
       }
     }
+    // ``red`` is the memory of x: a warp goes on to the output product's x, which may be there already, once every warp has its sums.
+    // The wait lies beside that for the other parts.
+    named_bar_sync(1, CT);
     if (a.split > 1) {
       // this CTA's share of the results, from all parts
       const uint2* p0 = a.part + (long long)(m * NG + hgp) * a.split * PART;
