@@ -9,7 +9,7 @@
 //    so the next product's weights arrive while activations travel, a norm or the attention of the layer runs;
 //  * eight consumer warps run the phases QKV | attention | output | gate and up with SwiGLU | down.
 //
-// Activations go from CTA to CTA through L2 without a barrier: a word is two bf16 and the number of the phase, stored at once;
+// Activations go from CTA to CTA through L2 without a barrier: a word is two bf16 and the number of the phase in one 64-bit access;
 // readers poll the words that they need.  (With a grid barrier per phase - fence, arrival, poll, then the loads - a boundary
 // took 6 us, more than the ring covers, and a layer 90 us.)  A word is not overwritten before all its readers are through:
 // the writer of the next layer's word has consumed, through the phases in between, results of every reader.
@@ -27,7 +27,7 @@
 //
 // Measured, us per 8B layer (386 MB; 59.8 at the measured copy bandwidth), chain of launches / this kernel:
 //   keys                50     839    1500    2000    3000    5000        2 x 50   2 x 1500      3 x 50    4 x 50
-//                 79.9/71.3 84.1/73.9 86.2/78.8 87.1/80.9 88.7/87.0 93.5/100  80.6/75.7 94.9/90.2  80.3/86.4 81.3/108
+//                 78.8/70.9 82.6/73.6 85.4/78.0 86.0/79.9 87.9/85.0 93.5/100  79.6/75.2 93.7/88.5  80.3/86.4 81.3/108
 // With three rows or more x takes the ring's place (4 and 3 stages) and the small phases grow; long documents are better off
 // with the attention kernel's deeper pipeline.  Hence the line at two rows and 3072 keys.
 // What bounds it now: 8 us from the last stage of QKV to the first of the output product (two hops of 2 us and the unit's own
@@ -244,19 +244,23 @@ __device__ __forceinline__ void produce(const Args& a, uint8_t* ring, Smem& s, i
   }
 }
 
-// ---- words between CTAs: two payloads and their phase numbers in 16 bytes, each half stored and read at once ----
+// ---- words between CTAs: a payload (low half) and its phase number (high half) in ONE element of 64 bits.  That they become
+// visible together is promised of an element only: of v2.u32 / v4.u32 every 32 bits are an access of their own.  The same time: a
+// layer of 50 keys took 71.3 us with those, 70.9 with these and a barrier more. ----
+__device__ __forceinline__ uint2 halves(uint64_t w) { return make_uint2((uint32_t)w, (uint32_t)(w >> 32)); }
 __device__ __forceinline__ uint4 ld_words(const uint2* p) {
-  uint4 v;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
+  uint64_t a, b;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+  const uint2 x = halves(a), y = halves(b);
+  return make_uint4(x.x, x.y, y.x, y.y);
 }
 __device__ __forceinline__ uint2 ld_word(const uint2* p) {
-  uint2 v;
-  asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
-  return v;
+  uint64_t a;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
+  return halves(a);
 }
 __device__ __forceinline__ void st_word(uint2* p, uint32_t v, uint32_t phase) {
-  asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(v), "r"(phase) : "memory");
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"((uint64_t)phase << 32 | v) : "memory");
 }
 // Polls until ``ready()`` holds in all lanes of the warp (``ready`` loads what is missing); false when it took too long or
 // another CTA gave up.

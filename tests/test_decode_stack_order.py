@@ -43,3 +43,11 @@ def test_attention_is_through_with_its_sums_before_the_next_product_stores_x(row
             break                                   # in no branch that was opened after the read
     else:
         pytest.fail("no barrier of all consumer warps between the sums and the end of the attention")
+
+
+def test_a_word_between_ctas_is_one_element_of_64_bits():
+    code = re.sub(r"//[^\n]*", "", SOURCE)
+    accesses = re.findall(r"(?:ld|st)\.(?:relaxed|volatile|acquire|release)\.gpu\.[\w.]+", code)
+    assert sorted(accesses) == ["ld.relaxed.gpu.global.b64", "ld.relaxed.gpu.global.v2.b64", "st.relaxed.gpu.global.b64"]
+    for name in ("x", "x1", "qkv", "o", "act", "part"):             # and nothing else touches the words
+        assert not re.search(rf"\*\s*\(?(?:reinterpret_cast<[^>]*>\()?a\.{name}\b", code)
