@@ -156,8 +156,7 @@ class InferenceEngine:
         if self.offload is not None:
             self.offload.set_phase("prefix" if branch == UND else "denoise")
         static = self.offload is None           # offloaded weights arrive from a copy stream between the kernels
-        if (static and isinstance(plan, DecodeRows) and not cfg.is_moe
-                and decode_stack.takes(R, H, cfg.ffn_size, cfg.num_heads, cfg.num_kv_heads, plan.max_keys)):
+        if isinstance(plan, DecodeRows) and self._one_launch(R, plan.max_keys):
             return self._decode_layers(x, branch, pos3, plan, kv_rows, kv_len)
         h1, h2, x1 = (ws.get(n, (R, H)) for n in ("i.h1", "i.h2", "i.x1"))
         xo = [ws.get(f"i.x{i}", (R, H)) for i in range(2)]
@@ -216,6 +215,12 @@ class InferenceEngine:
                 gain = p[f"layers.{l + 1}.attn_norm"][branch] if static and R <= moe.FEW_ROWS and l + 1 < cfg.num_layers else None
                 x, normed = self._moe_ffn(WE, h2, x1, branch, xo[l & 1], gain, h1), gain is not None
         return x
+
+    def _one_launch(self, rows: int, keys: int) -> bool:
+        """Whether a decode step of ``rows`` documents of up to ``keys`` keys is one launch for all layers."""
+        cfg = self.cfg
+        return (self.offload is None and not cfg.is_moe
+                and decode_stack.takes(rows, cfg.hidden_size, cfg.ffn_size, cfg.num_heads, cfg.num_kv_heads, keys))
 
     def _decode_layers(self, x, branch, pos3, plan, kv_rows, kv_len):
         """:meth:`layers` for one new token of a few documents: one launch for the whole stack."""
@@ -413,8 +418,23 @@ class InferenceEngine:
         graph = None
         stops = set(int(t) for t in stop_ids)
 
+        one_launch = first is not None and self._one_launch(n_docs, max_keys)
+
+        def tokens():
+            """The tokens so far.  A whole-stack launch that ran out of time (or follows one that did) leaves its output as it
+            was: the request fails, and the next one gets fresh scratch."""
+            new = rows.out[:, :done]
+            if not one_launch:
+                return new.tolist()
+            *flat, gave_up = torch.cat([new.reshape(-1), self._stack.count[-1:]]).tolist()       # one read for both
+            if gave_up:
+                self._stack = None
+                _lib.check_status()
+                raise _lib.NativeLibraryError("decode: a launch of the whole-stack kernel ran out of time")
+            return [flat[d * done:(d + 1) * done] for d in range(n_docs)]
+
         def finished():
-            toks = rows.out[:, :done].tolist()
+            toks = tokens() if stops else []
             return all(any(t in stops for t in row) for row in toks) if stops else False
 
         if sampling and sampling.get("do_sample", False) and sampling.get("seed") is not None and dev.type == "cuda":
@@ -431,9 +451,8 @@ class InferenceEngine:
             else:
                 step_fn()
             done += 1
-        toks = rows.out[:, :done].tolist()
         out = []
-        for row in toks:
+        for row in tokens():
             cut = len(row)
             for i, t in enumerate(row):
                 if t in stops:

@@ -24,7 +24,9 @@ def takes(rows: int, hidden: int, ffn: int, heads: int, kv_heads: int, keys: int
 
 
 class Scratch:
-    """What the CTAs of a launch exchange, for one engine; launches that share it must follow one another on the device."""
+    """What the CTAs of a launch exchange, for one engine; launches that share it must follow one another on the device.
+    ``count[-1]`` is not zero once a launch has run out of time: phase numbers may differ from then on, and every later launch
+    on this scratch returns at once."""
 
     def __init__(self, device):
         ctas = torch.cuda.get_device_properties(device).multi_processor_count

@@ -112,3 +112,24 @@ def test_two_engines_on_two_streams():
         t.join()
     E._lib.check_status()
     assert not errors and got == [[want[0]] * 4, [want[1]] * 4]
+
+
+@pytest.mark.parametrize("stop_ids", [(), (3,)])
+def test_a_launch_that_gave_up_fails_its_request_only(stop_ids):
+    E, cfg, eng = _engine(**SIZES[0])
+    doc = [torch.arange(5, 25)]
+
+    def request(new=12):
+        lay, h = eng.prefill(doc, reserve_image_tokens=new)
+        return eng.decode(lay, h, new, stop_ids=stop_ids, check_every=4)
+    want = request()
+    eng._stack.count[-1] = 1                                    # as a launch leaves it that has waited for too long
+    with pytest.raises(E._lib.NativeLibraryError):
+        request()
+    E._lib.check_status()                                       # the error has been reported: nothing is left for the next one
+    assert request() == want
+    eng.prefill(doc * 4, reserve_image_tokens=4)                # a chain of launches does not look at the scratch
+    eng._stack.count[-1] = 1
+    lay, h = eng.prefill(doc * 4, reserve_image_tokens=4)
+    assert len(eng.decode(lay, h, 4)) == 4
+    E._lib.check_status()
