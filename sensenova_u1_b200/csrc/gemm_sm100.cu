@@ -1084,7 +1084,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
                        long long b_group_stride, long long c_group_stride, int out_mode,
                        const void* residual, long long ldr, float alpha, long long a_rows,
                        long long b_rows, cudaStream_t stream, const CommArgs* comm = nullptr, int w_static = 0,
-                       int swiglu = 0) {
+                       int swiglu = 0, int in_parts = 0) {
   using namespace gemm;
   if (M <= 0 || N <= 0 || K < 0) {
     set_last_error("gemm: bad sizes M=%d N=%d K=%d", M, N, K);
@@ -1125,9 +1125,9 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   const int G = group_mode == 0 ? 1 : num_groups;
   // Few rows of A, plain y = x W^T: the weight-streaming kernel, up to 128 rows always, beyond (up to 1024, where a row tile
   // more reads the weights again from L2) as long as its 128 x 128 tiles are one wave: the 256 x 256 tiles of the pair kernel
-  // are then at most half of what the chip takes at once.  Beyond 128 rows only for an inference engine's weights (w_static):
-  // a reduction in parts has other roundings, which training amplifies from step to step.  us, weights cold in L2, streaming /
-  // pair:
+  // are then at most half of what the chip takes at once.  Beyond 128 rows only where the caller lets the reduction be taken in
+  // parts (in_parts: an inference engine, whether its weights are resident or not, so that both give the same bits): that has
+  // other roundings, which training amplifies from step to step.  us, weights cold in L2, streaming / pair:
   //   rows                  64         128         129         256         384         512         1024
   //   24576 x 4096     41.8/59.1   45.8/59.1   67.7/58.8   77.6/62.4               128/82.8
   //   151936 x 4096     216/252     260/254     469/270     497/275                1025/575
@@ -1137,7 +1137,7 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   //   4096 x 12288     26.7/74.7   28.7/68.3   32.2/62.1   32.7/62.2   54.5/62.0   54.3/62.5        -/74.1
   //   2048 x 4096      10.5/27.5   12.5/27.6   10.6/25.8   12.2/25.8   14.9/26.0   15.2/26.0   21.8/26.3
   //   128 x 2048                                9.6/14.6    9.8/14.7    9.8/14.7    9.8/14.7    9.8/14.7
-  const bool few = M <= 128 || (M <= 1024 && w_static && !swiglu && (long long)((N + 127) / 128) * ((M + 127) / 128) <= num_sms());
+  const bool few = M <= 128 || (M <= 1024 && in_parts && (long long)((N + 127) / 128) * ((M + 127) / 128) <= num_sms());
   if (few && group_mode == 0 && !a_mn && !b_mn && (out_mode == 0 || out_mode == 2) && comm == nullptr &&
       (g_pair_mode != 0 || swiglu) && K > 0)
     return launch_gemm_small(A, B, C, M, N, K, lda, ldb, ldc, out_mode == 2, residual, ldr, alpha, 0, w_static, swiglu,
@@ -1312,21 +1312,22 @@ SNU1_API int snu1_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
 }
 
 
-// y = alpha * x w^T (+ residual) with w[N,K] that no kernel in flight on the stream writes: a short product may start
-// reading w while the kernel in front of it is still running.  out_mode 0 (bf16) or 2 (fp32).
-SNU1_API int snu1_linear_static(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw,
-                                long long ldy, int out_mode, const void* residual, long long ldr, float alpha,
-                                void* stream) {
+// y = alpha * x w^T (+ residual) of an inference engine, whose reduction may be taken in parts (see launch_gemm).  w_static: no
+// kernel in flight on the stream writes w, so a short product may start reading it while the kernel in front is still running.
+// out_mode 0 (bf16) or 2 (fp32).
+SNU1_API int snu1_linear_infer(const void* x, const void* w, void* y, int M, int N, int K, long long ldx, long long ldw,
+                               long long ldy, int out_mode, const void* residual, long long ldr, float alpha, int w_static,
+                               void* stream) {
   if (out_mode != 0 && out_mode != 2) {
-    snu1::set_last_error("linear_static: out_mode must be 0 or 2");
+    snu1::set_last_error("linear_infer: out_mode must be 0 or 2");
     return snu1::kHostBadArg;
   }
   return snu1::launch_gemm(x, w, y, M, N, K, ldx, ldw, ldy, 0, 0, 0, 1, nullptr, nullptr, nullptr, 0, 0, out_mode,
-                           residual, ldr, alpha, M, N, reinterpret_cast<cudaStream_t>(stream), nullptr, 1);
+                           residual, ldr, alpha, M, N, reinterpret_cast<cudaStream_t>(stream), nullptr, w_static, 0, 1);
 }
 
 // y[M,F] = silu(x w_gate^T) * (x w_up^T) with w[2F,K] = F gate rows, then F up rows; gate and up are rounded to bf16
-// before the activation.  tile_group as in snu1_gemm_bf16 (null: one weight set).  w_static as in snu1_linear_static.
+// before the activation.  tile_group as in snu1_gemm_bf16 (null: one weight set).  w_static as in snu1_linear_infer.
 SNU1_API int snu1_linear_swiglu(const void* x, const void* w, void* y, int M, int F, int K, long long ldx, long long ldw,
                                 long long ldy, const int* tile_group, int num_groups, long long w_group_stride,
                                 int w_static, void* stream) {

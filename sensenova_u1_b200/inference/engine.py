@@ -181,7 +181,7 @@ class InferenceEngine:
             if not normed:
                 fused.rmsnorm_fwd(x, W("attn_norm"), None, h1, None, cfg.rms_eps)
             normed = False
-            gemm.gemm_nt(h1, W("wqkv"), out=qkv, w_static=static)
+            gemm.gemm_nt(h1, W("wqkv"), out=qkv, w_static=static, in_parts=True)
             if publish is None:
                 fused.qknorm_rope_cache(qkv, qf, self.kc[l], self.vc[l], kv_rows, W("qk_norm"), pos3, self.inv_t,
                                         self.inv_hw, cfg.num_heads, cfg.num_kv_heads, cfg.rms_eps)
@@ -205,11 +205,11 @@ class InferenceEngine:
                                           self.scale, o)
             else:
                 attn_ops.attention_fwd(q, k, v, plan, self.scale, out=o, want_lse=False)
-            gemm.gemm_nt(of, W("wo"), out=x1, residual=x, w_static=static)
+            gemm.gemm_nt(of, W("wo"), out=x1, residual=x, w_static=static, in_parts=True)
             fused.rmsnorm_fwd(x1, W("ffn_norm"), None, h2, None, cfg.rms_eps)
             if not cfg.is_moe:
                 gemm.linear_swiglu(h2, W("w13"), out=act, w_static=static)
-                x = gemm.gemm_nt(act, W("w2"), out=xo[l & 1], residual=x1, w_static=static)
+                x = gemm.gemm_nt(act, W("w2"), out=xo[l & 1], residual=x1, w_static=static, in_parts=True)
             else:
                 # the next layer's norm rides on the experts' combination when few rows are routed
                 gain = p[f"layers.{l + 1}.attn_norm"][branch] if static and R <= moe.FEW_ROWS and l + 1 < cfg.num_layers else None
@@ -246,7 +246,7 @@ class InferenceEngine:
         Fe = cfg.moe_intermediate_size
         gate = W(f"moe_{br}.gate")
         logits = gemm.gemm_nt(h2, gate, out=ws.get("i.moe.logits", (R, gate.shape[0]), torch.float32),
-                              out_mode=gemm.OUT_F32_STORE, w_static=self.offload is None)
+                              out_mode=gemm.OUT_F32_STORE, w_static=self.offload is None, in_parts=True)
         if R <= moe.FEW_ROWS:
             # Decoding: the experts' weights are streamed like those of any short product, only the experts in use.
             # One token (8 of 128 experts, 768 x 2048), whole block: 99 -> 45 us.

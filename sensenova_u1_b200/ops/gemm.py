@@ -81,11 +81,13 @@ def _raw_rows(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, grouped, G, tile_grou
 
 
 def gemm_nt(x, w, out=None, *, tile_group=None, residual=None, out_mode=OUT_BF16_STORE, alpha=1.0, rows_dev=None,
-            w_static=False):
+            w_static=False, in_parts=None):
     """``out[M,N] = x[M,K] @ w[(G,)N,K]^T``; ``tile_group[M/128]`` picks the weight set.
     ``rows_dev`` (int32 device scalar): only that many rows of ``x`` / ``out`` are in use.
     ``w_static``: no kernel that may still be running on the stream writes ``w`` (weights of an engine, not an
-    activation), so that a short product may read it while the kernel in front is still running."""
+    activation), so that a short product may read it while the kernel in front is still running.
+    ``in_parts`` (default: as ``w_static``): the sum over K may be taken in parts, which is faster for 129 to 1024 rows and
+    narrow weights and rounds differently; for inference."""
     _check(x, "x"); _check(w, "w")
     M, K = x.shape
     grouped = w.dim() == 3
@@ -100,10 +102,11 @@ def gemm_nt(x, w, out=None, *, tile_group=None, residual=None, out_mode=OUT_BF16
         _raw_rows(x, w, out, M, N, K, x.stride(0), w.stride(-2), out.stride(0), 0, 0, grouped, G, tile_group,
                   w.stride(0) if grouped else 0, out_mode, alpha, M, N, rows_dev)
         return out
-    if w_static and not grouped:
-        _lib.call("linear_static", c_void_p(x.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), c_int(M),
+    if (w_static if in_parts is None else in_parts) and not grouped:
+        _lib.call("linear_infer", c_void_p(x.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), c_int(M),
                   c_int(N), c_int(K), c_ll(x.stride(0)), c_ll(w.stride(0)), c_ll(out.stride(0)), c_int(out_mode),
-                  c_void_p(_lib.ptr(residual)), c_ll(_ldr(residual)), c_float(alpha), c_void_p(_lib.stream()))
+                  c_void_p(_lib.ptr(residual)), c_ll(_ldr(residual)), c_float(alpha), c_int(1 if w_static else 0),
+                  c_void_p(_lib.stream()))
         return out
     _raw(x, w, out, M, N, K, x.stride(0), w.stride(-2), out.stride(0), 0, 0,
          1 if grouped else 0, G, tile_group, None, None,

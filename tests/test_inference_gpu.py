@@ -150,3 +150,40 @@ def test_layer_offload_gives_identical_images(vram_mode):
     torch.cuda.synchronize(); _lib.check_status()
     assert torch.equal(full, off)
     assert m.engine.offload.bytes_streamed > 0
+
+
+@pytest.mark.parametrize("kind", ["dense", "mixture"])
+@pytest.mark.parametrize("size", [(128, 128), (192, 352)])             # 32 rows (with the next layer's norm), 132 rows
+def test_offloaded_products_take_their_sums_as_resident_ones(kind, size):
+    """The kernel of a product does not depend on where its weights were: the same bits, wide enough for sums in parts."""
+    from sensenova_u1_b200.config import tiny_mot
+    from sensenova_u1_b200.inference.api import ByteTokenizer, NEOChatModel
+    from sensenova_u1_b200.models.params import ParamStore
+    from sensenova_u1_b200.ops import _lib
+    kw = dict(num_experts=8, num_experts_per_tok=2, gen_num_experts=8, gen_num_experts_per_tok=2, moe_intermediate_size=256)
+    cfg = tiny_mot(head_dim=128, patch_size=16, num_layers=2, hidden_size=2048, num_heads=16, ffn_size=3072,
+                   **(kw if kind == "mixture" else {}))
+    host = ParamStore(cfg, device="cpu", with_grads=False)
+    host.init_weights(7)
+    dev = ParamStore(cfg, device="cuda", with_grads=False)
+    dev.copy_from(host)
+    args = dict(cfg_scale=3.0, timestep_shift=3.0, image_size=size, num_steps=2, seed=4)
+    tok = ByteTokenizer(cfg.vocab_size)
+    full = NEOChatModel(cfg, dev).t2i_generate(tok, "a boat", **args)
+    off = NEOChatModel(cfg, host, vram_mode="low", device="cuda").t2i_generate(tok, "a boat", **args)
+    _lib.check_status()
+    assert torch.equal(full, off)
+
+
+def test_the_norm_behind_the_experts_equals_the_norm_alone():
+    """Resident mixtures have it in the combination's launch, offloaded ones (whose next gain is not there yet) on its own."""
+    from sensenova_u1_b200.ops import fused, moe
+    from test_moe_few_rows_gpu import _Bufs
+    for R, K, H in [(1, 1, 8), (3, 8, 2048), (32, 5, 8192), (2, 6, 2056)]:
+        g = torch.Generator(device="cuda").manual_seed(H)
+        rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+        yp, res, gain = rnd(R * K * 128, H), rnd(R, H), rnd(H)
+        r = moe.route_few(torch.randn(R, 16, device="cuda", generator=g), K, True, _Bufs())
+        y, h = torch.empty_like(res), torch.empty_like(res)
+        moe.combine_norm(yp, r, res, y, gain, h, 1e-6)
+        assert torch.equal(h, fused.rmsnorm_fwd(y, gain, None, torch.empty_like(y), None, 1e-6))
