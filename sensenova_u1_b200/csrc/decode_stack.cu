@@ -28,8 +28,11 @@
 // Measured, us per 8B layer (386 MB; 59.8 at the measured copy bandwidth), chain of launches / this kernel:
 //   keys                50     839    1500    2000    3000    5000        2 x 50   2 x 1500      3 x 50    4 x 50
 //                 78.8/70.9 82.6/73.6 85.4/78.0 86.0/79.9 87.9/85.0 93.5/100  79.6/75.2 93.7/88.5  80.3/86.4 81.3/108
+//   two documents, keys of each  500, 50  1500, 50  1750, 50  2000, 50  2 x 1750  2 x 2000  2 x 2500   2 x 3000  3000, 50
+//                               83.1/76.8 91.3/87.5 90.8/90.9 91.0/92.4 93.7/91.8 94.0/93.7 96.8/98.4 97.1/101.4 91.6/99.7
 // With three rows or more x takes the ring's place (4 and 3 stages) and the small phases grow; long documents are better off
-// with the attention kernel's deeper pipeline.  Hence the line at two rows and 3072 keys.
+// with the attention kernel's deeper pipeline.  Hence the lines at two rows, and at 3072 keys of one document or 1792 of the
+// longer of two.
 // What bounds it now: 8 us from the last stage of QKV to the first of the output product (two hops of 2 us and the unit's own
 // chain), of which the ring covers 4.4.  Tried: asking L2 for stages beyond the ring (2 us per layer slower at any distance), a
 // grid barrier instead of the words (90 us), one accumulator per tile (a product waits 70 clocks for the one before it).

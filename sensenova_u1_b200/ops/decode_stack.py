@@ -15,12 +15,13 @@ def _words(rows: int, hidden: int, ffn: int, heads: int, kv_heads: int) -> int:
     return fn(c_int(rows), c_int(hidden), c_int(ffn), c_int(heads), c_int(kv_heads))
 
 
-MAX_KEYS = 3072      # longer documents: attention as a launch of its own is faster (both sides in csrc/decode_stack.cu)
+# by rows; longer documents: attention as a launch of its own is faster (both sides in csrc/decode_stack.cu)
+MAX_KEYS = {1: 3072, 2: 1792}
 
 
 def takes(rows: int, hidden: int, ffn: int, heads: int, kv_heads: int, keys: int) -> bool:
     """Whether the kernel is built for these sizes, and the better choice."""
-    return 0 < keys <= MAX_KEYS and _words(rows, hidden, ffn, heads, kv_heads) > 0
+    return 0 < keys <= MAX_KEYS.get(rows, 0) and _words(rows, hidden, ffn, heads, kv_heads) > 0
 
 
 class Scratch:

@@ -82,6 +82,12 @@ def test_takes_refuses_what_the_kernel_is_not_built_for():
         assert not takes(*bad)
 
 
+def test_two_long_documents_keep_the_chain():
+    from sensenova_u1_b200.ops.decode_stack import takes
+    at = lambda rows, keys: takes(rows, 4096, 12288, 32, 8, keys)
+    assert at(1, 3072) and not at(1, 3073) and at(2, 1792) and not at(2, 1793) and not at(3, 1)
+
+
 def test_two_engines_on_two_streams():
     """Whole-chip cooperative launches of two engines in two threads: each runs alone on the device, whichever comes first."""
     import threading
