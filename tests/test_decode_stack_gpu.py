@@ -1,4 +1,4 @@
-"""The whole-stack decode kernel (csrc/decode_stack.cu) against the kernels it stands in for and against fp64."""
+"""The whole-stack decode kernel (csrc/decode_stack.cu) against the kernels it stands in for and against the layers in fp64."""
 import pytest
 import torch
 
@@ -41,7 +41,7 @@ def test_stack_equals_the_layers_one_by_one(size, lens, monkeypatch):
         E._lib.check_status()
         return out, [t.clone() for t in eng.kc + eng.vc], rows
     want, cache, rows = step(False)
-    for _ in range(2):                                          # the barrier and the tickets are whole again after a launch
+    for _ in range(2):                                          # words of an earlier launch are not taken for this one's
         got, cache2, _ = step(True)
         # the same roundings to bf16 at the same places (half a unit in the last place each), on sums in another order: a
         # rounding that falls the other way is one unit, 2^-7, of one element; a handful of stages per layer compound
@@ -52,6 +52,84 @@ def test_stack_equals_the_layers_one_by_one(size, lens, monkeypatch):
             assert torch.equal(a[other], b[other])              # nothing else in the cache is touched
             assert (a[rows].double() - b[rows].double()).norm() <= 2.0 ** -7 * cfg.num_layers * b[rows].double().norm()
     monkeypatch.undo()
+
+
+def _exact(eng, cfg, x, pos3, first, rows, caches):
+    """The layers in fp64 for one new token per document: weights, x and the cache rows before the step as they are stored, angles
+    as fp32 products."""
+    p, D, Hq, Hk, eps = eng.p, 128, cfg.num_heads, cfg.num_kv_heads, cfg.rms_eps
+    norm = lambda v, g: v * (v.pow(2).mean(-1, keepdim=True) + eps).rsqrt() * g.double()
+    lin = lambda v, w: v @ w.double().t()
+    ang = [torch.cat([a, a], -1)[:, None].double() for a in (pos3[i].float()[:, None] * inv for i, inv in
+                                                              enumerate((eng.inv_t, eng.inv_hw, eng.inv_hw)))]
+
+    def rope(v, gains):
+        parts = torch.cat([norm(v[..., :64], gains[0]), norm(v[..., 64:], gains[1])], -1).split([64, 32, 32], -1)
+        turn = lambda t: torch.cat([-t[..., t.shape[-1] // 2:], t[..., :t.shape[-1] // 2]], -1)
+        return torch.cat([t * a.cos() + turn(t) * a.sin() for t, a in zip(parts, ang)], -1)
+    x = x.double()
+    for l in range(cfg.num_layers):
+        W = lambda n: p[f"layers.{l}.{n}"][0]
+        q, k, v = lin(norm(x, W("attn_norm")), W("wqkv")).split([Hq * D, Hk * D, Hk * D], -1)
+        q, k, v = rope(q.unflatten(-1, (Hq, D)), W("qk_norm")[:2]), rope(k.unflatten(-1, (Hk, D)), W("qk_norm")[2:]), v.unflatten(-1, (Hk, D))
+        o = torch.empty_like(q)
+        for d, (lo, hi) in enumerate(zip(first, rows)):
+            kd, vd = (torch.cat([c[lo:hi].double(), new[d:d + 1]]).repeat_interleave(Hq // Hk, 1)
+                      for c, new in ((caches[0][l], k), (caches[1][l], v)))
+            a = torch.softmax(torch.einsum("hd,khd->hk", q[d], kd) * D ** -0.5, -1)
+            o[d] = torch.einsum("hk,khd->hd", a, vd)
+        x = x + lin(o.flatten(1), W("wo"))
+        gate, up = lin(norm(x, W("ffn_norm")), W("w13")).chunk(2, -1)
+        x = x + lin(torch.nn.functional.silu(gate) * up, W("w2"))
+    return x
+
+
+WIDE = dict(hidden_size=4096, num_heads=32, num_kv_heads=8, ffn_size=12288, num_layers=2)      # the 8B model's widths
+DEEP = dict(hidden_size=1024, num_heads=8, num_kv_heads=2, ffn_size=1024, num_layers=49)       # two launches
+
+
+@pytest.mark.parametrize("size,lens", [(WIDE, n) for n in [(1,), (64,), (65,), (3000,), (1, 1), (64, 65), (1700, 3)]]
+                         + [(DEEP, (70,)), (DEEP, (9, 200))])
+def test_stack_against_the_layers_in_fp64(size, lens, monkeypatch):
+    E, cfg, eng = _engine(**size)
+    dev, n = eng.dev, len(lens)
+    g = torch.Generator(device=dev).manual_seed(sum(lens))
+    lay, _ = eng.prefill([torch.arange(5, 5 + k) % cfg.vocab_size for k in lens], reserve_image_tokens=4)
+    for c in eng.kc + eng.vc:                                   # keys and values of the size of the new ones
+        c.copy_(torch.randn(c.shape, device=dev, generator=g))
+    pos = torch.tensor([x.next_pos for x in lay], dtype=torch.int32, device=dev)
+    rows, first = torch.tensor([x.img_start for x in lay], device=dev), [x.kv_start for x in lay]
+    mq = E.attn_ops.make_meta(torch.arange(n, dtype=torch.int32, device=dev), pos)
+    eng._meta_k.index_copy_(0, rows, mq)
+    plan = E.DecodeRows(mq, eng._meta_k, torch.tensor(first, dtype=torch.int32, device=dev), max(lens) + 4)
+    x = torch.randn(n, cfg.hidden_size, device=dev, generator=g).to(torch.bfloat16)
+    pos3 = torch.stack([pos, pos * 0 + 3, pos * 0 + 5])
+    before = [[t.clone() for t in c] for c in (eng.kc, eng.vc)]
+
+    def step(stack):
+        monkeypatch.setattr(E.decode_stack, "takes", lambda *a: stack)
+        for new, old in zip(eng.kc + eng.vc, before[0] + before[1]):
+            new[rows] = old[rows]
+        out = eng.layers(x, E.UND, pos3, plan, rows, eng._meta_k.shape[0]).clone()
+        return out, torch.cat([t[rows].flatten() for t in eng.kc + eng.vc])
+    ref = _exact(eng, cfg, x, pos3, first, rows.tolist(), before)
+    err = {}
+    for stack in (False, True):
+        got = step(stack)
+        # ten roundings to bf16 per layer (half a unit in the last place, 2^-9 of the value): independent, each carried on at
+        # most at its own size.  One element: six deviations, and its own last rounding
+        err[stack], size = (got[0].double() - ref).abs(), ref.pow(2).mean().sqrt()
+        dev_ = 2.0 ** -9 * (10 * cfg.num_layers) ** 0.5 * size
+        print(f"stack={stack} {lens} rms {float(err[stack].pow(2).mean().sqrt() / size):.2e} (bound {float(dev_ / size):.2e}) "
+              f"max {float(err[stack].max() / size):.2e}")
+        assert err[stack].pow(2).mean().sqrt() <= dev_
+        assert (err[stack] <= 6 * dev_ + ref.abs() * 2.0 ** -8).all()
+    # no further away than the chain, whose roundings lie at the same places (the two differ by chance)
+    assert err[True].norm() <= 1.2 * err[False].norm()
+    for _ in range(60):                                         # sums have a fixed order: always the same bits
+        again = step(True)
+        assert torch.equal(again[0], got[0]) and torch.equal(again[1], got[1])
+    E._lib.check_status()
 
 
 @pytest.mark.parametrize("spoil", ["type", "shape", "stride"])
