@@ -373,7 +373,7 @@ class InferenceEngine:
         ``sampling = {do_sample, temperature, top_k, top_p, repetition_penalty, seed}`` (the knobs of the reference's
         ``generate``, src/sensenova_u1/models/neo_unify/modeling_neo_chat.py:1916-1975, examples/vqa/inference.py:29-112).
         ``prompt_ids`` (one id tensor per document) lets the repetition penalty see the prompt as well.
-        The reserved image rows of the cache are used for the new tokens.
+        The reserved image rows of the cache are used for the new tokens; a request that runs past the end of the cache raises.
 
         One decode step (LM head, argmax, embedding, metadata + tile plan of the new row, 42 layers)
         is about 500 small launches and launch-bound, so after one eager step the step is captured
@@ -417,6 +417,9 @@ class InferenceEngine:
         done = 0
         graph = None
         stops = set(int(t) for t in stop_ids)
+        room = kv_len - max(lay.img_start for lay in layouts)       # steps that the prefill left cache rows for
+        if room <= 0:
+            raise ValueError("decode: the prefill reserved no cache rows behind the last document")
 
         one_launch = first is not None and self._one_launch(n_docs, max_keys)
 
@@ -444,8 +447,10 @@ class InferenceEngine:
         if use_graph and max_new_tokens > 2:
             graph = self._capture(step_fn)
         while done < max_new_tokens:
-            if done % check_every == 0 and finished():
+            if (done % check_every == 0 or done >= room) and finished():
                 break
+            if done >= room:
+                raise ValueError(f"decode: the prefill reserved {room} cache rows, and not every document has stopped after as many tokens")
             if graph is not None:
                 graph.replay()
             else:
