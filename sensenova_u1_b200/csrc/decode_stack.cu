@@ -11,8 +11,9 @@
 //
 // Activations go from CTA to CTA through L2 without a barrier: a word is two bf16 and the number of the phase in one 64-bit access;
 // readers poll the words that they need.  (With a grid barrier per phase - fence, arrival, poll, then the loads - a boundary
-// took 6 us, more than the ring covers, and a layer 90 us.)  A word is not overwritten before all its readers are through:
-// the writer of the next layer's word has consumed, through the phases in between, results of every reader.
+// took 6 us, more than the ring covers, and a layer longer than as a chain of launches.)  A word is not overwritten before all
+// its readers are through: the writer of the next layer's word has consumed, through the phases in between, results of every
+// reader.
 //
 // Products: every CTA owns an even number of consecutive weight rows (gate and up rows of the same outputs), so that no CTA
 // has more than a per cent or two above the others; the rows of the residual stream stay in its shared memory.  Every warp
@@ -34,8 +35,11 @@
 // with the attention kernel's deeper pipeline.  Hence the lines at two rows, and at 3072 keys of one document or 1792 of the
 // longer of two.
 // What bounds it now: 8 us from the last stage of QKV to the first of the output product (two hops of 2 us and the unit's own
-// chain), of which the ring covers 4.4.  Tried: asking L2 for stages beyond the ring (2 us per layer slower at any distance), a
-// grid barrier instead of the words (90 us), one accumulator per tile (a product waits 70 clocks for the one before it).
+// chain), of which the ring covers 4.4.  Tried: asking L2 for stages beyond the ring (2 us per layer slower at any distance), one
+// accumulator per tile (a product waits 70 clocks for the one before it).  Nine warps leave 168
+// registers a thread (three of them share a quarter of the SM); one row spills 444 bytes, two rows 548 (stores).
+// The split follows the keys that the request may reach (max_keys), so a short document with a large budget has small parts.  50 keys,
+// chain / this kernel, budget of 32 tokens 80.0/70.7, 500 82.9/71.7, 1000 86.3/73.2, 3000 85.1/73.3.
 //
 // The launch is cooperative (all CTAs are resident).  Every wait is bounded; a CTA that gives up raises a flag that the
 // others poll, and the kernel then refuses later launches on the same scratch.
@@ -516,6 +520,8 @@ __device__ __forceinline__ void attend(const Args& a, Smem& s, float* red, const
   const int NG = a.Hq / HG, per_kv = a.Hq / a.Hkv / HG;
   const int units = a.M * NG * a.split;
   const long long ldk = (long long)a.Hkv * 128;
+  // One turn: there are never more units than CTAs (snu1_decode_stack_takes leaves at most 60 of (row, four heads), the split fills the
+  // rest).  Without the loop the compiler spills twice as much, us per layer with / without: 3000 keys 85.7/90.9, 2 x 1000 84.0/90.8.
   for (int ua = blockIdx.x; ua < units; ua += gridDim.x) {
     if (ua != (int)blockIdx.x) t = attention_unit(a, ua);
     Keys x{};

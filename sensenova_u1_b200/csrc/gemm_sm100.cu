@@ -1127,7 +1127,9 @@ static int launch_gemm(const void* A, const void* B, void* C, int M, int N, int 
   // more reads the weights again from L2) as long as its 128 x 128 tiles are one wave: the 256 x 256 tiles of the pair kernel
   // are then at most half of what the chip takes at once.  Beyond 128 rows only where the caller lets the reduction be taken in
   // parts (in_parts: an inference engine, whether its weights are resident or not, so that both give the same bits): that has
-  // other roundings, which training amplifies from step to step.  us, weights cold in L2, streaming / pair:
+  // other roundings, which training amplifies from step to step.  They are no larger: fp32 results against fp64, 129 rows, parts / pair,
+  // 4096 x 4096 2.1e-6 / 4.4e-6, 4096 x 12288 6.7e-6 / 1.4e-5, 128 x 2048 1.0e-6 / 2.1e-6; bf16 results 1.66e-3 either way.
+  // us, weights cold in L2, streaming / pair:
   //   rows                  64         128         129         256         384         512         1024
   //   24576 x 4096     41.8/59.1   45.8/59.1   67.7/58.8   77.6/62.4               128/82.8
   //   151936 x 4096     216/252     260/254     469/270     497/275                1025/575

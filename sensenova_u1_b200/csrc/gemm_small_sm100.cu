@@ -1,5 +1,6 @@
 // gemm_small: y[M,N] = x[M,K] w[N,K]^T for a few rows of x (text decoding, short prompts, thumbnails), where the
-// product is a stream of weights.
+// product is a stream of weights: up to 128 rows, and up to 1024 of an inference engine while the tiles are one wave (the rule and
+// both of its sides stand in launch_gemm).
 //
 // The roles of the operands are swapped: 128 rows of w are the M side of tcgen05.mma and the rows of x the N side
 // (16 .. 128), so no tensor-core row is spent on padding rows of x and the accumulator is [128 weight rows][rows
@@ -13,13 +14,15 @@
 // writes w (``w_static``: the layers of an inference engine); then the ring is filled with weights before the wait.
 //
 // Measured (weights cold in L2, one launch in a chain, us; before = the 256 x 256 pair kernel, of whose 16 - 96 tiles
-// these shapes fill a fraction of the chip; floor = weight bytes at 6.65 TB/s):
+// these shapes fill a fraction of the chip; floor = weight bytes at 6.54 TB/s; 24576 with SwiGLU, 4096 with a residual, 151936
+// with an fp32 result and without w_static):
 //   N x K            rows 1: before  now  floor    rows 24: before  now    rows 128: before  now
-//   6144 x 4096             27.8   11.5    7.6              27.6   12.9              29.0   16.7
-//   4096 x 4096             27.4    8.2    5.0              27.5    9.7              27.6   13.2
-//   24576 x 4096            63.4   35.2   30.3              54.1   36.3              56.1   43.5
-//   4096 x 12288            66.5   18.0   15.1              66.3   20.2              66.5   25.0
-//   151936 x 4096          335.5  188.2  187.2             263.5  228.4             280.8  263.8
+//   6144 x 4096             27.8   11.0    7.7              27.6   12.7              29.0   16.2
+//   4096 x 4096             27.4    8.4    5.1              27.5    9.6              27.6   13.0
+//   24576 x 4096            63.4   34.3   30.8              54.1   35.4              56.1   42.7
+//   4096 x 12288            66.5   17.3   15.4              66.3   19.7              66.5   24.2
+//   151936 x 4096          335.5  185.1  190.3             263.5  197.0             280.8  253.5
+// Registers: 86 and 88 for 16 and 32 rows, 148 with SwiGLU, 166 - 168 for 64 and 128 rows (two CTAs of 192 threads have 168); no spills.
 #include <string.h>
 
 #include <mutex>

@@ -375,8 +375,9 @@ class InferenceEngine:
         ``prompt_ids`` (one id tensor per document) lets the repetition penalty see the prompt as well.
         The reserved image rows of the cache are used for the new tokens; a request that runs past the end of the cache raises.
 
-        One decode step (LM head, argmax, embedding, metadata + tile plan of the new row, 42 layers)
-        is about 500 small launches and launch-bound, so after one eager step the step is captured
+        One decode step is the final norm, the LM head, the token, what follows from it, and the layers: one launch
+        for all of them where ``_one_launch`` says so, seven to ten short ones per layer otherwise.  The host takes longer to
+        launch those than they run, so after one eager step the step is captured
         in a CUDA graph and replayed; all of its state (token, position, cache row, output slot)
         lives in device tensors that the graph itself advances.  The host only looks at the tokens
         every ``check_every`` steps to see whether every document has stopped."""
