@@ -430,7 +430,8 @@ class InferenceEngine:
             new = rows.out[:, :done]
             if not one_launch:
                 return new.tolist()
-            *flat, gave_up = torch.cat([new.reshape(-1), self._stack.count[-1:]]).tolist()       # one read for both
+            count = self._stack.count
+            *flat, st["launches"], gave_up = torch.cat([new.reshape(-1), count[:1], count[-1:]]).tolist()     # one read for all
             if gave_up:
                 self._stack = None
                 _lib.check_status()
@@ -465,6 +466,8 @@ class InferenceEngine:
                     cut = i + 1
                     break
             out.append(row[:cut])
+        if st.get("launches", 0) > decode_stack.MAX_LAUNCHES:
+            self._stack = None                      # the next request starts with fresh scratch
         for lay in layouts:                         # every executed step consumed one cache row
             lay.img_start += done
             lay.prefix_len += done

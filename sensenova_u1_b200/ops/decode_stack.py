@@ -24,6 +24,12 @@ def takes(rows: int, hidden: int, ffn: int, heads: int, kv_heads: int, keys: int
     return 0 < keys <= MAX_KEYS.get(rows, 0) and _words(rows, hidden, ffn, heads, kv_heads) > 0
 
 
+# A launch has 384 phase numbers of 32 bits: they come round after 11 million launches, and a word that has not been written since
+# (of a second row, of more parts) could then be taken for a new one.  Scratch is replaced between requests well before that; a
+# request adds at most a launch per 48 layers and key.
+MAX_LAUNCHES = 1 << 23
+
+
 class Scratch:
     """What the CTAs of a launch exchange, for one engine; launches that share it must follow one another on the device.
     ``count[-1]`` is not zero once a launch has run out of time: phase numbers may differ from then on, and every later launch

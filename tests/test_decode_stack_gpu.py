@@ -217,3 +217,20 @@ def test_a_launch_that_gave_up_fails_its_request_only(stop_ids):
     lay, h = eng.prefill(doc * 4, reserve_image_tokens=4)
     assert len(eng.decode(lay, h, 4)) == 4
     E._lib.check_status()
+
+
+def test_scratch_is_replaced_before_its_phase_numbers_come_round():
+    E, cfg, eng = _engine(**SIZES[0])
+
+    def request(new=6):
+        lay, h = eng.prefill([torch.arange(5, 25)], reserve_image_tokens=new)
+        return eng.decode(lay, h, new)
+    want = request()
+    old = eng._stack
+    assert request() == want and eng._stack is old              # kept from one request to the next
+    numbers = 2 ** 32 // (48 * 8)
+    assert E.decode_stack.MAX_LAUNCHES + max(E.decode_stack.MAX_KEYS.values()) * 16 < numbers      # up to 768 layers
+    old.count[:-1] = E.decode_stack.MAX_LAUNCHES
+    assert request() == want and eng._stack is None
+    assert request() == want and int(eng._stack.count[0]) == 6
+    E._lib.check_status()
